@@ -48,7 +48,6 @@ cudaError_t oa_split_kc(cudaStream_t s, int nt, const double* X, int rows, int r
                         long kx0_cols, double w_kx0, __nv_bfloat16* P, long ldp, const int* cond = nullptr);
 int oa_tg_rows_pad(int rows, int box);
 int oa_tg_nb(int n);
-int oa_tg_nb_fwd(int n);
 cudaError_t oa_tfwd(cudaStream_t s, int nt, const __nv_bfloat16* PA, int rows_a, const __nv_bfloat16* PB, int rows_b,
                     int m, int n, long K, long ldp, double alpha, float* part, int max_kb, double* C, int* err_flag,
                     int nsm, const int* cond = nullptr);
@@ -1018,7 +1017,7 @@ void oa_planes_step_end(oa_ctx* c) {
 static bool plane_out(oa_ctx* c, int slot, int rows, int nt, OaPlaneOut* po) {
   oa_ctx_pc* p = pcx(c);
   const int nb = oa_tg_nb(rows);
-  if (!p->pl_big[slot] || nb == 0 || !(nt == 2 || nt == 3)) return false;
+  if (!p->pl_big[slot] || !(nt == 2 || nt == 3)) return false;
   const int rp = oa_tg_rows_pad(rows, nb);
   if (rp > p->pl_rows || 2L * c->ng > p->pl_ld) return false;
   *po = OaPlaneOut{p->pl_big[slot], rp, p->pl_ld, nt};
@@ -1063,9 +1062,9 @@ static cudaError_t mixed_fwd(oa_ctx* c, cudaStream_t s, int nt, const double* A,
                              const int* cond) {
   oa_ctx_pc* p = pcx(c);
   const int mx = c->nstate > c->natm_nl ? c->nstate : c->natm_nl;
-  const int nb = oa_tg_nb_fwd(n);
-  const int ra = oa_tg_rows_pad(m, 128), rb = nb ? oa_tg_rows_pad(n, nb) : 0;
-  if (nb && m <= mx && n <= mx && K <= p->pl_ld && ra <= p->pl_rows && rb <= p->pl_rows) {
+  const int nb = oa_tg_nb(n);
+  const int ra = oa_tg_rows_pad(m, 128), rb = oa_tg_rows_pad(n, nb);
+  if (m <= mx && n <= mx && K <= p->pl_ld && ra <= p->pl_rows && rb <= p->pl_rows) {
     const bool same = B == A && (w_kx0 == 1.0 || kx0_cols == 0) && ra % nb == 0;
     cudaError_t e = ensure_planes(c, s, nt, sa, A, m, ra, K, kx0_cols, w_kx0, cond);
     if (e != cudaSuccess) return e;
@@ -1101,8 +1100,8 @@ static cudaError_t mixed_bwd(oa_ctx* c, cudaStream_t s, int nt, const double* M1
         k.rows_pad > nkp && k.rows_pad % 32 == 0 && k.rows_pad <= p->pl_rows)
       nkp = k.rows_pad;
   }
-  const int ldm = oa_tg_nb(nj);  // M planes: leading size of the N tile, zero beyond nj
-  if (nj <= mx && nk <= mx && ncol <= p->pl_ld && ldm != 0 && nkp <= p->pl_rows && (!M2 || s1 != s2)) {
+  const int ldm = oa_tg_rows_pad(nj, oa_tg_nb(nj));  // M planes: leading size of whole N tiles, zero beyond nj
+  if (nj <= mx && nk <= mx && ncol <= p->pl_ld && ldm <= p->pl_rows && nkp <= p->pl_rows && (!M2 || s1 != s2)) {
     bf16 *pm1 = (bf16*)p->pl_ma, *pm2 = (bf16*)p->pl_mb;
     cudaError_t e = ensure_planes(c, s, nt, s1, X1, nk, nkp, ncol, 0, 1.0, cond);
     if (e == cudaSuccess) e = oa_split_kc(s, nt, M1, nk, nkp, nj, nj, 0, 1.0, pm1, ldm, cond);

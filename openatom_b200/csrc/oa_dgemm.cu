@@ -18,6 +18,7 @@
 // slabs of 32 doubles move global -> shared with 16-byte cp.async into a
 // ring of STAGES slabs (4 when A and B are one matrix, else 3: 144 / 216 KB),
 // so the loads of the next slabs overlap the DMMAs of the current one.
+#include <algorithm>
 #include "oa_internal.h"
 
 #define DG_TM 128
@@ -60,16 +61,38 @@ __device__ __forceinline__ void dg_load_slab(double* dst, const double* __restri
   }
 }
 
+// Output tiles of a product and the CTAs of each: tile t covers rows
+// 128 ti .., columns 128 tj .. and owns the CTAs [start[t], start[t + 1]), the
+// first n0[t] of them on the kx0 columns.  A tile's CTAs are in proportion to
+// the DMMAs that its busiest SM sub-partition issues (edge tiles and the
+// diagonal tiles of a symmetric product have fewer), so that all CTAs of the
+// product take the same time: S of 199 states on three tiles, for instance,
+// splits its SMs 59 : 44 : 44.
+// nt = 0 (more than 8 row or column tiles): CTA row y of the grid is tile
+// (y / tj[0], y mod tj[0]), all with the CTA counts of entry 0.
+#define DG_MAXT 64
+struct DgTiles {
+  int nt, sym;
+  short ti[DG_MAXT], tj[DG_MAXT], n0[DG_MAXT], start[DG_MAXT + 1];
+  signed char at[8][8];  // tile of (row tile, column tile), -1: the mirror of a symmetric product
+};
+
 template <bool SAME, int DG_STAGES>
 __global__ void __launch_bounds__(DG_THREADS, 1)
 k_dgemm_fwd(const double* __restrict__ A, const double* __restrict__ B, int m, int n, long K, long kx0_cols,
-            int n0, int nr, double* __restrict__ part, const int* __restrict__ cond) {
+            const __grid_constant__ DgTiles tiles, double* __restrict__ part, const int* __restrict__ cond) {
   if (cond && *cond == 0) return;
   extern __shared__ __align__(16) double dg_smem[];
+  int t = 0;
+  while (t + 1 < tiles.nt && (int)blockIdx.x >= tiles.start[t + 1]) ++t;
+  const int i0 = (tiles.nt ? tiles.ti[t] : (int)blockIdx.y / tiles.tj[0]) * DG_TM;
+  const int j0 = (tiles.nt ? tiles.tj[t] : (int)blockIdx.y % tiles.tj[0]) * DG_TM;
+  const int kb = blockIdx.x - tiles.start[t];
+  const int n0 = tiles.n0[t], nr = tiles.start[t + 1] - tiles.start[t] - n0;
+  // a diagonal tile of a symmetric product: one operand slab serves both sides
+  const bool diag = SAME || (tiles.sym && i0 == j0);
   double* As = dg_smem;
-  double* Bs = SAME ? dg_smem : dg_smem + DG_STAGES * DG_SLAB;
-  const int i0 = blockIdx.x * DG_TM, j0 = blockIdx.y * DG_TM;
-  const int kb = blockIdx.z;
+  double* Bs = diag ? dg_smem : dg_smem + DG_STAGES * DG_SLAB;
   // region and slab sequence of this CTA: slabs first, first + stride, ...
   const bool in0 = kb < n0;
   const long rbeg = in0 ? 0 : kx0_cols, rend = in0 ? kx0_cols : K;
@@ -77,18 +100,20 @@ k_dgemm_fwd(const double* __restrict__ A, const double* __restrict__ B, int m, i
   const long rslabs = (rend - rbeg + DG_KS - 1) / DG_KS;
   const int nslab = rslabs > first ? (int)((rslabs - first + stride - 1) / stride) : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // A == B (the overlap, one diagonal tile): the 32 x 32 blocks below the
-  // diagonal are the transposes of those above, which the reduction mirrors.
-  // The ten blocks on and above it go to warps 0-9, so that each SM
-  // sub-partition (warp mod 4) issues the DMMAs of at most three.
-  int wi = (warp >> 2) * 32, wj = (warp & 3) * 32;
-  if (SAME) {
+  // Block (wi, wj) of a warp: the blocks of a row or column go to different
+  // SM sub-partitions (warp mod 4), so that a tile with fewer than four block
+  // rows or columns loads them evenly.  On a diagonal tile of a symmetric
+  // product the 32 x 32 blocks below the diagonal are the transposes of those
+  // above, which the reduction mirrors; the ten blocks on and above it go to
+  // warps 0-9, at most three per sub-partition.
+  int wi = (warp >> 2) * 32, wj = (((warp & 3) + (warp >> 2)) & 3) * 32;
+  if (diag) {
     // 4 bi + bj of the upper blocks 0, 1, 2, 3, 5, 6, 7, 10, 11, 15, one hex digit per warp
     const int u = warp < 10 ? (int)((0xFBA7653210ull >> (4 * warp)) & 15u) : 0;
     wi = (u >> 2) * 32;
     wj = (u & 3) * 32;
   }
-  const bool active = (i0 + wi < m) && (j0 + wj < n) && (!SAME || warp < 10);
+  const bool active = (i0 + wi < m) && (j0 + wj < n) && (!diag || warp < 10);
   double acc[4][4][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -100,7 +125,7 @@ k_dgemm_fwd(const double* __restrict__ A, const double* __restrict__ B, int m, i
     if (s < nslab) {
       const long k0 = rbeg + ((long)first + (long)s * stride) * DG_KS;
       dg_load_slab(As + s * DG_SLAB, A, i0, m, K, k0, rend);
-      if (!SAME) dg_load_slab(Bs + s * DG_SLAB, B, j0, n, K, k0, rend);
+      if (!diag) dg_load_slab(Bs + s * DG_SLAB, B, j0, n, K, k0, rend);
     }
     dg_commit();
   }
@@ -114,7 +139,7 @@ k_dgemm_fwd(const double* __restrict__ A, const double* __restrict__ B, int m, i
         const int st = sn % DG_STAGES;
         const long k0 = rbeg + ((long)first + (long)sn * stride) * DG_KS;
         dg_load_slab(As + st * DG_SLAB, A, i0, m, K, k0, rend);
-        if (!SAME) dg_load_slab(Bs + st * DG_SLAB, B, j0, n, K, k0, rend);
+        if (!diag) dg_load_slab(Bs + st * DG_SLAB, B, j0, n, K, k0, rend);
       }
       dg_commit();
     }
@@ -149,25 +174,31 @@ k_dgemm_fwd(const double* __restrict__ A, const double* __restrict__ B, int m, i
     }
 }
 
-// C = alpha (w0 sum_{kb < n0} part[kb] + sum_{kb >= n0} part[kb]).  Block =
-// 64 outputs x 4 partial groups (group g sums the partials kb = g mod 4 of
+// C = alpha (w0 sum_{kb < n0} part[kb] + sum_{kb >= n0} part[kb]) over the
+// partials of an output's tile; an output below the diagonal blocks of a
+// symmetric product reads its transpose.  Block = 64 outputs x 4 partial groups (group g sums the partials kb = g mod 4 of
 // each range); the groups are combined in a fixed order, so the result does
 // not depend on scheduling.
 #define DR_COLS 64
 #define DR_GROUPS 4
 __global__ void __launch_bounds__(DR_COLS * DR_GROUPS)
-k_dgemm_fwd_reduce(const double* __restrict__ part, int n0, int nkb, size_t nn, double w0, double alpha,
-                   double* __restrict__ C, const int* __restrict__ cond, int sym_n) {
+k_dgemm_fwd_reduce(const double* __restrict__ part, const __grid_constant__ DgTiles tiles, int n, size_t nn,
+                   double w0, double alpha, double* __restrict__ C, const int* __restrict__ cond) {
   if (cond && *cond == 0) return;
   __shared__ double s0s[DR_GROUPS][DR_COLS], s1s[DR_GROUPS][DR_COLS];
   const int col = threadIdx.x % DR_COLS, g = threadIdx.x / DR_COLS;
   const size_t i = (size_t)blockIdx.x * DR_COLS + col;
-  // sym_n > 0: symmetric n x n result whose partials hold only the 32 x 32
-  // blocks on and above the diagonal; (r, c) below reads (c, r)
   size_t src = i;
-  if (sym_n > 0 && i < nn) {
-    const int r = (int)(i / sym_n), c = (int)(i - (size_t)r * sym_n);
-    if ((r >> 5) > (c >> 5)) src = (size_t)c * sym_n + r;
+  int n0 = 0, nkb = 0;
+  if (i < nn) {
+    int r = (int)(i / n), c = (int)(i - (size_t)r * n);
+    if (tiles.sym && (r >> 5) > (c >> 5)) {
+      src = (size_t)c * n + r;
+      const int s = r; r = c; c = s;
+    }
+    const int t = tiles.nt > 1 ? tiles.at[r >> 7][c >> 7] : 0;
+    n0 = tiles.n0[t];
+    nkb = tiles.start[t + 1] - tiles.start[t];
   }
   double s0 = 0.0, s1 = 0.0;
   if (i < nn) {
@@ -216,39 +247,69 @@ cudaError_t oa_dgemm_fwd(cudaStream_t s, const double* A, const double* B, int m
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0)
     nsm = 148;
   const int ti = (m + DG_TM - 1) / DG_TM, tj = (n + DG_TM - 1) / DG_TM;
+  const bool listed = ti <= 8 && tj <= 8;
+  const bool sym = A == B && m == n && listed;
+  DgTiles tiles;
+  tiles.sym = sym;
+  tiles.nt = 0;
+  // DMMA load of a tile: blocks of its busiest sub-partition
+  int load[DG_MAXT], total = 0;
+  for (int a = 0; listed && a < ti; ++a)
+    for (int b = 0; b < tj; ++b) {
+      tiles.at[a][b] = -1;
+      if (sym && b < a) continue;
+      const int rb = (std::min(m - a * DG_TM, DG_TM) + 31) / 32, cb = (std::min(n - b * DG_TM, DG_TM) + 31) / 32;
+      const int t = tiles.nt++;
+      tiles.ti[t] = (short)a;
+      tiles.tj[t] = (short)b;
+      tiles.at[a][b] = (signed char)t;
+      load[t] = sym && a == b ? (rb == 4 ? 3 : std::min(rb, 2)) : std::min(rb, cb);
+      total += load[t];
+    }
+  if (!listed) {
+    tiles.tj[0] = (short)tj;
+    load[0] = 1;
+    total = ti * tj;
+  }
   // about one CTA per SM; the kx0 region gets CTAs in proportion to its slabs
   const long s0 = (kx0_cols + DG_KS - 1) / DG_KS, sr = (K - kx0_cols + DG_KS - 1) / DG_KS;
-  int nk = nsm / (ti * tj);
-  if (nk > nkb) nk = nkb;
-  if (nk < 2) nk = 2;
-  int n0 = s0 > 0 ? (int)((nk * s0 + s0 + sr - 1) / (s0 + sr)) : 0;  // rounded up: no straggler
-  if (s0 > 0 && n0 < 1) n0 = 1;
-  if (n0 > s0) n0 = (int)s0;
-  int nr = nk - n0;
-  if (nr > sr) nr = (int)sr;
-  if (sr > 0 && nr < 1) return cudaErrorNotSupported;
-  const int nkb_eff = n0 + nr;
-  if (nkb_eff < 1 || nkb_eff > nkb) return cudaErrorNotSupported;
-  // one shared slab serves both operands only when the single output tile
-  // is diagonal (A == B and m, n <= 128)
-  const bool same = (A == B) && ti == 1 && tj == 1;
+  int cta = 0;
+  for (int t = 0; t < std::max(tiles.nt, 1); ++t) {
+    int nk = (int)((long)nsm * load[t] / total);
+    if (nk > nkb) nk = nkb;
+    if (nk < 2) nk = 2;
+    int n0 = s0 > 0 ? (int)((nk * s0 + s0 + sr - 1) / (s0 + sr)) : 0;  // rounded up: no straggler
+    if (s0 > 0 && n0 < 1) n0 = 1;
+    if (n0 > s0) n0 = (int)s0;
+    int nr = nk - n0;
+    if (nr > sr) nr = (int)sr;
+    if (sr > 0 && nr < 1) return cudaErrorNotSupported;
+    if (n0 + nr < 1 || n0 + nr > nkb) return cudaErrorNotSupported;
+    tiles.n0[t] = (short)n0;
+    tiles.start[t] = (short)cta;
+    cta += n0 + nr;
+    tiles.start[t + 1] = (short)cta;
+  }
+  const dim3 grid(cta, listed ? 1 : ti * tj);
+  // one shared slab per stage when the single output tile is diagonal
+  // (A == B, m = n <= 128)
+  const bool same = sym && tiles.nt == 1;
   const size_t sm = oa_dgemm_fwd_smem(same);
-  dim3 grid(ti, tj, nkb_eff);
   cudaError_t e;
   if (same) {
     e = oa_smem_limit(k_dgemm_fwd<true, DG_STAGES_SAME>);
     if (e != cudaSuccess) return e;
-    k_dgemm_fwd<true, DG_STAGES_SAME><<<grid, DG_THREADS, sm, s>>>(A, B, m, n, K, kx0_cols, n0, nr, part, cond);
+    k_dgemm_fwd<true, DG_STAGES_SAME><<<grid, DG_THREADS, sm, s>>>(A, B, m, n, K, kx0_cols, tiles, part, cond);
   } else {
     e = oa_smem_limit(k_dgemm_fwd<false, DG_STAGES_TWO>);
     if (e != cudaSuccess) return e;
-    k_dgemm_fwd<false, DG_STAGES_TWO><<<grid, DG_THREADS, sm, s>>>(A, B, m, n, K, kx0_cols, n0, nr, part, cond);
+    k_dgemm_fwd<false, DG_STAGES_TWO><<<grid, DG_THREADS, sm, s>>>(A, B, m, n, K, kx0_cols, tiles, part, cond);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const size_t mn = (size_t)m * n;
   k_dgemm_fwd_reduce<<<(unsigned)((mn + DR_COLS - 1) / DR_COLS), DR_COLS * DR_GROUPS, 0, s>>>(
-      part, n0, nkb_eff, mn, w_kx0, alpha, C, cond, same ? n : 0);
+      part, tiles, n, mn, w_kx0, alpha, C, cond);
   return cudaGetLastError();
 }
 
@@ -315,7 +376,8 @@ __device__ __forceinline__ void db_load_slab(double* ms, double* xs, const doubl
 // *cond2 != 0; vel (optional, when *vcond != 0) receives the finite
 // difference (result - previous out) vscale, previous out read by the
 // thread that overwrites it.
-template <bool TWO>
+// EDGE: the last row tile has idle 32-row blocks (nj not a multiple of 128)
+template <bool TWO, bool EDGE>
 __global__ void __launch_bounds__(DB_THREADS, 2)
 k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double a1_kx0, double a1_rest,
             const double* __restrict__ M2, const double* __restrict__ X2, double a2, int nj, int nk, long ncol,
@@ -331,7 +393,11 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
   const long c0 = (long)blockIdx.x * DB_TC;
   const int j0 = blockIdx.y * DB_TJ;  // rows j0 .. j0 + 127 of the output
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wj = (warp >> 1) * 32, wc = (warp & 1) * 32;
+  // the row block of a warp pair rotates with the block: the idle blocks of
+  // an edge tile then fall on different SM sub-partitions in the two
+  // resident blocks
+  const int wj = (((warp >> 1) + (EDGE ? (blockIdx.x & 1) : 0)) & 3) * 32, wc = (warp & 1) * 32;
+  const bool live = !EDGE || j0 + wj < nj;
   const int nsl = (nk + DB_KS - 1) / DB_KS;
   const int ntot = TWO ? 2 * nsl : nsl;
   double acc[4][4][2];
@@ -372,6 +438,7 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
     const double sa = (TWO && s >= nsl) ? a2 : 1.0;
     const double* ms = Ms + (s % DB_STAGES) * DB_MSLAB;
     const double* xs = Xs + (s % DB_STAGES) * DB_XSLAB;
+    if (live)
 #pragma unroll
     for (int k4 = 0; k4 < DB_KS; k4 += 4) {
       double af[4], bf[4];
@@ -471,19 +538,15 @@ cudaError_t oa_dgemm_bwd_ex(cudaStream_t s, const double* M1, const double* X1, 
   const size_t sm = (size_t)DB_STAGES * (DB_MSLAB + DB_XSLAB) * sizeof(double);
   // column tiles of 64 by row tiles of 128
   dim3 grid((unsigned)((ncol + DB_TC - 1) / DB_TC), (unsigned)((nj + DB_TJ - 1) / DB_TJ));
-  cudaError_t e;
-  if (M2) {
-    e = oa_smem_limit(k_dgemm_bwd<true>);
+  auto go = [&](auto kern) -> cudaError_t {
+    const cudaError_t e = oa_smem_limit(kern);
     if (e != cudaSuccess) return e;
-    k_dgemm_bwd<true><<<grid, DB_THREADS, sm, s>>>(M1, X1, a1_kx0, a1_rest, M2, X2, a2, nj, nk, ncol, kx0_cols, out,
-                                                    cond, yadd, out2, cond2, pz, vel, vscale, vcond);
-  } else {
-    e = oa_smem_limit(k_dgemm_bwd<false>);
-    if (e != cudaSuccess) return e;
-    k_dgemm_bwd<false><<<grid, DB_THREADS, sm, s>>>(M1, X1, a1_kx0, a1_rest, M2, X2, a2, nj, nk, ncol, kx0_cols,
-                                                     out, cond, yadd, out2, cond2, pz, vel, vscale, vcond);
-  }
-  return cudaGetLastError();
+    kern<<<grid, DB_THREADS, sm, s>>>(M1, X1, a1_kx0, a1_rest, M2, X2, a2, nj, nk, ncol, kx0_cols, out, cond, yadd,
+                                      out2, cond2, pz, vel, vscale, vcond);
+    return cudaGetLastError();
+  };
+  if (nj % DB_TJ == 0) return M2 ? go(k_dgemm_bwd<true, false>) : go(k_dgemm_bwd<false, false>);
+  return M2 ? go(k_dgemm_bwd<true, true>) : go(k_dgemm_bwd<false, true>);
 }
 
 cudaError_t oa_dgemm_bwd(cudaStream_t s, const double* M1, const double* X1, double a1_kx0, double a1_rest,

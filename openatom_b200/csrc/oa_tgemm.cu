@@ -335,7 +335,9 @@ k_tfwd_reduce(const float* __restrict__ part, int nkb, size_t nn, double alpha, 
 }
 
 // ---------------------------------------------------------------------------
-// backward, persistent: CTA b takes the 128-column tiles b, b + grid, ...;
+// backward, persistent: CTA b takes the tiles b, b + grid, ... of 128 columns
+// by NB output rows (the row tiles of one column tile next to each other, so
+// that CTAs running at the same time share its X planes in L2);
 // D_t[c][j] per term t in TMEM.  Warp roles: warp 0 lane 0 issues the TMA
 // loads over a ring of stages, warp 1 lane 0 issues the MMAs into one of
 // two TMEM accumulators (tile i uses buffer i & 1), warps 2-5 drain the
@@ -356,7 +358,7 @@ template <int NT, int NB>
 __global__ void __launch_bounds__(TB_THREADS, 1)
 k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensorMap tM1,
        const __grid_constant__ CUtensorMap tX2, const __grid_constant__ CUtensorMap tM2, int nterm, double a1_kx0,
-       double a1_rest, double a2, int nj, int nk, long ncol, long kx0_cols, int stages, double* out,
+       double a1_rest, double a2, int nj, int njt, int nk, long ncol, long kx0_cols, int stages, double* out,
        int* __restrict__ err_flag, const double* yadd, const int* __restrict__ cond) {
   if (cond && *cond == 0) return;
   extern __shared__ __align__(1024) unsigned char tg_raw[];
@@ -373,8 +375,8 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
   uint32_t* tslot = (uint32_t*)(acce + 2);
   volatile int* okflag = (volatile int*)(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long ntile = (ncol + TG_M - 1) / TG_M;
-  const int my_tiles = blockIdx.x < ntile ? (int)((ntile - 1 - blockIdx.x) / gridDim.x + 1) : 0;
+  const int ntile = (int)((ncol + TG_M - 1) / TG_M) * njt;
+  const int my_tiles = (int)blockIdx.x < ntile ? (ntile - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const int kch = (nk + TG_KS - 1) / TG_KS;
   const int nslab = nterm * kch;
   if (tid == 0) {
@@ -394,7 +396,8 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
       long g = 0;
       bool ok = true;
       for (int i = 0; i < my_tiles && ok; ++i) {
-        const int c0 = (int)(((long)blockIdx.x + (long)i * gridDim.x) * TG_M);
+        const int tile = (int)blockIdx.x + i * (int)gridDim.x, ct = njt == 1 ? tile : tile / njt;
+        const int c0 = ct * TG_M, jc = (tile - ct * njt) * (NB / 64);
         for (int sl = 0; sl < nslab; ++sl, ++g) {
           const int st = (int)(g % stages);
           if (!tg_wait(&empty[st], (uint32_t)((g / stages) & 1) ^ 1u) || !*okflag) { ok = false; break; }
@@ -410,7 +413,7 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
             tg_tma_box(sb + q * a_bytes, tx, k0, c0 / 64, q, &full[st]);
             tg_tma_box(sb + q * a_bytes + 4096, tx, k0, c0 / 64 + 1, q, &full[st]);
 #pragma unroll
-            for (int h = 0; h < NB / 64; ++h) tg_tma_box(sb + NT * a_bytes + q * b_bytes + h * 4096, tm, k0, h, q, &full[st]);
+            for (int h = 0; h < NB / 64; ++h) tg_tma_box(sb + NT * a_bytes + q * b_bytes + h * 4096, tm, k0, jc + h, q, &full[st]);
           }
         }
       }
@@ -475,7 +478,12 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
       if (!tg_wait(&accf[b], (uint32_t)((i >> 1) & 1))) { *okflag = 0; break; }
       tg_tc_after();
       if (!*okflag) break;
-      const long c = ((long)blockIdx.x + (long)i * gridDim.x) * TG_M + row;
+      const int tile = (int)blockIdx.x + i * (int)gridDim.x, ct = njt == 1 ? tile : tile / njt;
+      const long c = (long)ct * TG_M + row;
+      const int jb = (tile - ct * njt) * NB;  // first output row of the tile
+      const int nje = nj - jb;                // output rows from there
+      double* oc = out + (size_t)jb * ncol + c;
+      const double* yc = yadd ? yadd + (size_t)jb * ncol + c : nullptr;
       const double a1 = (c < kx0_cols) ? a1_kx0 : a1_rest;
       const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * NBP);
       for (int q0 = 0; q0 < NB; q0 += 16) {
@@ -486,14 +494,14 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
           // yadd may be out itself: all 16 reads go before the writes
           double ya[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) ya[e] = (yadd && q0 + e < nj) ? yadd[(size_t)(q0 + e) * ncol + c] : 0.0;
+          for (int e = 0; e < 16; ++e) ya[e] = (yc && q0 + e < nje) ? yc[(size_t)(q0 + e) * ncol] : 0.0;
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const int j = q0 + e;
-            if (j < nj) {
+            if (j < nje) {
               double r = a1 * (double)v1[e];
               if (nterm == 2) r += a2 * (double)v2[e];
-              out[(size_t)j * ncol + c] = r + ya[e];
+              oc[(size_t)j * ncol] = r + ya[e];
             }
           }
         }
@@ -558,11 +566,9 @@ cudaError_t oa_split_kc(cudaStream_t s, int nt, const double* X, int rows, int r
 
 // rows of the planes of an operand the kernels read in boxes of `box` rows
 int oa_tg_rows_pad(int rows, int box) { return (rows + box - 1) / box * box; }
-int oa_tg_nb(int n) { return n <= 64 ? 64 : (n <= 128 ? 128 : 0); }
-// N tile of the forward product: whole N up to 128, else tiles of 128
-int oa_tg_nb_fwd(int n) { return n <= 128 ? oa_tg_nb(n) : 128; }
+// N tile of the products: 64, or tiles of 128
+int oa_tg_nb(int n) { return n <= 64 ? 64 : 128; }
 
-static int tg_nb(int n) { return n <= 64 ? 64 : (n <= 128 ? 128 : 0); }
 // forward stages carry TG_KF columns of K, backward stages TG_KS rows of k
 static size_t tg_smem(int nt, int nb, int stages, bool fwd) {
   const size_t kk = fwd ? TG_KF : TG_KS;
@@ -580,8 +586,8 @@ static int tg_stages(int nt, int nb, bool fwd) {
 cudaError_t oa_tfwd(cudaStream_t s, int nt, const bf16* PA, int rows_a, const bf16* PB, int rows_b, int m, int n,
                     long K, long ldp, double alpha, float* part, int max_kb, double* C, int* err_flag, int nsm,
                     const int* cond) {
-  const int nb = oa_tg_nb_fwd(n);
-  if (nb == 0 || m > rows_a || n > rows_b) return cudaErrorNotSupported;
+  const int nb = oa_tg_nb(n);
+  if (m > rows_a || n > rows_b) return cudaErrorNotSupported;
   const int stages = tg_stages(nt, nb, true);
   if (stages < 2) return cudaErrorNotSupported;
   const int mt = (m + TG_M - 1) / TG_M, ntl = (n + nb - 1) / nb;
@@ -614,26 +620,27 @@ cudaError_t oa_tfwd(cudaStream_t s, int nt, const bf16* PA, int rows_a, const bf
 
 // out[j][c] = a1(c) sum_k M1[k][j] X1[k][c] + a2 sum_k M2[k][j] X2[k][c]
 // (+ yadd[j][c], which may be out itself) from X planes (rows nk, leading
-// size ldx) and M planes (rows nk, leading size oa_tg_nb(nj), zero beyond
-// nj); nk a multiple of 32 (planes padded with zero rows).  cond: optional device flag, nothing runs
+// size ldx) and M planes (rows nk, leading size nj rounded up to the N
+// tile oa_tg_nb(nj), zero beyond nj); nk a multiple of 32 (planes padded with zero rows).  cond: optional device flag, nothing runs
 // when it is 0.
 cudaError_t oa_tbwd(cudaStream_t s, int nt, const bf16* PM1, const bf16* PX1, double a1_kx0, double a1_rest,
                     const bf16* PM2, const bf16* PX2, double a2, int nj, int nk, long ncol, long ldx, long kx0_cols,
                     double* out, int* err_flag, const double* yadd, const int* cond) {
-  const int nb = tg_nb(nj);
-  if (nb == 0 || ((PM2 == nullptr) != (PX2 == nullptr)) || nk < TG_KS || (nk % TG_KS)) return cudaErrorNotSupported;
+  const int nb = oa_tg_nb(nj);
+  if (((PM2 == nullptr) != (PX2 == nullptr)) || nk < TG_KS || (nk % TG_KS)) return cudaErrorNotSupported;
   const int stages = tg_stages(nt, nb, false);
   if (stages < 2) return cudaErrorNotSupported;
+  const int njt = (nj + nb - 1) / nb;
   CUtensorMap tx1, tm1, tx2, tm2;
-  if (!tg_map(&tx1, PX1, nt, nk, ldx, TG_KS) || !tg_map(&tm1, PM1, nt, nk, nb, TG_KS)) return cudaErrorNotSupported;
+  if (!tg_map(&tx1, PX1, nt, nk, ldx, TG_KS) || !tg_map(&tm1, PM1, nt, nk, njt * nb, TG_KS)) return cudaErrorNotSupported;
   const int nterm = PM2 ? 2 : 1;
   if (nterm == 2) {
-    if (!tg_map(&tx2, PX2, nt, nk, ldx, TG_KS) || !tg_map(&tm2, PM2, nt, nk, nb, TG_KS)) return cudaErrorNotSupported;
+    if (!tg_map(&tx2, PX2, nt, nk, ldx, TG_KS) || !tg_map(&tm2, PM2, nt, nk, njt * nb, TG_KS)) return cudaErrorNotSupported;
   } else {
     tx2 = tx1; tm2 = tm1;
   }
   const size_t sm = tg_smem(nt, nb, stages, false);
-  const long ntile = (ncol + TG_M - 1) / TG_M;
+  const long ntile = (ncol + TG_M - 1) / TG_M * njt;
   int nsm = 148;
   {
     int dev = 0;
@@ -646,7 +653,7 @@ cudaError_t oa_tbwd(cudaStream_t s, int nt, const bf16* PM1, const bf16* PX1, do
   if (nt == NTT && nb == NBB) {                                                                                \
     e = oa_smem_limit(k_tbwd<NTT, NBB>);           \
     if (e != cudaSuccess) return e;                                                                            \
-    k_tbwd<NTT, NBB><<<grid, TB_THREADS, sm, s>>>(tx1, tm1, tx2, tm2, nterm, a1_kx0, a1_rest, a2, nj, nk, ncol,  \
+    k_tbwd<NTT, NBB><<<grid, TB_THREADS, sm, s>>>(tx1, tm1, tx2, tm2, nterm, a1_kx0, a1_rest, a2, nj, njt, nk, ncol, \
                                                   kx0_cols, stages, out, err_flag, yadd, cond);                \
     e = cudaGetLastError();                                                                                    \
   }

@@ -1,0 +1,60 @@
+"""Sizes off the presets: every kind of two-pass grid length (even and odd,
+with and without the band-pruned first DFT, the row-split FP64 density pass),
+odd state counts, state counts of several product tiles, and the one-block
+Newton-Schulz iteration, against the oracle."""
+import math
+
+import numpy as np
+import pytest
+
+from openatom_b200.system import make_system
+from oracle import cp_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.max(np.abs(np.asarray(a) - b)) / max(float(np.max(np.abs(b))), 1e-300))
+
+
+def grid_system(n, nstate, box=7.0, frac=1.0):
+    """A 2-water cell whose state sphere reaches kmax = (n - 1) / 4 (times frac).
+    The radius lies 0.3 above it: no squared radius of the states or of the
+    density is then a whole number, so that no point lies on the cutoff, where
+    the last bit of |g|^2 would decide which sphere it is in."""
+    kmax = max(2.5, frac * ((n - 1) // 4)) + 0.3
+    return make_system("w2", seed=3, nfft=(n, n, n), nstate=nstate, box=box,
+                       ecut_ry=(kmax * 2.0 * math.pi / box) ** 2)
+
+
+@pytest.mark.parametrize("nstate", [129, 150, 199, 256, 300])
+def test_products_of_several_tiles(nstate):
+    """S (symmetric tiles), Lambda, the two-term backward product and the
+    rotation: FP64 to rounding; split-BF16 to the rounding of FP32 sums of six
+    products (three per term) over the longest inner dimension, a random walk
+    of sqrt(6 nstate) steps of 2^-24 with a factor 4."""
+    import torch
+    from openatom_b200.gpu import CPContext
+    s = make_system("w4", seed=9, nstate=nstate, pseudo="analytic")
+    rng = np.random.default_rng(2)
+    F = (rng.standard_normal(s.psi.shape) + 1j * rng.standard_normal(s.psi.shape)) * 0.1
+    T = np.eye(nstate) + 1e-3 * rng.standard_normal((nstate, nstate))
+    fref, lref = O.lambda_step(s.psi, F, T, s)
+    ps = O.kx0_scale(s.psi, s, 1.0 / math.sqrt(2.0))
+    sref = O.pc_forward(ps, ps, s, 2.0)
+    psi, Fg, Tg = (torch.from_numpy(a).cuda() for a in (s.psi, F, T))
+    for precision, tol in (("fp64", 1e-12), ("mixed", 4 * math.sqrt(6 * nstate) * 2.0**-24)):
+        c = CPContext(s, precision)
+        S = torch.zeros(nstate, nstate, dtype=torch.float64, device="cuda")
+        lam, gam, out, rot = torch.zeros_like(S), torch.zeros_like(S), torch.zeros_like(psi), torch.zeros_like(psi)
+        fwd, bwd = (c.pc_forward, c.pc_backward) if precision == "fp64" else (c.pc_forward_mixed, c.pc_backward_mixed)
+        c.pc_forward(psi, psi, 2.0, 0.5, S)
+        fwd(psi, Fg, 1.0, 1.0, lam)
+        c.small_gemm(Tg, torch.from_numpy(lref).cuda(), 1.0, gam)
+        bwd(gam, psi, -0.5, -1.0, out, M2=Tg, X2=Fg, a2=1.0)
+        c.pc_backward(Tg, psi, 1.0, 1.0, rot)
+        c.check()
+        assert rel(S.cpu().numpy(), sref) < 1e-12 and torch.equal(S, S.T)
+        assert rel(lam.cpu().numpy(), lref) < tol
+        assert rel(out.cpu().numpy(), fref) < tol
+        assert rel(rot.cpu().numpy(), T.T @ s.psi) < 1e-12
