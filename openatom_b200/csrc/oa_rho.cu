@@ -812,7 +812,7 @@ k_rho_div_z(double2* __restrict__ dz, const double2* __restrict__ dzh, size_t fs
 
 cudaError_t oa_rho2_fwd(cudaStream_t s, int n, int nz, const double* rho, double scale, const double2* tw,
                         double2* dz, int ldl_d, int nf, size_t fin, size_t fout);
-cudaError_t oa_rho2_bwd(cudaStream_t s, int n, int nz, const double2* dz, int ldl_d, const double2* tw,
+cudaError_t oa_rho2_bwd(cudaStream_t s, int n, int nz, double2* dz, int ldl_d, const double2* tw,
                         const double* vxc, void* vks, int fp64, int nf, size_t fin, size_t fout);
 
 __global__ void k_phase_tables(const double* __restrict__ pos, int natm, int ktab, double tpi_l, double2* __restrict__ phase) {
@@ -890,7 +890,7 @@ static cudaError_t rho_xy_fwd(oa_ctx* c, cudaStream_t s, const double* src, doub
 
 // x-y inverse of nf fields of density z-lines into real grids (+ vxc when
 // not null), in FP64 or the compute precision
-static cudaError_t rho_xy_bwd(oa_ctx* c, cudaStream_t s, const double2* src, const double* vxc, void* dst, int fp64,
+static cudaError_t rho_xy_bwd(oa_ctx* c, cudaStream_t s, double2* src, const double* vxc, void* dst, int fp64,
                               int nf, size_t fin, size_t fout) {
   cudaError_t e = c->nx == c->ny
                       ? oa_rho2_bwd(s, c->nx, c->nz, src, c->ldl_d, c->tw_x, vxc, dst, fp64, nf, fin, fout)
@@ -954,7 +954,7 @@ static cudaError_t gga_front(oa_ctx* c, cudaStream_t s) {
   const size_t fz = (size_t)c->nz * c->ldl_d, fr = (size_t)c->npts;
   cudaError_t e;
   if ((e = gga_z(c, s, 0)) != cudaSuccess) return e;
-  if ((e = rho_xy_bwd(c, s, (const double2*)c->dzg, nullptr, c->grad, 1, 3, fz, fr)) != cudaSuccess) return e;
+  if ((e = rho_xy_bwd(c, s, (double2*)c->dzg, nullptr, c->grad, 1, 3, fz, fr)) != cudaSuccess) return e;
   k_rho_gga<<<oa_rho_xc_nblk(), OA_NTHREADS, 0, s>>>(c->rho, c->grad, fr, c->gga_cut, c->vxc,
                                                       c->red + oa_rho_gga_red_off(c));
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1020,5 +1020,5 @@ cudaError_t oa_launch_rho_fft_hart(oa_ctx* c, cudaStream_t s) {
   if (c->eesl && forces && (e = oa_launch_eesl_forces(c, s)) != cudaSuccess) return e;
   // white-byrd: V_KS z-lines -= z^-1 (i g . h(g))
   if (c->gga && (e = gga_z(c, s, 1)) != cudaSuccess) return e;
-  return rho_xy_bwd(c, s, (const double2*)c->dz, c->vxc, c->vks, c->precision == OA_FP64, 1, 0, 0);
+  return rho_xy_bwd(c, s, (double2*)c->dz, c->vxc, c->vks, c->precision == OA_FP64, 1, 0, 0);
 }

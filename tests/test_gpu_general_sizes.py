@@ -27,6 +27,23 @@ def grid_system(n, nstate, box=7.0, frac=1.0):
                        ecut_ry=(kmax * 2.0 * math.pi / box) ** 2)
 
 
+@pytest.mark.parametrize("n", [15, 60, 90, 120, 150])
+def test_density_path_lengths(n):
+    """The density transforms and the Hartree / XC path off the preset lengths."""
+    import torch
+    from openatom_b200.gpu import CPContext
+    s = grid_system(n, 2, frac=0.5)
+    ctx = CPContext(s, "fp64")
+    vks = torch.zeros(n, n, n, dtype=torch.float64, device="cuda")
+    ctx.state_fft_fwd(torch.from_numpy(s.psi).cuda())
+    ctx.vks_build(vks)
+    en = ctx.energies()
+    _, vref, eref = O.vks_build(O.state_g_to_r(s.psi, s), s)
+    assert rel(vks.cpu().numpy(), vref) < 1e-10
+    for k in ("EHART", "EEXT", "EEXC", "MUXC"):
+        assert abs(en[k] - eref[k]) <= 1e-10 * max(1.0, abs(eref[k])), k
+
+
 @pytest.mark.parametrize("nstate", [129, 150, 199, 256, 300])
 def test_products_of_several_tiles(nstate):
     """S (symmetric tiles), Lambda, the two-term backward product and the
