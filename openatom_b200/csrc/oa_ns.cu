@@ -57,7 +57,8 @@ struct NscProd {
   double alpha, diag;
 };
 __device__ __forceinline__ void nsc_gemm_blk(NscProd p0, NscProd p1, int np, int n, const NscGeom& G, int r0, int c0,
-                                             double* Xs, double* Ys, const double* __restrict__ Aold, double* err) {
+                                             double* Xs, double* Ys, const double* __restrict__ Aold, double* err,
+                                             bool y_is_c0 = false) {
   const int ldx = G.npad + 4, ldy = G.BC + 4;
   const size_t xstage = (size_t)G.BR * ldx, ystage = (size_t)G.npad * ldy;
   __syncthreads();  // the previous products are done with Xs / Ys
@@ -82,6 +83,14 @@ __device__ __forceinline__ void nsc_gemm_blk(NscProd p0, NscProd p1, int np, int
   asm volatile("cp.async.commit_group;\n" ::);
   asm volatile("cp.async.wait_group 0;\n" ::);
   __syncthreads();
+  if (y_is_c0) {
+    // Y was staged from B: the first iteration's C = 3I - B
+    for (int i = threadIdx.x; i < G.npad * G.BC; i += blockDim.x) {
+      const int k = i / G.BC, j = i - k * G.BC;
+      if (k < n && c0 + j < n) Ys[k * ldy + j] = (k == c0 + j ? 3.0 : 0.0) - Ys[k * ldy + j];
+    }
+    __syncthreads();
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rt_n = G.BR / 8, ct_n = G.BC / 8;
   double e = 0.0;
@@ -176,14 +185,29 @@ k_ortho_ns_cluster(const double* __restrict__ S, int n, double bscale, double to
   int it = 0;
   double err = 1.0;
   while (true) {
+    double e = 0.0;
+    if (it == 0) {
+      // A = I: C = 3I - B, so Bn = B (3I - B) / 2 and An = (3I - B) / 2 need
+      // neither the first product nor its cluster barrier
+      const NscProd p{B, B, Bn, 0.5, 0.0};
+      nsc_gemm_blk(p, p, 1, n, G, r0, c0, Xs, Ys, nullptr, nullptr, true);
+      for (int i = threadIdx.x; i < G.BR * G.BC; i += blockDim.x) {
+        const int r = r0 + i / G.BC, c = c0 + i % G.BC;
+        if (r >= n || c >= n) continue;
+        const size_t o = (size_t)r * n + c;
+        const double v = 0.5 * ((r == c ? 3.0 : 0.0) - B[o]), d = (r == c ? 1.0 : 0.0) - v;
+        An[o] = v;
+        e += d * d;
+      }
+    } else {
     // C = 3I - A B (own rows)
     nsc_gemm_blk(NscProd{A, B, Cm, -1.0, 3.0}, NscProd{A, B, Cm, -1.0, 3.0}, 1, n, G, r0, c0, Xs, Ys, nullptr,
                  nullptr);
     __threadfence();
     cl.sync();
     // Bn = B C / 2 ; An = C A / 2 (own rows), with the error partial
-    double e = 0.0;
     nsc_gemm_blk(NscProd{B, Cm, Bn, 0.5, 0.0}, NscProd{Cm, A, An, 0.5, 0.0}, 2, n, G, r0, c0, Xs, Ys, A, &e);
+    }
     e = nsc_block_sum(e, sh);
     if (threadIdx.x == 0) errpart[me] = e;
     __threadfence();
@@ -207,6 +231,114 @@ k_ortho_ns_cluster(const double* __restrict__ S, int n, double bscale, double to
     status[1] = (err <= tol) ? 1 : 0;
     errv[0] = err;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Up to NSS_MAXN states: the same iteration in one block, with A, B, C and the
+// new A, B in shared memory.  The products are short (32 states: 16 tiles of
+// 8 DMMAs), so what a cluster iteration costs is its two cluster barriers and
+// the L2 round trips between them; one block replaces them by block barriers.
+// Measured per call at 32 states (5 iterations): cluster 33 us, one block
+// 9 us; the products take over between 48 and 64 states, where one SM's FP64
+// tensor rate (2 us a product at 64) loses to sixteen SMs.
+// ---------------------------------------------------------------------------
+#define NSS_MAXN 48
+
+__device__ __forceinline__ void nss_tile(const double* X, const double* Y, int ld, int np, int rt, int ct, double& d0,
+                                         double& d1) {
+  const int lane = threadIdx.x & 31;
+  const double* xr = X + (rt * 8 + (lane >> 2)) * ld + (lane & 3);
+  const double* yc = Y + (lane & 3) * ld + ct * 8 + (lane >> 2);
+  d0 = 0.0;
+  d1 = 0.0;
+  for (int k4 = 0; k4 < np; k4 += 4) nsc_dmma(d0, d1, xr[k4], yc[k4 * ld]);
+}
+
+__global__ void __launch_bounds__(NSC_THREADS)
+k_ortho_ns_block(const double* __restrict__ S, int n, double bscale, double tol, int max_iter,
+                 double* __restrict__ T, int* __restrict__ status, double* __restrict__ errv) {
+  extern __shared__ __align__(16) double nsc_smem[];
+  __shared__ double sh[NSC_THREADS / 32];
+  const int np = (n + 7) & ~7, ld = np + 4, nt = np / 8;
+  const size_t sz = (size_t)np * ld;
+  double *A = nsc_smem, *B = A + sz, *Cm = B + sz, *An = Cm + sz, *Bn = An + sz;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double dmax = 0.0;
+  for (int i = threadIdx.x; i < np * np; i += NSC_THREADS) {
+    const int r = i / np, c = i - r * np;
+    double b = 0.0, a = 0.0;
+    if (r < n && c < n) {
+      const double s = S[(size_t)r * n + c];
+      a = r == c ? 1.0 : 0.0;
+      b = s * bscale;
+      dmax = fmax(dmax, fabs(s - (r == c ? 1.0 / bscale : 0.0)));
+    }
+    A[r * ld + c] = a;
+    B[r * ld + c] = b;
+  }
+  dmax = nsc_block_max(dmax, sh);
+  if (threadIdx.x == 0) errv[1] = dmax;
+  int it = 0;
+  double err = 1.0;
+  while (true) {
+    __syncthreads();
+    // C = 3I - A B
+    for (int t = warp; t < nt * nt; t += NSC_THREADS / 32) {
+      const int rt = t % nt, ct = t / nt;
+      double d0, d1;
+      nss_tile(A, B, ld, np, rt, ct, d0, d1);
+      const int i = rt * 8 + (lane >> 2), j = ct * 8 + 2 * (lane & 3);
+      Cm[i * ld + j] = (i == j && i < n ? 3.0 : 0.0) - d0;
+      Cm[i * ld + j + 1] = (i == j + 1 && i < n ? 3.0 : 0.0) - d1;
+    }
+    __syncthreads();
+    // Bn = B C / 2, An = C A / 2 and the change of A
+    double e = 0.0;
+    for (int t = warp; t < 2 * nt * nt; t += NSC_THREADS / 32) {
+      const int p = t / (nt * nt), tt = t - p * nt * nt;
+      const int rt = tt % nt, ct = tt / nt;
+      double d0, d1;
+      nss_tile(p ? Cm : B, p ? A : Cm, ld, np, rt, ct, d0, d1);
+      const int o = (rt * 8 + (lane >> 2)) * ld + ct * 8 + 2 * (lane & 3);
+      d0 *= 0.5;
+      d1 *= 0.5;
+      if (p) {
+        const double x = A[o] - d0, y = A[o + 1] - d1;
+        e += x * x + y * y;
+      }
+      (p ? An : Bn)[o] = d0;
+      (p ? An : Bn)[o + 1] = d1;
+    }
+    e = nsc_block_sum(e, sh);
+    ++it;
+    err = sqrt(e / ((double)n * n));
+    { double* t = A; A = An; An = t; t = B; B = Bn; Bn = t; }
+    if (!(err > tol && it < max_iter)) break;
+  }
+  for (int i = threadIdx.x; i < n * n; i += NSC_THREADS) {
+    const int r = i / n, c = i - r * n;
+    T[i] = A[r * ld + c];
+  }
+  if (threadIdx.x == 0) {
+    status[0] = it;
+    status[1] = (err <= tol) ? 1 : 0;
+    errv[0] = err;
+  }
+}
+
+static size_t nss_smem_bytes(int n) {
+  const int np = (n + 7) & ~7;
+  return (size_t)5 * np * (np + 4) * sizeof(double);
+}
+
+// cudaErrorNotSupported above NSS_MAXN states
+cudaError_t oa_launch_ortho_ns_block(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
+                                     double* T, int* status, double* errv) {
+  if (n > NSS_MAXN) return cudaErrorNotSupported;
+  const cudaError_t e = oa_smem_limit(k_ortho_ns_block);
+  if (e != cudaSuccess) return e;
+  k_ortho_ns_block<<<1, NSC_THREADS, nss_smem_bytes(n), s>>>(S, n, bscale, tol, max_iter, T, status, errv);
+  return cudaGetLastError();
 }
 
 // Cluster size for the Newton-Schulz kernel on this device (16 where the

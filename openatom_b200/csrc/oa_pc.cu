@@ -608,6 +608,8 @@ int oa_ns_grid(int n, int device) {
   return g;
 }
 
+cudaError_t oa_launch_ortho_ns_block(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
+                                     double* T, int* status, double* errv);
 cudaError_t oa_launch_ortho_ns_cluster(cudaStream_t s, const double* S, int n, double bscale, double tol,
                                        int max_iter, double* work, double* T, int* status, double* errv, int cs);
 
@@ -615,6 +617,9 @@ cudaError_t oa_launch_ortho_ns_cluster(cudaStream_t s, const double* S, int n, d
 // (oa_ns.cu) on a cluster of -grid blocks
 cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
                                double* work /* 5 n^2 + grid */, double* T, int* status, double* errv, int grid) {
+  // few states: one block (oa_ns.cu)
+  const cudaError_t eb = oa_launch_ortho_ns_block(s, S, n, bscale, tol, max_iter, T, status, errv);
+  if (eb != cudaErrorNotSupported) return eb;
   if (grid < 0) return oa_launch_ortho_ns_cluster(s, S, n, bscale, tol, max_iter, work, T, status, errv, -grid);
   const size_t nn = (size_t)n * n;
   double* A0 = work; double* A1 = A0 + nn; double* B0 = A1 + nn; double* B1 = B0 + nn; double* Cm = B1 + nn;

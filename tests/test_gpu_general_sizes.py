@@ -75,3 +75,18 @@ def test_products_of_several_tiles(nstate):
         assert rel(lam.cpu().numpy(), lref) < tol
         assert rel(out.cpu().numpy(), fref) < tol
         assert rel(rot.cpu().numpy(), T.T @ s.psi) < 1e-12
+
+
+@pytest.mark.parametrize("nstate", [1, 2, 7, 8, 31, 32, 48, 50, 51])
+def test_newton_schulz_sizes(nstate):
+    import torch
+    from openatom_b200.gpu import CPContext
+    s = make_system("w2", seed=9, nstate=nstate, pseudo="analytic")
+    e = np.random.default_rng(nstate).standard_normal((nstate, nstate)) * 5e-3
+    S = 2.0 * np.eye(nstate) + e + e.T
+    T = torch.zeros(nstate, nstate, dtype=torch.float64, device="cuda")
+    it, err, ok, smax = CPContext(s, "fp64").ortho_invsqrt(torch.from_numpy(S).cuda(), T, 1e-15, 100, with_smax=True)
+    tref, iref, _ = O.newton_schulz(S, 1e-15, 100)
+    assert ok and abs(it - iref) <= 1
+    assert rel(T.cpu().numpy(), tref) < 1e-13
+    assert abs(smax - np.max(np.abs(S - 2.0 * np.eye(nstate)))) < 1e-15
