@@ -9,12 +9,13 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liboa_gpu.so")
-SOURCES = ["oa_state.cu", "oa_pencil.cu", "oa_pair_plane.cu", "oa_rho.cu", "oa_rho_pencil.cu", "oa_pc.cu", "oa_dgemm.cu", "oa_ns.cu", "oa_umma.cu", "oa_tgemm.cu", "oa_ozaki.cu", "oa_nl.cu", "oa_ions.cu", "oa_eesl.cu", "oa_step.cu", "oa_noalloc.cu", "oa_abi.cu"]
+SOURCES = ["oa_state.cu", "oa_pencil.cu", "oa_pp.cu", "oa_pp_f0.cu", "oa_pp_f1.cu", "oa_pp_f2.cu", "oa_pp_f3.cu", "oa_pp_d0.cu", "oa_pp_d1.cu", "oa_pp_d2.cu", "oa_pp_d3.cu", "oa_pp_ees_f.cu", "oa_pp_ees_d.cu", "oa_rho.cu", "oa_rho_pencil.cu", "oa_pc.cu", "oa_dgemm.cu", "oa_ns.cu", "oa_umma.cu", "oa_tgemm.cu", "oa_ozaki.cu", "oa_nl.cu", "oa_ions.cu", "oa_eesl.cu", "oa_step.cu", "oa_noalloc.cu", "oa_abi.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -35,12 +36,12 @@ def build(verbose: bool = False, force: bool = False) -> str:
             return LIB
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    objs = []
     flags = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-rdc=false",
                     "-I", os.path.join(ROOT, "include"), "-I", CSRC]
     if verbose:
         flags += ["-Xptxas", "-v"]
-    for s in srcs:
+
+    def compile_one(s):
         o = os.path.join(objdir, os.path.basename(s) + ".o")
         cmd = [nvcc()] + flags + ["-c", s, "-o", o]
         r = subprocess.run(cmd, capture_output=True, text=True)
@@ -48,7 +49,10 @@ def build(verbose: bool = False, force: bool = False) -> str:
             sys.stderr.write(r.stdout + r.stderr)
         if r.returncode:
             raise RuntimeError(f"nvcc failed on {s}")
-        objs.append(o)
+        return o
+
+    with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(compile_one, srcs))
     cmd = [nvcc()] + ARCH + ["-shared", "-o", LIB] + objs + ["-lcudart"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode:

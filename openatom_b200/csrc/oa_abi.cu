@@ -4,6 +4,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <algorithm>
+#include <atomic>
 #include <vector>
 #include <cuda_bf16.h>
 #include "oa_internal.h"
@@ -27,7 +28,9 @@ int oa_ns_cluster_size(int n);
 cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
                                double* work, double* T, int* status, double* errv, int grid);
 int oa_integrate_nblk(int ng, int nstate);
-int oa_pair_plane_supported(int n, int nkx, int nlines, int ldl);
+cudaError_t oa_pair_plane_shape(oa_ctx* c, int* dbps, int* vbps, int* split);
+cudaError_t oa_ees_pair_shape(oa_ctx* c, int* bps);
+int oa_plane2_supported(int n);
 cudaError_t oa_launch_integrate(cudaStream_t s, const double2* F, double2* V, double2* P, const double2* P_in,
                                 const int* sel, const double* cmass, int ng, int nstate, int r0, int r1, int iend,
                                 double dt, int complete_prev, double* kepart, int nblk);
@@ -80,6 +83,31 @@ extern "C" const char* oa_gpu_last_error(void) { return g_err; }
   do {                                                  \
     if (!(cond)) { oa_set_error(msg, __FILE__, __LINE__); return OA_ERR_BAD_ARG; } \
   } while (0)
+
+// open-addressing set of (kernel, device); a full probe sequence just means
+// that the limit is set again at that launch
+static std::atomic<uintptr_t> g_smem_set[1024];
+static uintptr_t smem_key(const void* kernel) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return (uintptr_t)kernel ^ ((uintptr_t)(dev + 1) << 56);
+}
+bool oa_smem_raised(const void* kernel) {
+  const uintptr_t k = smem_key(kernel);
+  for (size_t i = 0, h = (k >> 4) * 0x9E3779B97F4A7C15ull >> 54; i < 8; ++i) {
+    const uintptr_t v = g_smem_set[(h + i) & 1023].load(std::memory_order_acquire);
+    if (v == k) return true;
+    if (v == 0) return false;
+  }
+  return false;
+}
+void oa_smem_mark(const void* kernel) {
+  const uintptr_t k = smem_key(kernel);
+  for (size_t i = 0, h = (k >> 4) * 0x9E3779B97F4A7C15ull >> 54; i < 8; ++i) {
+    uintptr_t v = 0;
+    if (g_smem_set[(h + i) & 1023].compare_exchange_strong(v, k, std::memory_order_acq_rel) || v == k) return;
+  }
+}
 
 // FP64-accurate int8 tensor-core products of the mixed form (oa_ozaki.cu)
 struct oa_oz;
@@ -200,16 +228,33 @@ static bool column_runs(const oa_system_desc* d, int nkx, std::vector<int>* out)
   return true;
 }
 
-static int pick_groups(int nz, int nstate, int bps, int nsm, int fixed = 0) {
-  // minimise ceil(nz g / (nsm bps)) * (ceil(nstate / g) + fixed): waves of
-  // blocks times the items each block runs, plus a fixed per-block cost in
-  // items (pipeline fill and drain, twiddle and table loads)
+static int pick_groups(int nz, int nstate, int bps, int nsm) {
+  // minimise ceil(nz g / (nsm bps)) * ceil(nstate / g): waves of blocks times
+  // the states each block runs
   int best = 1;
   long bestc = -1;
   for (int g = 1; g <= 32 && g <= nstate; ++g) {
     const long waves = (nz * (long)g + (long)nsm * bps - 1) / ((long)nsm * bps);
-    const long cost = waves * ((nstate + g - 1) / g + fixed);
+    const long cost = waves * ((nstate + g - 1) / g);
     if (bestc < 0 || cost < bestc) { bestc = cost; best = g; }
+  }
+  return best;
+}
+
+// State groups of a state-pair kernel: blocks = nplane * groups on nsm * bps
+// slots, np / groups pairs each (split evenly, one more or less) plus a fixed
+// cost of 0.6 pairs (tables, first loads, sums).  Over the group counts 1-24
+// measured at fourteen lengths from 24 to 160, both forms, this picks the
+// fastest or one within 3% of it; whole waves matter most (108 planes, 64
+// pairs, two blocks per SM: 2.92 waves of 8 groups 288 us, 1.82 of 5 304 us).
+static int pick_pair_groups(int nplane, int np, int bps, int nsm) {
+  int best = 1;
+  double bestc = -1.0;
+  if (bps < 1) bps = 1;
+  for (int g = 1; g <= 32 && g <= np; ++g) {
+    const long waves = (nplane * (long)g + (long)nsm * bps - 1) / ((long)nsm * bps);
+    const double cost = (double)waves * ((double)np / g + 0.6);
+    if (bestc < 0.0 || cost < bestc) { bestc = cost; best = g; }
   }
   return best;
 }
@@ -222,6 +267,7 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
   OA_ARG_CHECK(d->natm == 0 || d->atm_type, "null atm_type");
   for (int a = 0; a < d->natm; ++a) OA_ARG_CHECK(d->atm_type[a] >= 0 && d->atm_type[a] < d->ntype, "atom type out of range");
   *out = nullptr;
+  for (auto& v : g_smem_set) v.store(0, std::memory_order_release);
   oa_ctx_full* F = (oa_ctx_full*)calloc(1, sizeof(oa_ctx_full));
   if (!F) return OA_ERR_CUDA;
   oa_ctx* c = &F->c;
@@ -273,10 +319,7 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     if (bps < 1) bps = 1;
   }
   c->ngroup = pick_groups(d->nz, d->nstate, bps, nsm);
-  // the state-pair kernels software-pipeline the pairs of a block: a fixed
-  // cost of about two pairs per block, which is what the autotuner's
-  // measurements over 8-32 water systems on 64^3-108^3 grids imply
-  c->ngroup_pair = pick_groups(d->nz, (d->nstate + 1) / 2, 1, nsm, 2);
+  c->ngroup_pair = 1;
   c->pair_kymax = 0;
   c->z_ext = 0;
   for (int l = 0; l < d->nlines; ++l) {
@@ -357,12 +400,34 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     c->zbuf_bytes = (size_t)d->nstate * d->nz * c->ldl * csz;
     TRY(cudaMalloc(&c->zbuf, c->zbuf_bytes));
     {
+      // state-pair kernels: lines in column runs, room for psi(r) of all
+      // states (without it the per-state kernels redo the forward transforms)
       std::vector<int> runs;
-      if (precision == OA_MIXED && d->nx == d->ny &&
-          oa_pair_plane_supported(d->nx, c->nkx_s, d->nlines, c->ldl) && column_runs(d, c->nkx_s, &runs))
-        TRY(upload(&c->pair_cols, runs.data(), runs.size()));
+      const bool pairs = d->nx == d->ny && column_runs(d, c->nkx_s, &runs);
+      if (pairs) TRY(upload(&c->pair_cols, runs.data(), runs.size()));
+      if (pairs || (d->nx == d->ny && oa_plane2_supported(d->nx))) {
+        if (cudaMalloc(&c->psir, (size_t)(d->nstate + 1) / 2 * 2 * c->npts * rsz) != cudaSuccess) {
+          c->psir = nullptr;
+          cudaGetLastError();
+        }
+      }
+      int dbps = 1, vbps = 1, split = 1;
+      const int npair = (d->nstate + 1) / 2;
+      c->pair_on = c->pair_cols != nullptr;
+      if (oa_pair_plane_shape(c, &dbps, &vbps, &split) == cudaSuccess) {
+        c->ngroup_pair = pick_pair_groups(d->nz * split, npair, dbps, nsm);
+        c->ngroup_vks = pick_pair_groups(d->nz, npair, vbps, nsm);
+      } else {
+        cudaGetLastError();
+        c->pair_on = 0;
+        if (c->psir && !(d->nx == d->ny && oa_plane2_supported(d->nx))) {
+          cudaFree(c->psir);
+          c->psir = nullptr;
+        }
+        c->ngroup_pair = pick_pair_groups(d->nz, npair, 1, nsm);
+      }
     }
-    if (c->pair_cols) {
+    if (c->pair_on && precision == OA_MIXED) {
       // charge partials of the z forward pass (state x 16-line block) and of
       // the pair density pass (group x plane) for the density renormalisation
       c->nq = d->nstate * ((d->nlines + OA_LB - 1) / OA_LB);
@@ -377,8 +442,6 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
       TRY(cudaMalloc(&c->rho_part, (size_t)ng * c->npts * sizeof(double)));
       c->rho_groups_cap = ng;
     }
-    if (d->nx == d->ny && oa_pencil_supported(d->nx))
-      TRY(cudaMalloc(&c->psir, (size_t)(d->nstate + 1) / 2 * 2 * c->npts * rsz));
     TRY(cudaMalloc(&c->rho, (size_t)c->npts * sizeof(double)));
     TRY(cudaMalloc(&c->vxc, (size_t)c->npts * sizeof(double)));
     TRY(cudaMalloc(&c->vks, (size_t)c->npts * rsz));
@@ -922,7 +985,7 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
   const int gs = t->group_state ? t->group_state : c->ngroup;
   const int gp = t->group_pair ? t->group_pair : c->ngroup_pair;
   const int need = gs > gp ? gs : gp;
-  if (need > c->rho_groups_cap || (c->pair_cols && gp * c->nz > c->nq2_cap)) {
+  if (need > c->rho_groups_cap || (c->qpart && gp * c->nz > c->nq2_cap)) {
     OA_CUDA_TRY(cudaDeviceSynchronize());
     if (need > c->rho_groups_cap) {
       double* r = nullptr;
@@ -931,7 +994,7 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
       c->rho_part = r;
       c->rho_groups_cap = need;
     }
-    if (c->pair_cols && gp * c->nz > c->nq2_cap) {
+    if (c->qpart && gp * c->nz > c->nq2_cap) {
       double* q = nullptr;
       OA_CUDA_TRY(cudaMalloc(&q, (size_t)gp * c->nz * sizeof(double)));
       cudaFree(c->qpart2);
@@ -941,7 +1004,7 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
   }
   c->ngroup = gs;
   c->ngroup_pair = gp;
-  if (c->pair_cols) c->nq2 = gp * c->nz;
+  if (c->qpart) c->nq2 = gp * c->nz;
   if (t->dgemm_kblocks) p->nkb = t->dgemm_kblocks;
   if (t->tgemm_kblocks) p->umax_kb = t->tgemm_kblocks;
   if (t->fft_path) c->fft_runtime = t->fft_path == 2 ? 1 : 0;
@@ -960,7 +1023,7 @@ extern "C" oa_status oa_gpu_sizes(const oa_ctx* c, long* out) {
   // graphed step): state_fft_fwd 3 + vks_build 5 + nl_sf 7 + vks_apply 4 + lambda 4 +
   // integrate 3 + S 2 + Newton-Schulz 1 + Psi T 1
   out[9] = 3 + 5 + 7 + 4 + 4 + 3 + 2 + 1 + 1;
-  out[10] = c->pair_cols ? 1 : 0;  // state-pair plane kernels in use (mixed form)
+  out[10] = c->pair_on && !c->fft_runtime ? 1 : 0;  // state-pair plane kernels in use
   out[11] = c->ngroup_pair;
   out[12] = (c->precision == OA_MIXED && c->nstate <= 128) ? 1 : 0;  // int8 overlap / rotation available
   return OA_OK;
@@ -1364,13 +1427,19 @@ extern "C" oa_status oa_gpu_ees_init(oa_ctx* c, int na, int nb, int nc, int orde
   TRYE(upload(&e->dyp, (const double2*)dyp_host, (size_t)c->ng));
   TRYE(cudaMalloc(&e->idx, (size_t)c->natm_nl * 3 * order * sizeof(int)));
   TRYE(cudaMalloc(&e->mn, (size_t)c->natm_nl * 3 * order * sizeof(double)));
-  TRYE(cudaMalloc(&e->zpart, (size_t)c->nstate * c->natm_nl * order * sizeof(double)));
+  TRYE(cudaMalloc(&e->zpart, (size_t)c->nstate * c->natm_nl * order * order * sizeof(double)));
   TRYE(cudaMalloc(&e->zmat, (size_t)c->nstate * c->natm_nl * sizeof(double)));
   TRYE(cudaMalloc(&e->zs, (size_t)c->nstate * c->natm_nl * sizeof(double)));
   TRYE(cudaMalloc(&e->enl, (size_t)c->nstate * sizeof(double)));
   TRYE(cudaMalloc(&e->dmn, (size_t)c->natm_nl * 3 * order * sizeof(double)));
-  TRYE(cudaMalloc(&e->fpart, (size_t)c->nstate * c->natm_nl * order * 3 * sizeof(double)));
+  TRYE(cudaMalloc(&e->fpart, (size_t)c->nstate * c->natm_nl * order * order * 3 * sizeof(double)));
 #undef TRYE
+  int pbps = 1;
+  e->ngroup_pair = 0;
+  if (oa_ees_pair_shape(c, &pbps) == cudaSuccess)
+    e->ngroup_pair = pick_pair_groups(nc, (c->nstate + 1) / 2, pbps, pcx(c)->nsm);
+  else
+    cudaGetLastError();
   return OA_OK;
 }
 

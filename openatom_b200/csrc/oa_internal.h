@@ -11,34 +11,46 @@
 #define OA_LB 16          // z-lines per block in the z passes
 #define OA_MAX_SMEM (227 * 1024)
 
+// Kernels whose dynamic shared-memory limit has been raised on the current
+// device (oa_abi.cu).  The limit lasts as long as the device's context: every
+// oa_gpu_init forgets the set, so that contexts made after a device reset
+// raise it again.
+bool oa_smem_raised(const void* kernel);
+void oa_smem_mark(const void* kernel);
+
 // Raise a kernel's dynamic shared-memory limit to the most a block can have
 // beside its static shared memory.  The limit is a per-function setting that
 // all launches share (graphs holding systems of several sizes included), so
-// it is never lowered to one launch's need.
+// it is never lowered to one launch's need.  The two runtime calls cost about
+// a microsecond, a third of a launch: they are made once per kernel.
 template <typename K>
 static inline cudaError_t oa_smem_limit(K kernel) {
+  if (oa_smem_raised((const void*)kernel)) return cudaSuccess;
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, (const void*)kernel);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(OA_MAX_SMEM - a.sharedSizeBytes));
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(OA_MAX_SMEM - a.sharedSizeBytes));
+  if (e == cudaSuccess) oa_smem_mark((const void*)kernel);
+  return e;
 }
 
 // EES nonlocal path (nonlocal grid na x nb x nc, B-spline order)
 struct oa_ees {
   int na, nb, nc, order, ngroup;
+  int ngroup_pair;     // pair groups of the state-pair kernels (0: they do not take this grid)
   OaFftPlan pa, pb, pc;
   double2 *tw_a, *tw_b, *tw_c;
   void* zbuf;          // [nstate][nc][ldl] compute precision
   double2* dyp;        // [ng] d(g) y00 p(|g|)
   int* idx;            // [natm_nl][3][order]
   double* mn;          // [natm_nl][3][order]
-  double* zpart;       // [nstate][natm_nl][order]
+  double* zpart;       // [nstate][natm_nl][order] per stencil plane, or [order^2] per stencil row (pair kernels)
   double* zmat;        // [nstate][natm_nl]
   double* zs;          // [nstate][natm_nl]
   double* enl;         // [nstate]
   double* dmn;         // [natm_nl][3][order] B-spline derivative weights (ion dynamics)
-  double* fpart;       // [nstate][natm_nl][order][3] per-plane atom-force sums (ion dynamics)
+  double* fpart;       // [3] atom-force sums beside each zpart entry (ion dynamics)
 };
 
 // EES local pseudopotential and reciprocal Ewald path (oa_gpu_set_ees_local,
@@ -99,13 +111,15 @@ struct oa_ctx {
   int nkx_d;              // density half-spectrum columns (nx/2 + 1)
   int nlines_d, ldl_d;    // density z-lines (nkx_d * ny) and padded stride
   int ngroup;             // state groups in the plane kernels
-  int ngroup_pair;        // pair groups in the state-pair plane kernels
+  int ngroup_pair;        // pair groups of the state-pair density kernel (oa_tuning group_pair)
+  int ngroup_vks;         // pair groups of the state-pair V_KS kernel
   int rho_ngroup;         // groups summed in rho_part by the last density pass
-  int* pair_cols;         // [nkx_s] {first line, ky of the first line, lines, 0}: FP32 pair kernels
+  int* pair_cols;         // [nkx_s] {first line, ky of the first line, lines, 0} when the lines form column runs
+  int pair_on;            // the state-pair plane kernels take this system
   int pair_kymax;         // largest |ky| of the state lines
   int z_ext;              // largest kz count of a state line on either side (max of nneg, npos)
   void* psir;             // psi(r), compute precision: [nstate][nz][ny][nx] (two-pass kernels)
-                          // or [nstate/2][nz][ny][nx] pairs (state-pair kernels)
+                          // or the private pair layout of oa_pp.cuh (state-pair kernels)
   int psir_valid;         // the last density pass stored psir: 1 per state, 2 per pair
   double box, vol, ecut_psi, ecut_rho, alp_ewd;
   double gzvps_sum;
@@ -198,10 +212,10 @@ cudaError_t oa_launch_state_zbwd(oa_ctx* c, cudaStream_t s, const double2* psi, 
 cudaError_t oa_launch_rho_xc(oa_ctx* c, cudaStream_t s);
 cudaError_t oa_launch_rho_fft_hart(oa_ctx* c, cudaStream_t s);
 cudaError_t oa_launch_ees(oa_ctx* c, cudaStream_t s, const double2* psi, double2* fnl);
-cudaError_t oa_launch_ees_zreduce(oa_ctx* c, cudaStream_t s);
+cudaError_t oa_launch_ees_zreduce(oa_ctx* c, cudaStream_t s, int np);
 cudaError_t oa_launch_ees_bspline(oa_ctx* c, cudaStream_t s);
 cudaError_t oa_launch_nl_sf_force(oa_ctx* c, cudaStream_t s, const double* psi);
-cudaError_t oa_launch_ees_atom_force(oa_ctx* c, cudaStream_t s);
+cudaError_t oa_launch_ees_atom_force(oa_ctx* c, cudaStream_t s, int np);
 cudaError_t oa_launch_eesl_front(oa_ctx* c, cudaStream_t s);
 cudaError_t oa_launch_eesl_forces(oa_ctx* c, cudaStream_t s);
 void oa_eesl_free(oa_ctx* c);

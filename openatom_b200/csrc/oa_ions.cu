@@ -69,19 +69,19 @@ __global__ void k_nl_sf_force(const double2* __restrict__ y, const double2* __re
 }
 
 // EES nonlocal atom forces (eesEnergyAtmForcRchare's force loop,
-// cp_ees_nonlocal.C:1560-1720): F_a = -sum_s zs[s][a] sum over the stencil
-// planes of the gathered sums (x n_a / L, y n_b / L, z n_c / L), with zs the
+// cp_ees_nonlocal.C:1560-1720): F_a = -sum_s zs[s][a] sum over the np partials
+// (stencil planes or rows) of the gathered sums (x n_a / L, y n_b / L, z n_c / L), with zs the
 // scaled Z = 2 vnorm / V occ Z.  One block per nonlocal atom.
 __global__ void k_ees_atom_force(const double* __restrict__ fpart, const double* __restrict__ zs, int nstate,
-                                 int natm_nl, int order, const int* __restrict__ nl_atm, double sa, double sb,
+                                 int natm_nl, int np, const int* __restrict__ nl_atm, double sa, double sb,
                                  double sc, double* __restrict__ fnl) {
   __shared__ double sh[3 * 32];
   const int a = blockIdx.x;
   double f[3] = {0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < nstate * order; i += blockDim.x) {
-    const int s = i / order, jc = i - s * order;
+  for (int i = threadIdx.x; i < nstate * np; i += blockDim.x) {
+    const int s = i / np, j = i - s * np;
     const double z = zs[(size_t)s * natm_nl + a];
-    const double* fp = fpart + (((size_t)s * natm_nl + a) * order + jc) * 3;
+    const double* fp = fpart + (((size_t)s * natm_nl + a) * np + j) * 3;
     f[0] += z * fp[0];
     f[1] += z * fp[1];
     f[2] += z * fp[2];
@@ -245,13 +245,13 @@ static double ewald_self_bgr(const oa_ctx* c, const double* q_host) {
   return vself * (1.0 - erfc_x) + vbgr;
 }
 
-cudaError_t oa_launch_ees_atom_force(oa_ctx* c, cudaStream_t s) {
+cudaError_t oa_launch_ees_atom_force(oa_ctx* c, cudaStream_t s, int np) {
   oa_ions* io = c->ions;
   const oa_ees* e = c->ees;
   cudaError_t err = cudaMemsetAsync(io->fnl, 0, (size_t)3 * c->natm * sizeof(double), s);
   if (err != cudaSuccess) return err;
   if (c->natm_nl == 0) return cudaSuccess;
-  k_ees_atom_force<<<c->natm_nl, 128, 0, s>>>(e->fpart, e->zs, c->nstate, c->natm_nl, e->order, c->nl_atm,
+  k_ees_atom_force<<<c->natm_nl, 128, 0, s>>>(e->fpart, e->zs, c->nstate, c->natm_nl, np, c->nl_atm,
                                               (double)e->na / c->box, (double)e->nb / c->box, (double)e->nc / c->box,
                                               io->fnl);
   return cudaGetLastError();

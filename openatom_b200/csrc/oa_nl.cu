@@ -49,20 +49,25 @@ __global__ void k_nl_sf(const int* __restrict__ kx, const int* __restrict__ ky, 
 }
 
 // ENL per state and the scaled, transposed, negated Z for the force GEMM:
-// zt[a][s] = -2 vnorm_a / V Z[s][a]
-__global__ void k_nl_zscale(const double* __restrict__ Z, int nstate, int natm_nl, const int* __restrict__ nl_atm,
-                            const int* __restrict__ atm_type, const double* __restrict__ vnorm, double rvol,
-                            const double* __restrict__ occ, double* __restrict__ zt, double* __restrict__ enl) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// zt[a][s] = -2 vnorm_a / V Z[s][a].  One warp per state, lanes over the
+// atoms (a thread per state walked its atoms one dependent load at a time:
+// 14 us at 256 states and 64 atoms).
+__global__ void __launch_bounds__(128)
+k_nl_zscale(const double* __restrict__ Z, int nstate, int natm_nl, const int* __restrict__ nl_atm,
+            const int* __restrict__ atm_type, const double* __restrict__ vnorm, double rvol,
+            const double* __restrict__ occ, double* __restrict__ zt, double* __restrict__ enl) {
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= nstate) return;
   double e = 0.0;
-  for (int a = 0; a < natm_nl; ++a) {
+  for (int a = lane; a < natm_nl; a += 32) {
     const double vn = vnorm[atm_type[nl_atm[a]]] * rvol;
     const double z = Z[(size_t)s * natm_nl + a];
     e += z * z * vn;
     zt[(size_t)a * nstate + s] = -2.0 * vn * z;
   }
-  enl[s] = e * occ[s];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  if (lane == 0) enl[s] = e * occ[s];
 }
 
 cudaError_t oa_launch_nl_sf(cudaStream_t s, const int* kx, const int* ky, const int* kz, int ng, const int* nl_atm,
@@ -79,7 +84,7 @@ cudaError_t oa_launch_nl_sf(cudaStream_t s, const int* kx, const int* ky, const 
 cudaError_t oa_launch_nl_zscale(cudaStream_t s, const double* Z, int nstate, int natm_nl, const int* nl_atm,
                                 const int* atm_type, const double* vnorm, double rvol, const double* occ, double* zt,
                                 double* enl) {
-  k_nl_zscale<<<(nstate + 127) / 128, 128, 0, s>>>(Z, nstate, natm_nl, nl_atm, atm_type, vnorm, rvol, occ, zt, enl);
+  k_nl_zscale<<<(nstate + 3) / 4, 128, 0, s>>>(Z, nstate, natm_nl, nl_atm, atm_type, vnorm, rvol, occ, zt, enl);
   return cudaGetLastError();
 }
 
@@ -101,24 +106,29 @@ __global__ void k_ees_bspline(const double* __restrict__ pos, const int* __restr
   ees_bspline_axis(pos[nl_atm[a] * 3 + ax], box, ngrid, order, idx + o, mn + o, dmn ? dmn + o : nullptr);
 }
 
-// Z = sum over stencil planes; ENL = occ vnorm/V sum Z^2; zs = 2 vnorm/V occ Z
+// Z = sum over the np partials of the gather (stencil planes, or stencil rows
+// of the pair kernels); ENL = occ vnorm/V sum Z^2; zs = 2 vnorm/V occ Z
 // (eesEnergyAtmForcRchare, cp_ees_nonlocal.C:1480-1560)
-__global__ void k_ees_zreduce(const double* __restrict__ zpart, int nstate, int natm_nl, int order,
-                              const int* __restrict__ nl_atm, const int* __restrict__ atm_type,
-                              const double* __restrict__ vnorm, double rvol, const double* __restrict__ occ,
-                              double* __restrict__ zmat, double* __restrict__ zs, double* __restrict__ enl) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per state, lanes over the atoms.
+__global__ void __launch_bounds__(128)
+k_ees_zreduce(const double* __restrict__ zpart, int nstate, int natm_nl, int np, const int* __restrict__ nl_atm,
+              const int* __restrict__ atm_type, const double* __restrict__ vnorm, double rvol,
+              const double* __restrict__ occ, double* __restrict__ zmat, double* __restrict__ zs,
+              double* __restrict__ enl) {
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= nstate) return;
   double e = 0.0;
-  for (int a = 0; a < natm_nl; ++a) {
+  for (int a = lane; a < natm_nl; a += 32) {
     double z = 0.0;
-    for (int j = 0; j < order; ++j) z += zpart[((size_t)s * natm_nl + a) * order + j];
+    for (int j = 0; j < np; ++j) z += zpart[((size_t)s * natm_nl + a) * np + j];
     const double vn = vnorm[atm_type[nl_atm[a]]] * rvol;
     zmat[(size_t)s * natm_nl + a] = z;
     e += z * z * vn;
     zs[(size_t)s * natm_nl + a] = 2.0 * vn * occ[s] * z;
   }
-  enl[s] = e * occ[s];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  if (lane == 0) enl[s] = e * occ[s];
 }
 
 cudaError_t oa_launch_ees_bspline(oa_ctx* c, cudaStream_t s) {
@@ -129,9 +139,9 @@ cudaError_t oa_launch_ees_bspline(oa_ctx* c, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t oa_launch_ees_zreduce(oa_ctx* c, cudaStream_t s) {
+cudaError_t oa_launch_ees_zreduce(oa_ctx* c, cudaStream_t s, int np) {
   oa_ees* e = c->ees;
-  k_ees_zreduce<<<(c->nstate + 127) / 128, 128, 0, s>>>(e->zpart, c->nstate, c->natm_nl, e->order, c->nl_atm,
+  k_ees_zreduce<<<(c->nstate + 3) / 4, 128, 0, s>>>(e->zpart, c->nstate, c->natm_nl, np, c->nl_atm,
                                                         c->atm_type, c->nl_vnorm, 1.0 / c->vol, c->occ, e->zmat, e->zs,
                                                         e->enl);
   return cudaGetLastError();

@@ -20,6 +20,7 @@
 #include "oa_rdft.cuh"
 #include "oa_state_common.cuh"
 #include "oa_planes.cuh"
+#include "oa_lengths.h"
 
 // Smallest odd stride >= minv, congruent to want (odd) modulo 16 when want >= 0.
 __host__ __device__ constexpr int pencil_stride(int minv, int want) {
@@ -563,18 +564,30 @@ static Plane2Smem plane2_layout(int nkx, int mode) {
   return L;
 }
 
-template <int N> struct SplitOf { static constexpr int n1 = Split<N>::n1, n2 = Split<N>::n2; };
-
-#define OA_PENCIL_LENGTHS(X) X(12) X(20) X(24) X(36) X(40) X(64) X(96) X(108) X(160)
+// Lengths of the z passes: every two-pass length.
+#define OA_ZCASE(NN, A, B) case NN: return OA_CALL(A, B);
+#define OA_ZPASS_DISPATCH(n) switch (n) { OA_LENGTHS_ALL(OA_ZCASE) default: break; }
 
 int oa_pencil_supported(int n) {
+#define OA_CALL(A, B) 1
+  OA_ZPASS_DISPATCH(n)
+#undef OA_CALL
+  return 0;
+}
+
+// Lengths of k_plane2: the nonlocal grids (MODE 2, 3), and the per-state
+// passes of systems without the state-pair kernels (oa_pp.cuh): line orders
+// other than the reference's, or planes too large for them.
+#define OA_PLANE2_LENGTHS(X) X(12) X(20) X(24) X(36) X(40) X(64) X(96) X(108) X(160)
+
+int oa_plane2_supported(int n) {
 #define OA_PS_CASE(NN) if (n == NN) return 1;
-  OA_PENCIL_LENGTHS(OA_PS_CASE)
+  OA_PLANE2_LENGTHS(OA_PS_CASE)
 #undef OA_PS_CASE
   return 0;
 }
 
-#define OA_PENCIL_DISPATCH(n, CALL)                                  \
+#define OA_PLANE2_DISPATCH(n, CALL)                                  \
   switch (n) {                                                       \
     case 12: return CALL(4, 3);                                      \
     case 20: return CALL(4, 5);                                      \
@@ -633,7 +646,7 @@ static cudaError_t zfwd2(cudaStream_t st, int n, const double2* psi, int ng, int
                          const int* nneg, const int* npos, int nlines, void* zbuf, int ldl, const double2* tw,
                          const double2* dyp, int zseg, OaCharge qc, int zext) {
 #define OA_CALL(A, B) zfwd2_n<R, A, B>(st, psi, ng, s0, ns, off, nneg, npos, nlines, zbuf, ldl, tw, dyp, zseg, qc, zext)
-  OA_PENCIL_DISPATCH(n, OA_CALL)
+  OA_ZPASS_DISPATCH(n)
 #undef OA_CALL
   return cudaErrorNotSupported;
 }
@@ -673,7 +686,7 @@ static cudaError_t zbwd2(cudaStream_t st, int n, const void* zbuf, int ldl, int 
 #define OA_CALL(A, B)                                                                                          \
   zbwd2_n<R, A, B>(st, zbuf, ldl, nlines, lkx, off, nneg, npos, tw, psi, fnl, force, g2, occ, ng, s0, ns, scale, \
                    ecut, eke_part, nblk, dyp, po, zseg)
-  OA_PENCIL_DISPATCH(n, OA_CALL)
+  OA_ZPASS_DISPATCH(n)
 #undef OA_CALL
   return cudaErrorNotSupported;
 }
@@ -712,7 +725,7 @@ static cudaError_t plane2(cudaStream_t st, int n, void* zbuf, int nstate, int ld
                           double* rho_part, int ngroup, const EesArgs& E, void* psir) {
 #define OA_CALL(A, B) \
   plane2_n<R, MODE, A, B>(st, zbuf, nstate, ldl, nlines, lkx, lky, nz, nkx, tw, occ, vks, rho_part, ngroup, E, psir)
-  OA_PENCIL_DISPATCH(n, OA_CALL)
+  OA_PLANE2_DISPATCH(n, OA_CALL)
 #undef OA_CALL
   return cudaErrorNotSupported;
 }
@@ -752,7 +765,7 @@ size_t oa_pencil_plane_smem(int precision, int n, int nkx) {
 #define OA_CALL(A, B)                                                                  \
   (precision == OA_FP64 ? plane2_smem_max<double2, double, A, B>(nkx)                  \
                         : plane2_smem_max<float2, float, A, B>(nkx))
-  OA_PENCIL_DISPATCH(n, OA_CALL)
+  OA_PLANE2_DISPATCH(n, OA_CALL)
 #undef OA_CALL
   return 0;
 }

@@ -115,24 +115,6 @@ template <int SIGN> struct RDft<5, SIGN> {
   template <typename C> OA_HD static void run(C* v) { dft5<SIGN>(v); }
 };
 
-// Two-pass factorisations N = N1 * N2 of the pencil lengths with kernels.
-template <int N> struct Split { static constexpr bool ok = false; static constexpr int n1 = 1, n2 = 1; };
-#define OA_SPLIT(NN, A, B)                                                   \
-  template <> struct Split<NN> {                                             \
-    static constexpr bool ok = true;                                         \
-    static constexpr int n1 = A, n2 = B;                                     \
-  };
-OA_SPLIT(12, 4, 3)
-OA_SPLIT(20, 4, 5)
-OA_SPLIT(24, 6, 4)
-OA_SPLIT(36, 6, 6)
-OA_SPLIT(40, 8, 5)
-OA_SPLIT(64, 8, 8)
-OA_SPLIT(96, 12, 8)
-OA_SPLIT(108, 12, 9)
-OA_SPLIT(160, 16, 10)
-#undef OA_SPLIT
-
 // odd leading dimension (complex elements) so that strided accesses by
 // consecutive threads fall into distinct shared-memory banks
 __host__ __device__ constexpr int odd_ld(int n) { return n | 1; }

@@ -19,6 +19,7 @@
 #include "oa_internal.h"
 
 #include "oa_state_common.cuh"
+#include "oa_pp.h"
 
 // ---------------------------------------------------------------------------
 // z pass, forward: packed sphere -> zero-filled z-lines -> FFT(-) -> zbuf[s][z][l]
@@ -346,9 +347,7 @@ cudaError_t oa_pencil_zbwd(int precision, cudaStream_t st, int n, const void* zb
                            const double2* psi, const double2* fnl, double2* force, const double* g2,
                            const double* occ, int ng, int s0, int ns, double scale, double ecut, double* eke_part,
                            int nblk, const double2* dyp, OaPlaneOut po, int zseg);
-cudaError_t oa_pair_plane(int mode, cudaStream_t st, int n, void* zbuf, int nstate, int nz, int ldl, int nlines,
-                          const int* cols, int nkx, const double2* tw, const double* occ, const void* vks,
-                          double* rho_part, int ngroup, void* psir, int kymax, double* qpart);
+int oa_plane2_supported(int n);
 cudaError_t oa_pencil_plane(int precision, int mode, cudaStream_t st, int n, void* zbuf, int nstate, int ldl,
                             int nlines, const int* lkx, const int* lky, int nz, int nkx, const double2* tw,
                             const double* occ, const void* vks, double* rho_part, int ngroup, const EesArgs& E,
@@ -400,7 +399,7 @@ static cudaError_t launch_zbwd(oa_ctx* c, cudaStream_t st, const double2* psi, c
 }
 
 size_t oa_plane_smem_bytes(int precision, int nx, int ny, int nkx) {
-  if (nx == ny && oa_pencil_supported(nx)) {
+  if (nx == ny && oa_plane2_supported(nx)) {
     const size_t p = oa_pencil_plane_smem(precision, nx, nkx);
     if (p > 0 && p <= (size_t)OA_MAX_SMEM) return p;
   }
@@ -432,24 +431,33 @@ cudaError_t oa_launch_state_zfwd(oa_ctx* c, cudaStream_t s, const double2* psi, 
   return c->precision == OA_FP64 ? launch_zfwd<double>(c, s, psi, s0, ns) : launch_zfwd<float>(c, s, psi, s0, ns);
 }
 static cudaError_t pencil_plane(oa_ctx* c, cudaStream_t s, int mode, void* psir) {
-  if (c->fft_runtime || c->nx != c->ny || !oa_pencil_supported(c->nx)) return cudaErrorNotSupported;
+  if (c->fft_runtime || c->nx != c->ny || !oa_plane2_supported(c->nx)) return cudaErrorNotSupported;
   const EesArgs E = {nullptr, nullptr, nullptr, nullptr, 0, 0};
   return oa_pencil_plane(c->precision, mode, s, c->nx, c->zbuf, c->nstate, c->ldl, c->nlines, c->line_kx,
                          c->line_ky, c->nz, c->nkx_s, c->tw_x, c->occ, c->vks, c->rho_part, c->ngroup, E, psir);
 }
 
-// The density pass also stores psi(r) (c->psir) when the two-pass kernels
-// run; the V_KS pass then starts from it (MODE 4) instead of redoing the
-// forward y and x transforms.  c->psir_valid marks that the last density
-// pass stored it.
-// In the mixed form with the state-pair kernels (c->pair_cols set) both
-// passes run two states per x transform and psi(r) is stored per pair
-// (psir_valid 2).
+// State-pair plane kernels (c->pair_cols set): mode 0 density, 4 V_KS, -1
+// the launch shape (resident blocks per SM, row splits).
+static cudaError_t pair_plane(oa_ctx* c, cudaStream_t s, int mode, double* qpart, int* dbps = nullptr,
+                              int* vbps = nullptr, int* split = nullptr) {
+  if (c->fft_runtime || !c->pair_on || !c->psir) return cudaErrorNotSupported;
+  PpArgs A;
+  A.mode = mode; A.n = c->nx; A.st = s; A.zbuf = c->zbuf;
+  A.nstate = c->nstate; A.nz = c->nz; A.ldl = c->ldl; A.nlines = c->nlines;
+  A.cols = c->pair_cols; A.nkx = c->nkx_s; A.kymax = c->pair_kymax;
+  A.tw = c->tw_x; A.occ = c->occ; A.vks = c->vks; A.rho_part = c->rho_part; A.ngroup = mode == 4 ? c->ngroup_vks : c->ngroup_pair;
+  A.psir = c->psir; A.qpart = qpart; A.dbps = dbps; A.vbps = vbps; A.split = split;
+  return oa_pp_plane(c->precision, A);
+}
+
+// The density pass also stores psi(r) (c->psir) when the state-pair or the
+// two-pass kernels run; the V_KS pass then starts from it instead of redoing
+// the forward y and x transforms.  c->psir_valid marks that the last density
+// pass stored it: 2 per pair (state-pair kernels), 1 per state.
 cudaError_t oa_launch_state_plane_density(oa_ctx* c, cudaStream_t s) {
-  if (c->pair_cols && c->psir) {
-    const cudaError_t e = oa_pair_plane(0, s, c->nx, c->zbuf, c->nstate, c->nz, c->ldl, c->nlines, c->pair_cols,
-                                        c->nkx_s, c->tw_x, c->occ, nullptr, c->rho_part, c->ngroup_pair, c->psir,
-                                        c->pair_kymax, c->qvalid ? c->qpart2 : nullptr);
+  {
+    const cudaError_t e = pair_plane(c, s, 0, c->qvalid ? c->qpart2 : nullptr);
     c->psir_valid = e == cudaSuccess ? 2 : 0;
     if (e == cudaSuccess && c->qvalid) c->qvalid = 2;
     c->rho_ngroup = c->ngroup_pair;
@@ -462,12 +470,20 @@ cudaError_t oa_launch_state_plane_density(oa_ctx* c, cudaStream_t s) {
   return c->precision == OA_FP64 ? launch_plane<double, 0>(c, s) : launch_plane<float, 0>(c, s);
 }
 cudaError_t oa_launch_state_plane_vks(oa_ctx* c, cudaStream_t s) {
-  if (c->psir_valid == 2)
-    return oa_pair_plane(4, s, c->nx, c->zbuf, c->nstate, c->nz, c->ldl, c->nlines, c->pair_cols, c->nkx_s,
-                         c->tw_x, c->occ, c->vks, nullptr, c->ngroup_pair, c->psir, c->pair_kymax, nullptr);
+  if (c->psir_valid == 0) {
+    // psi(r) of the z-line buffer by the density kernel (its density sums go
+    // to the partials of the last density pass, which rho has taken up)
+    const cudaError_t e = pair_plane(c, s, 0, nullptr);
+    if (e == cudaSuccess) c->psir_valid = 2;
+    else if (e != cudaErrorNotSupported) return e;
+  }
+  if (c->psir_valid == 2) return pair_plane(c, s, 4, nullptr);
   const cudaError_t e = c->psir_valid ? pencil_plane(c, s, 4, c->psir) : pencil_plane(c, s, 1, nullptr);
   if (e != cudaErrorNotSupported) return e;
   return c->precision == OA_FP64 ? launch_plane<double, 1>(c, s) : launch_plane<float, 1>(c, s);
+}
+cudaError_t oa_pair_plane_shape(oa_ctx* c, int* dbps, int* vbps, int* split) {
+  return pair_plane(c, nullptr, -1, nullptr, dbps, vbps, split);
 }
 cudaError_t oa_launch_state_zbwd(oa_ctx* c, cudaStream_t s, const double2* psi, const double2* fnl,
                                  double2* force, int s0, int ns) {
@@ -510,9 +526,20 @@ static cudaError_t launch_ees(oa_ctx* c, cudaStream_t st, const double2* psi, do
   PlaneSmem L = plane_smem_layout<C, R>(e->na, e->nb, c->nkx_s);
   EesArgs E = {e->idx, e->mn, e->zpart, e->zs, c->natm_nl, e->order, e->dmn, c->ions ? e->fpart : nullptr};
   dim3 pgrid(e->nc, e->ngroup);
-  const bool pp = !c->fft_runtime && e->na == e->nb && oa_pencil_supported(e->na);
+  const bool pp = !c->fft_runtime && e->na == e->nb && oa_plane2_supported(e->na);
+  PeArgs pe;
+  pe.n = e->na; pe.st = st; pe.zbuf = e->zbuf; pe.nstate = c->nstate; pe.nz = e->nc; pe.ldl = c->ldl;
+  pe.nlines = c->nlines; pe.cols = c->pair_cols; pe.nkx = c->nkx_s; pe.kymax = c->pair_kymax; pe.tw = e->tw_a;
+  pe.ngroup = e->ngroup_pair; pe.E = &E; pe.bps = nullptr;
+  const bool pairs = !c->fft_runtime && e->ngroup_pair > 0;
+  int np = e->order;  // Z partials per (state, atom): stencil planes, or stencil rows of the pair kernels
   err = cudaErrorNotSupported;
-  if (pp)
+  if (pairs) {
+    pe.mode = 2;
+    err = oa_pe_plane(c->precision, pe);
+    if (err == cudaSuccess) np = e->order * e->order;
+  }
+  if (err == cudaErrorNotSupported && pp)
     err = oa_pencil_plane(c->precision, 2, st, e->na, e->zbuf, c->nstate, c->ldl, c->nlines, c->line_kx, c->line_ky,
                           e->nc, c->nkx_s, e->tw_a, c->occ, nullptr, nullptr, e->ngroup, E, nullptr);
   if (err == cudaErrorNotSupported) {
@@ -524,12 +551,16 @@ static cudaError_t launch_ees(oa_ctx* c, cudaStream_t st, const double2* psi, do
     err = cudaGetLastError();
   }
   if (err != cudaSuccess) return err;
-  err = oa_launch_ees_zreduce(c, st);
+  err = oa_launch_ees_zreduce(c, st, np);
   if (err != cudaSuccess) return err;
   // with ion dynamics: the nonlocal atom forces from the gathered sums and zs
-  if (c->ions && (err = oa_launch_ees_atom_force(c, st)) != cudaSuccess) return err;
+  if (c->ions && (err = oa_launch_ees_atom_force(c, st, np)) != cudaSuccess) return err;
   err = cudaErrorNotSupported;
-  if (pp)
+  if (pairs) {
+    pe.mode = 3;
+    err = oa_pe_plane(c->precision, pe);
+  }
+  if (err == cudaErrorNotSupported && pp)
     err = oa_pencil_plane(c->precision, 3, st, e->na, e->zbuf, c->nstate, c->ldl, c->nlines, c->line_kx, c->line_ky,
                           e->nc, c->nkx_s, e->tw_a, c->occ, nullptr, nullptr, e->ngroup, E, nullptr);
   if (err == cudaErrorNotSupported) {
@@ -555,6 +586,18 @@ static cudaError_t launch_ees(oa_ctx* c, cudaStream_t st, const double2* psi, do
         e->tw_c, psi, nullptr, fnl, c->g2, c->occ, c->ng, 0, 1.0, c->ecut_psi, c->eke_part, c->nblk_z, e->dyp);
   }
   return cudaGetLastError();
+}
+
+// resident blocks per SM of the nonlocal-grid pair kernels
+cudaError_t oa_ees_pair_shape(oa_ctx* c, int* bps) {
+  const oa_ees* e = c->ees;
+  if (!c->pair_cols || e->na != e->nb) return cudaErrorNotSupported;
+  EesArgs E = {e->idx, e->mn, e->zpart, e->zs, c->natm_nl, e->order, e->dmn, e->fpart};
+  PeArgs pe;
+  pe.mode = -1; pe.n = e->na; pe.st = nullptr; pe.zbuf = e->zbuf; pe.nstate = c->nstate; pe.nz = e->nc;
+  pe.ldl = c->ldl; pe.nlines = c->nlines; pe.cols = c->pair_cols; pe.nkx = c->nkx_s; pe.kymax = c->pair_kymax;
+  pe.tw = e->tw_a; pe.ngroup = 1; pe.E = &E; pe.bps = bps;
+  return oa_pe_plane(c->precision, pe);
 }
 
 cudaError_t oa_launch_ees(oa_ctx* c, cudaStream_t s, const double2* psi, double2* fnl) {

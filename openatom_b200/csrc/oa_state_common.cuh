@@ -52,11 +52,11 @@ __device__ __forceinline__ C herm_x(const C* P, int ldy, int nkx, int nx, int k,
 struct EesArgs {
   const int* idx;       // [natm][3][order] grid index per axis (a, b, c)
   const double* mn;     // [natm][3][order] B-spline weight per axis
-  double* zpart;        // [nstate][natm][order] MODE 2: per-plane Z contributions
+  double* zpart;        // [nstate][natm][order] MODE 2: per-plane Z contributions ([order^2] pair kernels)
   const double* zs;     // [nstate][natm]        MODE 3: scaled Z to scatter
   int natm, order;
   const double* dmn;    // [natm][3][order] derivative weights (with fpart)
-  double* fpart;        // [nstate][natm][order][3] MODE 2, null: no atom forces
+  double* fpart;        // [3] beside each zpart entry, null: no atom forces
 };
 
 

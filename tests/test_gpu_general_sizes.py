@@ -27,6 +27,32 @@ def grid_system(n, nstate, box=7.0, frac=1.0):
                        ecut_ry=(kmax * 2.0 * math.pi / box) ** 2)
 
 
+# FP64: rounding; mixed: FP32 transforms, about 3 log2(n) roundings of 6e-8
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("mixed", 1e-5)])
+@pytest.mark.parametrize("n,nstate", [(16, 4), (25, 5), (27, 3), (45, 3), (50, 2), (72, 5), (80, 3), (100, 3),
+                                      (120, 3), (125, 2), (128, 3), (135, 2), (144, 3), (160, 2)])
+def test_grid_lengths(n, nstate, precision, tol):
+    import torch
+    from openatom_b200.gpu import CPContext
+    s = grid_system(n, nstate)
+    ctx = CPContext(s, precision)
+    psi = torch.from_numpy(s.psi).cuda()
+    rho = torch.zeros(n, n, n, dtype=torch.float64, device="cuda")
+    f = torch.zeros_like(psi)
+    f2 = torch.zeros_like(psi)
+    v = np.random.default_rng(4).standard_normal((n, n, n)) * 0.3
+    ctx.state_fft_fwd(psi, rho)
+    ctx.set_vks(torch.from_numpy(v).cuda())
+    ctx.vks_apply_fft_bwd(psi, f)
+    ctx.vks_apply_fft_bwd(psi, f2, recompute_fwd=True)
+    torch.cuda.synchronize()
+    psir = O.state_g_to_r(s.psi, s)
+    fr, _ = O.eke(s.psi, O.add_forces(O.vks_forces(psir, v, s), None, s), s)
+    assert rel(rho.cpu().numpy(), O.density(psir, s)) < tol
+    assert rel(f.cpu().numpy(), fr) < tol
+    assert rel(f2.cpu().numpy(), fr) < tol
+
+
 @pytest.mark.parametrize("n", [15, 60, 90, 120, 150])
 def test_density_path_lengths(n):
     """The density transforms and the Hartree / XC path off the preset lengths."""
@@ -42,6 +68,23 @@ def test_density_path_lengths(n):
     assert rel(vks.cpu().numpy(), vref) < 1e-10
     for k in ("EHART", "EEXT", "EEXC", "MUXC"):
         assert abs(en[k] - eref[k]) <= 1e-10 * max(1.0, abs(eref[k])), k
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-9), ("mixed", 1e-5)])
+@pytest.mark.parametrize("n,nstate,order,scale", [(40, 5, 4, 1.2), (45, 3, 6, 1.3), (64, 4, 8, 1.0), (96, 3, 4, 1.2)])
+def test_ees_pairs(n, nstate, order, scale, precision, tol):
+    import torch
+    from openatom_b200.gpu import CPContext
+    s = grid_system(n, nstate)
+    ctx = CPContext(s, precision)
+    ctx.ees_init(scale, order)
+    f = torch.zeros(s.psi.shape, dtype=torch.complex128, device="cuda")
+    enl = torch.zeros(nstate, dtype=torch.float64, device="cuda")
+    ctx.nl_ees(torch.from_numpy(s.psi).cuda(), f, enl_out=enl)
+    torch.cuda.synchronize()
+    fr, er, _ = O.nl_ees_energy_forces(s.psi, s, O.ees_setup(s, scale, order))
+    assert rel(enl.cpu().numpy(), er) < tol
+    assert rel(f.cpu().numpy(), fr) < tol
 
 
 @pytest.mark.parametrize("nstate", [129, 150, 199, 256, 300])
