@@ -33,11 +33,12 @@ cudaError_t oa_ees_pair_shape(oa_ctx* c, int* bps);
 int oa_plane2_supported(int n);
 cudaError_t oa_launch_integrate(cudaStream_t s, const double2* F, double2* V, double2* P, const double2* P_in,
                                 const int* sel, const double* cmass, int ng, int nstate, int r0, int r1, int iend,
-                                double dt, int complete_prev, double* kepart, int nblk);
-cudaError_t oa_launch_sync_redundant(cudaStream_t s, double2* P, double2* V, const int* partner, int nred, int ng,
-                                     int nstate);
-cudaError_t oa_launch_sum_partials_multi(cudaStream_t s, int njob, const double* const* part, const int* n,
-                                         const int* stride, const int* off, const double* scale, double* const* out);
+                                double dt, int complete_prev, const int* mirror, int nkx0, double* kepart, int nblk);
+cudaError_t oa_launch_sync_redundant(cudaStream_t s, double2* P, const int* partner, int nred, int ng, int nstate);
+cudaError_t oa_launch_sum_partials_multi(cudaStream_t s, const OaSumJobs& J);
+cudaError_t oa_launch_step_record(cudaStream_t s, const OaSumJobs& J, const int* status, const double* errv,
+                                  const double* dev_e, double norb_tol, int* flag, double* ring, int ring_cap,
+                                  unsigned* ticket);
 cudaError_t oa_launch_sum_partials(cudaStream_t s, const double* part, int n, int stride, int off, double scale,
                                    double* out);
 cudaError_t oa_launch_umma_fwd(cudaStream_t s, int nterm, const double* A, const double* B, int m, int n, long K,
@@ -129,6 +130,7 @@ struct oa_ctx_pc {
   int* ns_status;    // [2] device
   double* ns_err;    // [1] device
   int* partner;      // [nkx0_red]
+  int* mirror;       // [nkx0] redundant point of a unique one, else -1
   double* cmass;     // [ng]
   double* ke_part;   // integrate partials
   int ke_nblk;
@@ -379,6 +381,12 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     }
     TRY(upload(&c->pos, d->pos, (size_t)3 * d->natm));
     TRY(upload(&p->partner, d->red_partner, d->nkx0_red));
+    {
+      std::vector<int> mirror(d->nkx0, -1);
+      for (int i = 0; i < d->nkx0_red; ++i)
+        if (d->red_partner[i] >= 0 && d->red_partner[i] < d->nkx0) mirror[d->red_partner[i]] = i;
+      TRY(upload(&p->mirror, mirror.data(), mirror.size()));
+    }
     TRY(upload(&c->ky, d->ky, d->ng));
     TRY(upload(&c->kz, d->kz, d->ng));
     c->natm_nl = d->natm_nl;
@@ -390,7 +398,6 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     TRY(cudaMalloc(&c->zmat, ((size_t)d->natm_nl * d->nstate + 1) * sizeof(double)));
     TRY(cudaMalloc(&c->zt, ((size_t)d->natm_nl * d->nstate + 1) * sizeof(double)));
     TRY(cudaMalloc(&c->enl, (size_t)d->nstate * sizeof(double)));
-    TRY(cudaMalloc(&c->enl_eke, (size_t)d->nstate * sizeof(double)));
     TRY(upload(&p->cmass, d->cmass, d->ng));
     c->tw_x = make_twiddles(d->nx);
     c->tw_y = make_twiddles(d->ny);
@@ -460,7 +467,8 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     p->ns_grid = oa_ns_grid(d->nstate, c->device);
     p->ns_cluster = oa_ns_cluster_size(d->nstate);
     TRY(cudaMalloc(&p->ns_work, ((size_t)5 * d->nstate * d->nstate + p->ns_grid + 32) * sizeof(double)));
-    TRY(cudaMalloc(&p->ns_status, 4 * sizeof(int)));
+    TRY(cudaMalloc(&p->ns_status, 4 * sizeof(int)));  // [2] status, [3] ticket of the step record
+    TRY(cudaMemset(p->ns_status, 0, 4 * sizeof(int)));
     TRY(cudaMalloc(&p->ns_err, 2 * sizeof(double)));
     p->ke_nblk = oa_integrate_nblk(d->ng, d->nstate);
     TRY(cudaMalloc(&p->ke_part, p->ke_nblk * sizeof(double)));
@@ -527,10 +535,10 @@ extern "C" oa_status oa_gpu_destroy(oa_ctx* c) {
   void* dev[] = {c->line_kx, c->line_ky, c->line_off, c->line_nneg, c->line_npos, c->kx, c->g2, c->tw_x, c->tw_y,
                  c->tw_z, c->spl, c->q_type, c->atm_type, c->atm_perm, c->pos, c->psir, c->pair_cols, c->phase, c->occ, c->zbuf, c->rho_part, c->rho,
                  c->vks, c->vxc, c->dz, c->red, c->eke_part, p->part, p->ns_work, p->ns_status, p->ns_err,
-                 p->partner, p->cmass, p->ke_part, p->dev_e, p->mat_a, p->mat_x, p->eye, p->vtmp, p->upart,
+                 p->partner, p->mirror, p->cmass, p->ke_part, p->dev_e, p->mat_a, p->mat_x, p->eye, p->vtmp, p->upart,
                  p->pl_big[0], p->pl_big[1], p->pl_big[2], p->pl_ma, p->pl_mb,
                  p->err_flag, c->ky, c->kz, c->nl_atm, c->nl_spl, c->nl_vnorm, c->nl_gz0, c->sf, c->zmat, c->zt,
-                 c->enl, c->enl_eke, c->grad, c->dzg, c->qpart, c->qpart2, c->qscale};
+                 c->enl, c->grad, c->dzg, c->qpart, c->qpart2, c->qscale};
   for (void* q : dev) if (q) cudaFree(q);
   if (p->h_status) cudaFreeHost(p->h_status);
   if (p->h_vals) cudaFreeHost(p->h_vals);
@@ -563,26 +571,47 @@ __global__ void k_to_float(const double* a, float* b, size_t n) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) b[i] = (float)a[i];
 }
 
+// EEXC = (0.75 ex + ec) V/N ; MUXC = sum vxc rho V/N; EGGA = (ex + ec of the
+// gradient correction) V/N, the two halves of each block's partials (an
+// empty sum, zero, without it)
+static void vks_sums(oa_ctx* c, OaSumJobs* J) {
+  oa_ctx_pc* p = pcx(c);
+  const int nx = oa_rho_xc_nblk(), nzb = oa_rho_z_nblk(c);
+  const double vs = c->vol / (double)c->npts;
+  const double *xc = c->red, *zp = c->red + 3 * nx, *gp = c->red + oa_rho_gga_red_off(c);
+  J->add(xc, nx, 3, 0, 0.75 * vs, p->dev_e + 8);
+  J->add(xc, nx, 3, 1, vs, p->dev_e + 9);
+  J->add(xc, nx, 3, 2, vs, p->dev_e + OA_E_MUXC);
+  J->add(zp, nzb, 3, 0, 0.5, p->dev_e + OA_E_EHART);
+  J->add(zp, nzb, 3, 1, 1.0, p->dev_e + OA_E_EEXT);
+  J->add(zp, nzb, 3, 2, 0.5, p->dev_e + OA_E_EWALD);
+  J->add(gp, c->gga ? nx : 0, 2, 0, vs, p->dev_e + 11);
+  J->add(gp, c->gga ? nx : 0, 2, 1, vs, p->dev_e + 12);
+}
+
+// every energy sum of a native step, the PsiV check and the step record
+cudaError_t oa_step_record(oa_ctx* c, cudaStream_t s, double norb_tol, int* flag, double* ring, int ring_cap) {
+  oa_ctx_pc* p = pcx(c);
+  OaSumJobs J;
+  J.njob = 0;
+  vks_sums(c, &J);
+  J.add(c->eke_part, c->nstate * c->nblk_z, 1, 0, 0.5, p->dev_e + OA_E_EKE);
+  J.add(c->ees ? c->ees->enl : c->enl, c->ees || c->natm_nl > 0 ? c->nstate : 0, 1, 0, 1.0, p->dev_e + OA_E_ENL);
+  J.add(p->ke_part, p->ke_nblk, 1, 0, 1.0, p->dev_e + OA_E_FICT);
+  return oa_launch_step_record(s, J, p->ns_status, p->ns_err, p->dev_e, norb_tol, flag, ring, ring_cap,
+                               (unsigned*)(p->ns_status + 3));
+}
+
 extern "C" oa_status oa_gpu_vks_build(oa_ctx* c, void* stream, double* vks_out) {
   OA_ARG_CHECK(c, "null argument");
   cudaStream_t s = (cudaStream_t)stream;
   oa_ctx_pc* p = pcx(c);
   OA_CUDA_TRY(oa_launch_rho_fft_hart(c, s));
-  const int nx = oa_rho_xc_nblk(), nzb = oa_rho_z_nblk(c);
-  const double vs = c->vol / (double)c->npts;
-  // EEXC = (0.75 ex + ec) V/N ; MUXC = sum vxc rho V/N; EGGA = (ex + ec of the
-  // gradient correction) V/N, the two halves of each block's partials
-  {
-    const double* gp = c->red + oa_rho_gga_red_off(c);
-    const double* part[8] = {c->red, c->red, c->red, c->red + 3 * nx, c->red + 3 * nx, c->red + 3 * nx, gp, gp + 1};
-    const int n[8] = {nx, nx, nx, nzb, nzb, nzb, nx, nx};
-    const int stride[8] = {3, 3, 3, 3, 3, 3, 2, 2};
-    const int off[8] = {0, 1, 2, 0, 1, 2, 0, 0};
-    const double scale[8] = {0.75 * vs, vs, vs, 0.5, 1.0, 0.5, vs, vs};
-    double* out[8] = {p->dev_e + 8, p->dev_e + 9, p->dev_e + OA_E_MUXC, p->dev_e + OA_E_EHART,
-                      p->dev_e + OA_E_EEXT, p->dev_e + OA_E_EWALD, p->dev_e + 11, p->dev_e + 12};
-    OA_CUDA_TRY(oa_launch_sum_partials_multi(s, c->gga ? 8 : 6, part, n, stride, off, scale, out));
-    if (!c->gga) OA_CUDA_TRY(cudaMemsetAsync(p->dev_e + 11, 0, 2 * sizeof(double), s));
+  if (!p->pl_cache) {  // (a native step sums at its end)
+    OaSumJobs J;
+    J.njob = 0;
+    vks_sums(c, &J);
+    OA_CUDA_TRY(oa_launch_sum_partials_multi(s, J));
   }
   if (vks_out) {
     if (c->precision == OA_FP64)
@@ -624,21 +653,30 @@ __global__ void k_eke_states(const double* part, int nblk, double* eke_state) {
   }
 }
 
-extern "C" oa_status oa_gpu_vks_apply_fft_bwd(oa_ctx* c, void* stream, const double* psi, int recompute_fwd,
-                                              const double* fnl, double* force, double* eke_out) {
-  OA_ARG_CHECK(c && psi && force, "null argument");
-  cudaStream_t s = (cudaStream_t)stream;
+// fnl_ready (optional): the z pass, which adds fnl, waits for this event
+oa_status oa_vks_apply(oa_ctx* c, cudaStream_t s, const double* psi, int recompute_fwd, const double* fnl,
+                       cudaEvent_t fnl_ready, double* force, double* eke_out) {
   if (recompute_fwd) {
     OA_CUDA_TRY(oa_launch_state_zfwd(c, s, (const double2*)psi, 0, c->nstate));
     c->psir_valid = 0;  // the z-line buffer is newer than psi(r)
   }
   OA_CUDA_TRY(oa_launch_state_plane_vks(c, s));
+  if (fnl_ready) OA_CUDA_TRY(cudaStreamWaitEvent(s, fnl_ready, 0));
   OA_CUDA_TRY(oa_launch_state_zbwd(c, s, (const double2*)psi, (const double2*)fnl, (double2*)force, 0, c->nstate));
-  double* es = eke_out ? eke_out : c->enl_eke;
-  k_eke_states<<<c->nstate, 128, 0, s>>>(c->eke_part, c->nblk_z, es);
-  OA_CUDA_TRY(cudaGetLastError());
-  OA_CUDA_TRY(oa_launch_sum_partials(s, es, c->nstate, 1, 0, 1.0, pcx(c)->dev_e + OA_E_EKE));
+  // (a native step sums at its end)
+  if (eke_out) {
+    k_eke_states<<<c->nstate, 128, 0, s>>>(c->eke_part, c->nblk_z, eke_out);
+    OA_CUDA_TRY(cudaGetLastError());
+  }
+  if (!pcx(c)->pl_cache)
+    OA_CUDA_TRY(oa_launch_sum_partials(s, c->eke_part, c->nstate * c->nblk_z, 1, 0, 0.5, pcx(c)->dev_e + OA_E_EKE));
   return OA_OK;
+}
+
+extern "C" oa_status oa_gpu_vks_apply_fft_bwd(oa_ctx* c, void* stream, const double* psi, int recompute_fwd,
+                                              const double* fnl, double* force, double* eke_out) {
+  OA_ARG_CHECK(c && psi && force, "null argument");
+  return oa_vks_apply(c, (cudaStream_t)stream, psi, recompute_fwd, fnl, nullptr, force, eke_out);
 }
 
 extern "C" oa_status oa_gpu_pc_forward(oa_ctx* c, void* stream, const double* left, const double* right,
@@ -722,7 +760,7 @@ extern "C" oa_status oa_gpu_min_step(oa_ctx* c, void* stream, const double* forc
   OA_CUDA_TRY(oa_launch_min_step(s, (const double2*)force, (double2*)conj_grad, (double2*)psi, p->cmass, c->g2,
                                  c->ecut_psi, c->ng, c->nstate, gamma, dt));
   // Gamma redundancy sync of psi (computeRedPsi, gspace.ci:692-708)
-  OA_CUDA_TRY(oa_launch_sync_redundant(s, (double2*)psi, nullptr, p->partner, c->nkx0_red, c->ng, c->nstate));
+  OA_CUDA_TRY(oa_launch_sync_redundant(s, (double2*)psi, p->partner, c->nkx0_red, c->ng, c->nstate));
   return OA_OK;
 }
 
@@ -769,12 +807,12 @@ oa_status oa_integrate_sel(oa_ctx* c, cudaStream_t s, const double* force, doubl
   oa_ctx_pc* p = pcx(c);
   const int r0 = c->nkx0_red, r1 = c->nkx0_red + c->nkx0_zero, iend = c->nkx0_red + c->nkx0_uni;
   OA_CUDA_TRY(oa_launch_integrate(s, (const double2*)force, (double2*)vpsi, (double2*)psi, (const double2*)psi_in,
-                                  sel, p->cmass, c->ng, c->nstate, r0, r1, iend, dt, complete_prev, p->ke_part,
-                                  p->ke_nblk));
-  OA_CUDA_TRY(oa_launch_sum_partials(s, p->ke_part, p->ke_nblk, 1, 0, 1.0, p->dev_e + OA_E_FICT));
+                                  sel, p->cmass, c->ng, c->nstate, r0, r1, iend, dt, complete_prev, p->mirror,
+                                  c->nkx0, p->ke_part, p->ke_nblk));
+  if (!p->pl_cache)  // (a native step sums at its end)
+    OA_CUDA_TRY(oa_launch_sum_partials(s, p->ke_part, p->ke_nblk, 1, 0, 1.0, p->dev_e + OA_E_FICT));
   if (fict_ke_out)
     OA_CUDA_TRY(cudaMemcpyAsync(fict_ke_out, p->dev_e + OA_E_FICT, sizeof(double), cudaMemcpyDeviceToDevice, s));
-  OA_CUDA_TRY(oa_launch_sync_redundant(s, (double2*)psi, (double2*)vpsi, p->partner, c->nkx0_red, c->ng, c->nstate));
   return OA_OK;
 }
 
@@ -1333,7 +1371,7 @@ extern "C" oa_status oa_gpu_nl_sf(oa_ctx* c, void* stream, const double* psi, in
   const int n = c->nstate, na = c->natm_nl;
   if (na == 0) {
     OA_CUDA_TRY(cudaMemsetAsync(fnl_out, 0, (size_t)n * c->ng * sizeof(double2), s));
-    OA_CUDA_TRY(cudaMemsetAsync(p->dev_e + OA_E_ENL, 0, sizeof(double), s));
+    if (!p->pl_cache) OA_CUDA_TRY(cudaMemsetAsync(p->dev_e + OA_E_ENL, 0, sizeof(double), s));
     if (enl_out) OA_CUDA_TRY(cudaMemsetAsync(enl_out, 0, (size_t)n * sizeof(double), s));
     return OA_OK;
   }
@@ -1360,7 +1398,7 @@ extern "C" oa_status oa_gpu_nl_sf(oa_ctx* c, void* stream, const double* psi, in
   else
     OA_CUDA_TRY(mixed_bwd(c, s, nterm, c->zt, (const double*)c->sf, 1.0, 1.0, nullptr, nullptr, 0.0, n, na, K, 0,
                           fnl_out, PL_SF, PL_OTHER));
-  OA_CUDA_TRY(oa_launch_sum_partials(s, c->enl, n, 1, 0, 1.0, p->dev_e + OA_E_ENL));
+  if (!p->pl_cache) OA_CUDA_TRY(oa_launch_sum_partials(s, c->enl, n, 1, 0, 1.0, p->dev_e + OA_E_ENL));
   if (enl_out) OA_CUDA_TRY(cudaMemcpyAsync(enl_out, c->enl, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   // ion dynamics: the nonlocal atom forces from the same Z
   if (c->ions) OA_CUDA_TRY(oa_launch_nl_sf_force(c, s, psi));
@@ -1520,7 +1558,8 @@ extern "C" oa_status oa_gpu_nl_ees(oa_ctx* c, void* stream, const double* psi, d
   oa_ees* e = c->ees;
   OA_CUDA_TRY(oa_launch_ees_bspline(c, s));
   OA_CUDA_TRY(oa_launch_ees(c, s, (const double2*)psi, (double2*)fnl_out));
-  OA_CUDA_TRY(oa_launch_sum_partials(s, e->enl, c->nstate, 1, 0, 1.0, pcx(c)->dev_e + OA_E_ENL));
+  if (!pcx(c)->pl_cache)
+    OA_CUDA_TRY(oa_launch_sum_partials(s, e->enl, c->nstate, 1, 0, 1.0, pcx(c)->dev_e + OA_E_ENL));
   if (enl_out) OA_CUDA_TRY(cudaMemcpyAsync(enl_out, e->enl, (size_t)c->nstate * sizeof(double), cudaMemcpyDeviceToDevice, s));
   return OA_OK;
 }

@@ -145,7 +145,6 @@ struct oa_ctx {
   double *nl_spl, *nl_vnorm, *nl_gz0;
   double2 *sf;            // [natm_nl][ng] structure factor x projector
   double *zmat, *zt, *enl;
-  double *enl_eke;        // [nstate] per-state EKE scratch
   // scratch (FFT path precision R; byte sizes)
   void *zbuf;             // [nstate][nz][ldl] C
   size_t zbuf_bytes;
@@ -179,6 +178,7 @@ struct oa_ctx {
   oa_eesl *eesl;          // EES local path, after oa_gpu_set_ees_local
   int eesl_gen;           // bumped by every oa_gpu_set_ees_local (captured graphs depend on it)
   int fft_runtime;        // oa_tuning fft_path 2: runtime-plan transforms for the state path
+  int phase_done;         // inside a native step: the phase tables are this step's
   int rho_groups_cap;     // groups the density partials are allocated for
   int nq2_cap;            // entries of qpart2 allocated
   double gzvps_t[4];      // g = 0 limit of the local part per type
@@ -188,6 +188,24 @@ struct oa_ctx {
   int nq, nq2;
   int qvalid;             // the last density pass wrote both partial sets
 };
+
+// Block sums out[b] = scale[b] sum_{i < n[b]} part[b][i stride[b] + off[b]]
+#define OA_MAX_SUMS 12
+struct OaSumJobs {
+  int njob;
+  const double* part[OA_MAX_SUMS];
+  double* out[OA_MAX_SUMS];
+  double scale[OA_MAX_SUMS];
+  int n[OA_MAX_SUMS], stride[OA_MAX_SUMS], off[OA_MAX_SUMS];
+  void add(const double* p, int count, int st, int o, double sc, double* dst) {
+    part[njob] = p; n[njob] = count; stride[njob] = st; off[njob] = o; scale[njob] = sc; out[njob] = dst;
+    ++njob;
+  }
+};
+
+// Step record of the native step: the 16 energy accumulators, NS iterations,
+// converged, residual, max|S - 2I|
+#define OA_REC 20
 
 enum { OA_E_EKE = 0, OA_E_EHART, OA_E_EEXT, OA_E_EWALD, OA_E_EEXC, OA_E_MUXC, OA_E_ENL, OA_E_FICT };
 #define OA_E_EGGA 10      // device energy slot of EGGA (slots 8, 9 hold the EEXC halves)

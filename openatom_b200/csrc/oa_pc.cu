@@ -8,7 +8,8 @@
 //   PairCalculator::multiplyResult/bwMultiplyHelper/bwMultiplyDynOrthoT
 //     (ckPairCalculator.C:1201-1468, 1710-2031)                       -> k_pc_bwd_f64
 //   CPINTEGRATE::CP_integrate_dyn/cp_evolve_vel/get_fictKE (cp_dynamics.C:29-270)
-//     + Gamma redundancy sync (CP_State_GSpacePlane.C:2829-2970)     -> k_integrate + k_sync_redundant
+//     + Gamma redundancy sync (CP_State_GSpacePlane.C:2829-2970)     -> k_integrate (k_sync_redundant after a
+//     minimisation step)
 //
 // Operand layout: every state row is its coefficients as 2*ng contiguous
 // doubles (the DGEMM real view).  kx = 0 rows of the reference's 1/sqrt(2),
@@ -204,16 +205,6 @@ k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int n, 
   if (i < n && j < n) C[(size_t)i * n + j] = alpha * acc;
 }
 
-// Several single-block sums in one launch: block b writes
-// out[b] = scale[b] * sum_i part[b][i * stride[b] + off[b]], in the order of
-// k_sum_partials.
-struct SumJobs {
-  const double* part[8];
-  double* out[8];
-  double scale[8];
-  int n[8], stride[8], off[8];
-};
-
 // ---------------------------------------------------------------------------
 // Newton-Schulz S^-1/2 (ortho.C), one cooperative kernel, bounded iterations.
 //   B = S/2 (or S for lsda); A = I; repeat:
@@ -363,7 +354,8 @@ k_ortho_ns(const double* __restrict__ S, int n, double bscale, double tol, int m
 __global__ void __launch_bounds__(256)
 k_integrate(const double2* __restrict__ F, double2* __restrict__ V, double2* P, const double2* P_in,
             const int* __restrict__ sel, const double* __restrict__ cmass, int ng, int nstate, int r0, int r1,
-            int iend, double dt, int complete_prev, double* __restrict__ kepart) {
+            int iend, double dt, int complete_prev, const int* __restrict__ mirror, int nkx0,
+            double* __restrict__ kepart) {
   __shared__ double sh[8];
   const double dt2 = 0.5 * dt;
   const size_t base = (size_t)blockIdx.y * ng;
@@ -397,6 +389,14 @@ k_integrate(const double2* __restrict__ F, double2* __restrict__ V, double2* P, 
     V[base + i] = vv;
     pp.x += vv.x * dt; pp.y += vv.y * dt;
     P[base + i] = pp;
+    if (i < nkx0) {
+      // Gamma redundancy: the mirror of a unique kx = 0 point is its conjugate
+      const int k = mirror[i];
+      if (k >= 0) {
+        V[base + k] = make_double2(vv.x, -vv.y);
+        P[base + k] = make_double2(pp.x, -pp.y);
+      }
+    }
   }
   double w = ke;
 #pragma unroll
@@ -474,15 +474,14 @@ cudaError_t oa_launch_min_step(cudaStream_t s, const double2* F, double2* conj, 
   return cudaGetLastError();
 }
 
-__global__ void k_sync_redundant(double2* __restrict__ P, double2* __restrict__ V, const int* __restrict__ partner,
-                                 int nred, int ng, int nstate) {
+__global__ void k_sync_redundant(double2* __restrict__ P, const int* __restrict__ partner, int nred, int ng,
+                                 int nstate) {
   const size_t total = (size_t)nstate * nred;
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int s = (int)(t / nred), i = (int)(t - (size_t)s * nred);
     const size_t src = (size_t)s * ng + partner[i];
     const size_t dst = (size_t)s * ng + i;
     double2 p = P[src]; p.y = -p.y; P[dst] = p;
-    if (V) { double2 v = V[src]; v.y = -v.y; V[dst] = v; }
   }
 }
 
@@ -520,11 +519,46 @@ __global__ void k_sum_partials(const double* __restrict__ part, int n, int strid
   if (threadIdx.x == 0) out[0] = scale * t;
 }
 
-__global__ void k_sum_partials_multi(SumJobs J) {
+// Several single-block sums in one launch: block b writes
+// out[b] = scale[b] sum_i part[b][i stride[b] + off[b]], summed as in
+// k_sum_partials.
+__global__ void k_sum_partials_multi(OaSumJobs J) {
   __shared__ double sh[32];
   const int b = blockIdx.x;
   const double t = sum_strided_block(J.part[b], J.n[b], J.stride[b], J.off[b], sh);
   if (threadIdx.x == 0) J.out[b][0] = J.scale[b] * t;
+}
+
+// End of a native step: all of its energy sums (one block each), and by the
+// last block to finish the PsiV flag (max|S - 2I| > norb_tol on a good step),
+// the first failing step and the step record.  One launch in place of the
+// six that each sum and the check were: at 32 states on 64^3 a step of 38
+// launches is a quarter launch latency.
+__global__ void __launch_bounds__(512)
+k_step_record(OaSumJobs J, const int* __restrict__ status, const double* __restrict__ errv, const double* dev_e,
+              double norb_tol, int* flag, double* __restrict__ ring, int ring_cap, unsigned* ticket) {
+  __shared__ double sh[32];
+  const int b = blockIdx.x;
+  const double t = sum_strided_block(J.part[b], J.n[b], J.stride[b], J.off[b], sh);
+  if (threadIdx.x != 0) return;
+  J.out[b][0] = J.scale[b] * t;
+  __threadfence();
+  if (atomicAdd(ticket, 1u) + 1u != gridDim.x) return;
+  *ticket = 0u;  // for the next step
+  __threadfence();
+  const int k = flag[1];
+  const double err = errv[0], smax = errv[1];
+  const int code = (!(err == err) || !(smax == smax)) ? 2 : (status[1] ? 0 : 1);
+  // set or clear: the flag of the previous step's PsiV reset ends here
+  flag[0] = (code == 0 && smax > norb_tol) ? 1 : 0;
+  if (code != 0 && flag[2] == 0) { flag[2] = code; flag[3] = k; }
+  double* r = ring + (size_t)(k % ring_cap) * OA_REC;
+  for (int i = 0; i < 16; ++i) r[i] = __ldcg(dev_e + i);
+  r[16] = (double)status[0];
+  r[17] = (double)status[1];
+  r[18] = err;
+  r[19] = smax;
+  flag[1] = k + 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -581,17 +615,15 @@ cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* 
   return cudaGetLastError();
 }
 
-// six reductions of the density / Hartree partials in one launch (see
-// oa_gpu_vks_build): entries b < njob of the arrays
-cudaError_t oa_launch_sum_partials_multi(cudaStream_t s, int njob, const double* const* part, const int* n,
-                                         const int* stride, const int* off, const double* scale, double* const* out) {
-  if (njob < 1 || njob > 8) return cudaErrorInvalidValue;
-  SumJobs J;
-  for (int b = 0; b < njob; ++b) {
-    J.part[b] = part[b]; J.out[b] = out[b]; J.scale[b] = scale[b];
-    J.n[b] = n[b]; J.stride[b] = stride[b]; J.off[b] = off[b];
-  }
-  k_sum_partials_multi<<<njob, 512, 0, s>>>(J);
+cudaError_t oa_launch_sum_partials_multi(cudaStream_t s, const OaSumJobs& J) {
+  k_sum_partials_multi<<<J.njob, 512, 0, s>>>(J);
+  return cudaGetLastError();
+}
+
+cudaError_t oa_launch_step_record(cudaStream_t s, const OaSumJobs& J, const int* status, const double* errv,
+                                  const double* dev_e, double norb_tol, int* flag, double* ring, int ring_cap,
+                                  unsigned* ticket) {
+  k_step_record<<<J.njob, 512, 0, s>>>(J, status, errv, dev_e, norb_tol, flag, ring, ring_cap, ticket);
   return cudaGetLastError();
 }
 
@@ -631,19 +663,19 @@ cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bs
 
 cudaError_t oa_launch_integrate(cudaStream_t s, const double2* F, double2* V, double2* P, const double2* P_in,
                                 const int* sel, const double* cmass, int ng, int nstate, int r0, int r1, int iend,
-                                double dt, int complete_prev, double* kepart, int nblk) {
+                                double dt, int complete_prev, const int* mirror, int nkx0, double* kepart, int nblk) {
   if (nblk != oa_integrate_nblk(ng, nstate) || (P_in && !sel)) return cudaErrorInvalidValue;
   const dim3 grid((ng + OA_INT_CHUNK - 1) / OA_INT_CHUNK, nstate);
-  k_integrate<<<grid, 256, 0, s>>>(F, V, P, P_in, sel, cmass, ng, nstate, r0, r1, iend, dt, complete_prev, kepart);
+  k_integrate<<<grid, 256, 0, s>>>(F, V, P, P_in, sel, cmass, ng, nstate, r0, r1, iend, dt, complete_prev, mirror,
+                                    nkx0, kepart);
   return cudaGetLastError();
 }
 
-cudaError_t oa_launch_sync_redundant(cudaStream_t s, double2* P, double2* V, const int* partner, int nred, int ng,
-                                     int nstate) {
+cudaError_t oa_launch_sync_redundant(cudaStream_t s, double2* P, const int* partner, int nred, int ng, int nstate) {
   if (nred == 0) return cudaSuccess;
   const size_t total = (size_t)nstate * nred;
   const int nb = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-  k_sync_redundant<<<nb, 256, 0, s>>>(P, V, partner, nred, ng, nstate);
+  k_sync_redundant<<<nb, 256, 0, s>>>(P, partner, nred, ng, nstate);
   return cudaGetLastError();
 }
 

@@ -964,8 +964,8 @@ static cudaError_t gga_front(oa_ctx* c, cudaStream_t s) {
 cudaError_t oa_launch_rho_fft_hart(oa_ctx* c, cudaStream_t s) {
   const double tpi_l = 2.0 * 3.14159265358979323846 / c->box;
   cudaError_t e;
-  // phase tables exp(i 2 pi k x / L)
-  if ((e = oa_launch_phase_tables(c, s)) != cudaSuccess) return e;
+  // phase tables exp(i 2 pi k x / L) (a native step makes them first of all)
+  if (!c->phase_done && (e = oa_launch_phase_tables(c, s)) != cudaSuccess) return e;
   if ((e = rho_xy_fwd(c, s, c->rho, c->vol / c->npts, (double2*)c->dz, 1, 0, 0)) != cudaSuccess) return e;
   if (c->gga && (e = gga_front(c, s)) != cudaSuccess) return e;
   RhoTypeOff toff;

@@ -17,12 +17,9 @@
 
 // entry points of oa_abi.cu used here
 extern "C" {
-oa_status oa_gpu_state_fft_fwd(oa_ctx* ctx, void* stream, const double* psi, double* rho_out);
 oa_status oa_gpu_vks_build(oa_ctx* ctx, void* stream, double* vks_out);
 oa_status oa_gpu_nl_sf(oa_ctx* ctx, void* stream, const double* psi, int nterm, double* fnl_out, double* enl_out);
 oa_status oa_gpu_nl_ees(oa_ctx* ctx, void* stream, const double* psi, double* fnl_out, double* enl_out);
-oa_status oa_gpu_vks_apply_fft_bwd(oa_ctx* ctx, void* stream, const double* psi, int recompute_fwd,
-                                   const double* fnl, double* force, double* eke_out);
 oa_status oa_gpu_pc_forward(oa_ctx* ctx, void* stream, const double* left, const double* right, double alpha,
                             double w_kx0, double* C);
 oa_status oa_gpu_pc_forward_mixed(oa_ctx* ctx, void* stream, const double* left, const double* right, double alpha,
@@ -38,6 +35,8 @@ oa_status oa_gpu_integrate(oa_ctx* ctx, void* stream, const double* force, doubl
 }
 
 int oa_ns_capturable(oa_ctx* c);
+oa_status oa_vks_apply(oa_ctx* c, cudaStream_t s, const double* psi, int recompute_fwd, const double* fnl,
+                       cudaEvent_t fnl_ready, double* force, double* eke_out);
 oa_status oa_integrate_sel(oa_ctx* c, cudaStream_t s, const double* force, double* vpsi, double* psi,
                            const double* psi_in, const int* sel, double dt, int complete_prev, double* fict_ke_out);
 oa_status oa_psi_t_settle(oa_ctx* c, cudaStream_t s, const double* psi, double* psi_t, const int* flag);
@@ -46,12 +45,10 @@ oa_status oa_psi_t_and_psiv(oa_ctx* c, cudaStream_t s, const double* T, double* 
 
 cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
                                double* work, double* T, int* status, double* errv, int grid);
+cudaError_t oa_step_record(oa_ctx* c, cudaStream_t s, double norb_tol, int* flag, double* ring, int ring_cap);
 cudaError_t oa_step_ortho_args(oa_ctx* c, double** work, int** status, double** errv, int* grid, double** dev_e,
                                int** h_status, double** h_vals, double** eye);
 
-// per-step record: the 16 energy accumulators, NS iterations, converged,
-// residual, max|S - 2I|
-#define OA_REC 20
 #define OA_NREC_OUT 14  // values per step handed back (oa_gpu_cp_step)
 
 // one step record -> EKE EHART EEXT EWALD EEXC MUXC FICT ENL, Newton-Schulz
@@ -68,6 +65,8 @@ struct oa_step_scratch {
   int* flag;              // device: [0] PsiV pending, [1] steps recorded, [2] first error code, [3] its step
   double* ring;           // device: [ring_cap][OA_REC]
   int ring_cap;
+  cudaStream_t side;      // the nonlocal branch of a step
+  cudaEvent_t fork, join;
   double* ring_host;      // pinned copy of the ring
   int flag_host[4];
   cudaGraphExec_t exec;   // PsiV reset .. S
@@ -100,8 +99,11 @@ static oa_status ensure_scratch(oa_ctx* c) {
   if (cudaMalloc(&s->F, cb) != cudaSuccess || cudaMalloc(&s->F2, cb) != cudaSuccess ||
       cudaMalloc(&s->Fnl, cb) != cudaSuccess || cudaMalloc(&s->S, mb) != cudaSuccess ||
       cudaMalloc(&s->lam, mb) != cudaSuccess || cudaMalloc(&s->gam, mb) != cudaSuccess ||
-      cudaMalloc(&s->flag, 4 * sizeof(int)) != cudaSuccess || cudaMemset(s->flag, 0, 4 * sizeof(int)) != cudaSuccess) {
-    oa_set_error("cudaMalloc failed for the step scratch", __FILE__, __LINE__);
+      cudaMalloc(&s->flag, 4 * sizeof(int)) != cudaSuccess || cudaMemset(s->flag, 0, 4 * sizeof(int)) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming) != cudaSuccess) {
+    oa_set_error("allocation of the step scratch failed", __FILE__, __LINE__);
     oa_step_free(c);
     return OA_ERR_CUDA;
   }
@@ -128,26 +130,6 @@ static oa_status ensure_ring(oa_ctx* c, int n) {
   return OA_OK;
 }
 
-// After Newton-Schulz: the PsiV flag (max|S - 2I| > norb_tol on a good step),
-// the first failing step, and the step record.  One thread.
-__global__ void k_step_check(const int* __restrict__ status, const double* __restrict__ errv,
-                             const double* __restrict__ dev_e, double norb_tol, int* __restrict__ flag,
-                             double* __restrict__ ring, int ring_cap) {
-  const int k = flag[1];
-  const double err = errv[0], smax = errv[1];
-  const int code = (!(err == err) || !(smax == smax)) ? 2 : (status[1] ? 0 : 1);
-  // set or clear: the flag of the previous step's PsiV reset ends here
-  flag[0] = (code == 0 && smax > norb_tol) ? 1 : 0;
-  if (code != 0 && flag[2] == 0) { flag[2] = code; flag[3] = k; }
-  double* r = ring + (size_t)(k % ring_cap) * OA_REC;
-  for (int i = 0; i < 16; ++i) r[i] = dev_e[i];
-  r[16] = (double)status[0];
-  r[17] = (double)status[1];
-  r[18] = err;
-  r[19] = smax;
-  flag[1] = k + 1;
-}
-
 void oa_step_free(oa_ctx* c) {
   oa_step_scratch* s = step_scratch(c);
   if (!s) return;
@@ -156,6 +138,9 @@ void oa_step_free(oa_ctx* c) {
   void* p[] = {s->F, s->F2, s->Fnl, s->S, s->lam, s->gam, s->flag, s->ring};
   for (void* q : p) if (q) cudaFree(q);
   if (s->ring_host) cudaFreeHost(s->ring_host);
+  if (s->fork) cudaEventDestroy(s->fork);
+  if (s->join) cudaEventDestroy(s->join);
+  if (s->side) cudaStreamDestroy(s->side);
   free(s);
   c->step = nullptr;
 }
@@ -174,16 +159,29 @@ oa_status oa_planes_psi_refresh(oa_ctx* c, cudaStream_t s, const double* psi, in
 static oa_status launch_step_a(oa_ctx* c, cudaStream_t s, oa_cp_state* st, int complete_prev) {
   oa_step_scratch* w = step_scratch(c);
   const int nt = st->mixed_nterm;
-  // forces on the orthonormal psi (computePsiFandVKS, ParticlePlane, combineForcesGetEke)
-  OA_STEP_TRY(oa_gpu_state_fft_fwd(c, s, st->psi, nullptr));
-  OA_STEP_TRY(oa_gpu_vks_build(c, s, nullptr));
+  // forces on the orthonormal psi (computePsiFandVKS, ParticlePlane, combineForcesGetEke).
+  // The nonlocal forces need psi and the atoms only, and the z pass at the
+  // end is the first to read them: they run on a second stream beside the
+  // density path, whose kernels (one grid in FP64, not one per state) leave
+  // most SMs idle.
+  OA_CUDA_TRY(oa_launch_phase_tables(c, s));
+  OA_CUDA_TRY(oa_launch_state_zfwd(c, s, (const double2*)st->psi, 0, c->nstate));
+  OA_CUDA_TRY(oa_launch_state_plane_density(c, s));
+  OA_CUDA_TRY(cudaEventRecord(w->fork, s));
+  OA_CUDA_TRY(cudaStreamWaitEvent(w->side, w->fork, 0));
+  OA_CUDA_TRY(oa_launch_rho_xc(c, s));
+  c->phase_done = 1;
+  const oa_status rv = oa_gpu_vks_build(c, s, nullptr);
+  c->phase_done = 0;
+  OA_STEP_TRY(rv);
   // nonlocal: the EES method once oa_gpu_ees_init enabled it
   // (cp_nonloc_ees_opt; CP_State_ParticlePlane.C:867-1136), else the
   // structure-factor method (StructureFactor.C:35-113)
-  if (c->ees) OA_STEP_TRY(oa_gpu_nl_ees(c, s, st->psi, w->Fnl, nullptr));
-  else OA_STEP_TRY(oa_gpu_nl_sf(c, s, st->psi, nt, w->Fnl, nullptr));
+  if (c->ees) OA_STEP_TRY(oa_gpu_nl_ees(c, w->side, st->psi, w->Fnl, nullptr));
+  else OA_STEP_TRY(oa_gpu_nl_sf(c, w->side, st->psi, nt, w->Fnl, nullptr));
+  OA_CUDA_TRY(cudaEventRecord(w->join, w->side));
   if (nt) oa_planes_force_begin(c, nt);
-  const oa_status rf = oa_gpu_vks_apply_fft_bwd(c, s, st->psi, 0, w->Fnl, w->F, nullptr);
+  const oa_status rf = oa_vks_apply(c, s, st->psi, 0, w->Fnl, w->join, w->F, nullptr);
   oa_planes_force_end(c, w->F);
   OA_STEP_TRY(rf);
   // constraint force (computeLambdaAndCg): Lambda, Gamma = T Lambda, F' = F T - Psi Gamma
@@ -223,14 +221,11 @@ static oa_status launch_step_ns(oa_ctx* c, cudaStream_t s, oa_cp_state* st) {
   return OA_OK;
 }
 
-// psi = psi_t T (FP64), the PsiV check and the step record (part B)
+// The step's energy sums, PsiV check and record, then psi = psi_t T (FP64)
+// with the reset that the check asked for (part B)
 static oa_status launch_step_b(oa_ctx* c, cudaStream_t s, oa_cp_state* st) {
   oa_step_scratch* w = step_scratch(c);
-  double *work, *errv, *dev_e, *hv, *eye;
-  int *status, *hs, grid;
-  OA_CUDA_TRY(oa_step_ortho_args(c, &work, &status, &errv, &grid, &dev_e, &hs, &hv, &eye));
-  k_step_check<<<1, 1, 0, s>>>(status, errv, dev_e, st->norb_tol, w->flag, w->ring, w->ring_cap);
-  OA_CUDA_TRY(cudaGetLastError());
+  OA_CUDA_TRY(oa_step_record(c, s, st->norb_tol, w->flag, w->ring, w->ring_cap));
   // psi = psi_t T, and the PsiV reset when the check asked for it
   OA_STEP_TRY(oa_psi_t_and_psiv(c, s, st->T, st->psi_t, st->psi, st->vpsi, st->T, w->flag, st->mixed_nterm, st->dt));
   return OA_OK;
