@@ -14,45 +14,8 @@
 // factor of cp_hart_ext.C gives E_ext = integral rho V_loc.
 #include "oa_internal.h"
 #include "oa_rdft.cuh"
-
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// block sum of NV doubles; results in out[] of thread 0
-template <int NV>
-__device__ void block_sum_n(double* v, double* sh /* 32*NV */) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = warp_sum_d(v[k]);
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh[k * 32 + wid] = v[k];
-  }
-  __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double r = (lane < nw) ? sh[k * 32 + lane] : 0.0;
-      v[k] = warp_sum_d(r);
-    }
-  }
-}
-
-__host__ __device__ static inline size_t align_up_r(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
-// 16-byte global -> shared copy without a register round trip, so that a
-// block's staging copies are all in flight together (the caller commits
-// the group and waits for it)
-__device__ __forceinline__ void rho_cp16(void* sdst, const void* gsrc) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc));
-}
-__device__ __forceinline__ void rho_cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void rho_cp_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+#include "oa_rho_common.cuh"
+#include "oa_lengths.h"
 
 // ---------------------------------------------------------------------------
 // density sum + PZ-LDA
@@ -247,325 +210,6 @@ k_rho_plane_bwd(const double2* __restrict__ dz, int ldl_d, int nx, int ny, int n
       if (y2 < ny) oz[y2 * nx + x] = (R)(v.y + (vz ? vz[y2 * nx + x] : 0.0));
     }
     __syncthreads();
-  }
-}
-
-struct RhoTypeOff { int off[5]; };
-
-// z pass: FFT(-) -> Hartree + local pseudopotential + Ewald (recip) in G -> FFT(+)
-// The structure factor S_t(g) = sum_{a in t} e^{i g.R_a} factorises per
-// z-line: pxy[line][a] = e^{i (gx x_a + gy y_a)} is formed once per block in
-// shared memory (atoms grouped by type), and each g of the line multiplies
-// it by the z phase e^{i gz z_a}.
-
-// FORCES: also the atom forces of the local pseudopotential and the
-// reciprocal Ewald sum (CP_hart_eext_calc's force loop, cp_hart_ext.C:300-360):
-// per g of the block the per-type coefficients
-//   A_t = w (Re rho v_t + Re S_q ewf q_t),  B_t = w (-Im rho v_t + Im S_q ewf q_t)
-// go to shared memory, then one warp per atom sums
-//   F_a += g (A_t Im h_a - B_t Re h_a),  h_a = e^{i g.R_a},
-// over the block's g-points into fpart[block][atom][3].
-// EES (ees.zq set; eesHartEextGchare / eesEwaldGchare, cp_hart_ext.C:1005-1340):
-// the per-type structure factors are b(g) Qhat_t(g), Qhat_t taken from the
-// transformed B-spline grids (types 2k, 2k+1 split from complex grid k by
-// the conjugate point -g); FORCES writes the per-type force transforms
-//   Y_t = v_t conj(rho b) + q_t ewf conj(b) S_q
-// (the Ewald part folded in by the type's charge) into ees.zy at g and, for
-// kx > 0, their conjugates at -g, instead of reducing over atoms here.
-template <int N1, int N2, bool FORCES>
-__global__ void __launch_bounds__(OA_NTHREADS, 2)
-k_rho_zpass(double2* __restrict__ dz, int ldl_d, int nlines_d, int nx, int ny, int nz,
-            OaFftPlan pz, const double2* __restrict__ twz,
-            double tpi_l, double vol, double ecut4, double falp2, double gz_term,
-            int natm, int ntype, const int* __restrict__ atm_perm, RhoTypeOff toff,
-            const double* __restrict__ q_type, const double2* __restrict__ phase, int ktab,
-            const double* __restrict__ spl, int nspl, double gmin, double dg,
-            double* __restrict__ part, double* __restrict__ fpart, EesLocArgs ees) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int ldz = nz + 1;
-  const bool use_ees = ees.zq != nullptr;
-  constexpr bool TP = N1 > 0;  // two-pass compile-time transforms
-  const int ldb = TP ? (ZLd<N1, N2>::PS > ldz ? ZLd<N1, N2>::PS : ldz) : ldz;
-  double2* tw = (double2*)smem_raw;
-  double2* a = tw + align_up_r(nz, 2);
-  double2* b = a + OA_LB * ldz;
-  double2* pxy = b + OA_LB * ldb;  // [OA_LB][natm], atoms in type order
-  __shared__ double sh[3 * 32];
-  const int l0 = blockIdx.x * OA_LB;
-  const int nb = min(OA_LB, nlines_d - l0);
-  const int nt = 2 * ktab + 1;
-  load_twiddles(tw, twz, nz);
-  int* zoff = (int*)(pxy + OA_LB * natm);  // [natm]: z-phase row of atom ia (type order)
-  // FORCES: [OA_LB * nz][ntype] per-type (A, B) coefficients after zoff
-  double2* cf = (double2*)(smem_raw + (((size_t)((char*)(zoff + natm) - (char*)smem_raw) + 15) & ~(size_t)15));
-  // the density coefficients of the block's lines: every 16-byte copy
-  // issued before any is waited for
-  for (int idx = threadIdx.x; idx < nz * OA_LB; idx += blockDim.x) {
-    const int zz = idx / OA_LB, lb = idx - zz * OA_LB;
-    if (lb < nb) rho_cp16(a + lb * ldz + zz, dz + (size_t)zz * ldl_d + l0 + lb);
-  }
-  rho_cp_commit();
-  for (int ia = threadIdx.x; ia < natm; ia += blockDim.x) zoff[ia] = (atm_perm[ia] * 3 + 2) * nt + ktab;
-#pragma unroll 4
-  for (int idx = use_ees ? OA_LB * natm : threadIdx.x; idx < OA_LB * natm; idx += blockDim.x) {
-    const int lb = idx / natm, ia = idx - lb * natm;
-    const int l = l0 + lb;
-    const int kx = l / ny;
-    int ky = l - kx * ny; if (2 * ky >= ny) ky -= ny;
-    double2 v = make_double2(0.0, 0.0);
-    if (lb < nb && kx <= ktab && abs(ky) <= ktab) {
-      const double2* ph = phase + (size_t)atm_perm[ia] * 3 * nt;
-      v = cmul(ph[kx + ktab], ph[nt + ky + ktab]);
-    }
-    pxy[lb * natm + ia] = v;
-  }
-  rho_cp_wait();
-  __syncthreads();
-  double2* r;
-  if constexpr (TP) {
-    zfft2<N1, N2, -1>(a, b, ldz, nb, tw);
-    r = a;
-  } else {
-    r = fft_pingpong<-1>(a, b, ldz, nb, pz, tw);
-  }
-  const double pi = 3.14159265358979323846;
-  const double fpi = 4.0 * pi;
-  double acc[3] = {0.0, 0.0, 0.0};
-  // One thread per (z, group of ZP_L lines): every z-phase load of the atom
-  // sums serves ZP_L g-points (the z phase depends on kz and the atom only),
-  // and the atoms' z-phase rows are addressed through zoff in shared memory.
-  constexpr int ZP_L = 2;
-  const int ngrp = (nb + ZP_L - 1) / ZP_L;
-  for (int idx = threadIdx.x; idx < ngrp * nz; idx += blockDim.x) {
-    const int grp = idx / nz, zz = idx - grp * nz;
-    int kz = zz; if (2 * kz >= nz) kz -= nz;
-    const double gzv = tpi_l * kz;
-    double2 rho[ZP_L], sf_q[ZP_L], vext[ZP_L];
-    double g2v[ZP_L], hh[ZP_L], wn[ZP_L];
-    double vtt[ZP_L][4];  // FORCES: v_t(|g|) / V per type
-    int cls[ZP_L], ii[ZP_L];  // cls: 0 outside, 1 g = 0, 2 inside the density sphere
-    size_t ep[ZP_L], em[ZP_L];  // EES: grid offsets of g and -g
-    double2 bgv[ZP_L];          // EES: b(g)
-    bool any = false;
-#pragma unroll
-    for (int j = 0; j < ZP_L; ++j) {
-      const int lb = grp * ZP_L + j;
-      cls[j] = 0; ii[j] = 1; hh[j] = 0.0; wn[j] = 1.0; g2v[j] = 0.0;
-      ep[j] = 0; em[j] = 0;
-      bgv[j] = make_double2(0.0, 0.0);
-      rho[j] = make_double2(0.0, 0.0);
-      sf_q[j] = make_double2(0.0, 0.0);
-      vext[j] = make_double2(0.0, 0.0);
-      if (lb >= nb) continue;
-      const int l = l0 + lb;
-      const int kx = l / ny;
-      int ky = l - kx * ny; if (2 * ky >= ny) ky -= ny;
-      if (use_ees && abs(kx) <= ktab && abs(ky) <= ktab && abs(kz) <= ktab) {
-        // kx >= 0 here; |k| <= ktab < n / 2 on each axis of the EES grid
-        const int ia = kx, ib = ky < 0 ? ky + ees.nb : ky, ic = kz < 0 ? kz + ees.nc : kz;
-        const int iam = kx == 0 ? 0 : ees.na - kx, ibm = ky > 0 ? ees.nb - ky : -ky, icm = kz > 0 ? ees.nc - kz : -kz;
-        ep[j] = ((size_t)ic * ees.nb + ib) * ees.na + ia;
-        em[j] = ((size_t)icm * ees.nb + ibm) * ees.na + iam;
-        bgv[j] = cmul(cmul(ees.ba[ia], ees.bb[ib]), ees.bc[ic]);
-      }
-      const double gx = tpi_l * kx, gy = tpi_l * ky;
-      const double g2 = gx * gx + gy * gy + gzv * gzv;
-      g2v[j] = g2;
-      rho[j] = r[lb * ldz + zz];
-      if (g2 == 0.0) {
-        cls[j] = 1;
-      } else if (g2 <= ecut4 && abs(kx) <= ktab && abs(ky) <= ktab && abs(kz) <= ktab) {
-        cls[j] = 2;
-        any = true;
-        wn[j] = (kx == 0) ? 1.0 : 2.0;
-        // spline interval of the local pseudopotential (CP_get_vpsnow, cp_hart_ext.C:433-480)
-        const double g = sqrt(g2);
-        int i1 = (int)((g - gmin) / dg + 1.0);
-        i1 = min(i1, nspl); i1 = max(i1, 1);
-        ii[j] = i1;
-        hh[j] = g - ((double)(i1 - 1) * dg + gmin);
-      }
-    }
-    if (any) {
-      // structure factors per type, S_t(g) = sum_{a in t} pxy[line][a] e^{i gz z_a},
-      // then V_ext = sum_t S_t v_t(|g|) / V and the Ewald charge sum sum_t q_t S_t
-      for (int t = 0; t < ntype && t < 4; ++t) {
-        double2 st[ZP_L];
-#pragma unroll
-        for (int j = 0; j < ZP_L; ++j) st[j] = make_double2(0.0, 0.0);
-        if (use_ees) {
-          // Qhat_t = (Z +- conj Z(-g)) / (2 or 2i) of grid t / 2, times b(g)
-          const double2* zg = ees.zq + (size_t)(t >> 1) * ees.gstride;
-#pragma unroll
-          for (int j = 0; j < ZP_L; ++j) {
-            if (cls[j] != 2) continue;
-            const double2 z = zg[ep[j]], zm = zg[em[j]];
-            const double2 qh = (t & 1) ? make_double2(0.5 * (z.y + zm.y), 0.5 * (zm.x - z.x))
-                                       : make_double2(0.5 * (z.x + zm.x), 0.5 * (z.y - zm.y));
-            st[j] = cmul(bgv[j], qh);
-          }
-        } else {
-          const double2* pl = pxy + grp * ZP_L * natm;
-          // four z-phase loads in flight per thread (the loop is bound by
-          // their latency, not by the multiply-adds)
-          // (the force variant, short of registers, takes them one at a time)
-          const int a0 = toff.off[t], a1 = toff.off[t + 1];
-          int ia = a0;
-          for (; !FORCES && ia + 4 <= a1; ia += 4) {
-            double2 hz[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) hz[u] = phase[zoff[ia + u] + kz];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-              for (int j = 0; j < ZP_L; ++j) {
-                const double2 h = cmul(pl[j * natm + ia + u], hz[u]);
-                st[j].x += h.x; st[j].y += h.y;
-              }
-          }
-          for (; ia < a1; ++ia) {
-            const double2 hz = phase[zoff[ia] + kz];
-#pragma unroll
-            for (int j = 0; j < ZP_L; ++j) {
-              const double2 h = cmul(pl[j * natm + ia], hz);
-              st[j].x += h.x; st[j].y += h.y;
-            }
-          }
-        }
-        const double qa = q_type[t];
-#pragma unroll
-        for (int j = 0; j < ZP_L; ++j) {
-          if (cls[j] != 2) continue;
-          sf_q[j].x += qa * st[j].x; sf_q[j].y += qa * st[j].y;
-          const double* cc = spl + ((size_t)t * nspl + (ii[j] - 1)) * 4;
-          const double vt = (((cc[3] * hh[j] + cc[2]) * hh[j] + cc[1]) * hh[j] + cc[0]) / vol;
-          vext[j].x += st[j].x * vt; vext[j].y += st[j].y * vt;
-          if constexpr (FORCES) vtt[j][t] = vt;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < ZP_L; ++j) {
-      const int lb = grp * ZP_L + j;
-      if (lb >= nb) continue;
-      double2 out = make_double2(0.0, 0.0);
-      if (cls[j] == 1) {
-        double gzt = gz_term;
-        if (use_ees) {
-          // sum_t gzvps_t b(0) Qhat_t(0) / V (eesHartEextGchare's g = 0 branch)
-          const double b0 = cmul(cmul(ees.ba[0], ees.bb[0]), ees.bc[0]).x;
-          gzt = 0.0;
-          for (int t = 0; t < ntype && t < 4; ++t) {
-            const double2 z0 = ees.zq[(size_t)(t >> 1) * ees.gstride];
-            const double yt = ees.gzvps[t] / vol * b0;
-            gzt += yt * ((t & 1) ? z0.y : z0.x);
-            if constexpr (FORCES) {
-              double* w0 = (double*)(ees.zy + (size_t)(t >> 1) * ees.gstride);
-              w0[t & 1] = yt * rho[j].x;
-            }
-          }
-        }
-        out.x = gzt;
-        acc[1] += gzt * rho[j].x;
-      } else if (cls[j] == 2) {
-        const double g2 = g2v[j];
-        const double hf = fpi / (g2 * vol);
-        acc[0] += hf * (rho[j].x * rho[j].x + rho[j].y * rho[j].y) * wn[j];
-        out.x = rho[j].x * hf; out.y = rho[j].y * hf;
-        const double ewf = fpi * exp(-g2 / falp2) / (g2 * vol);
-        acc[2] += ewf * (sf_q[j].x * sf_q[j].x + sf_q[j].y * sf_q[j].y) * wn[j];
-        out.x += vext[j].x; out.y -= vext[j].y;            // vks += conj(vext)
-        acc[1] += (rho[j].x * vext[j].x - rho[j].y * vext[j].y) * wn[j];  // Re(rho vext)
-      }
-      r[lb * ldz + zz] = out;
-      if (FORCES && use_ees) {
-        if (cls[j] == 2) {
-          const double g2 = g2v[j];
-          const double ewf = fpi * exp(-g2 / falp2) / (g2 * vol);
-          const double2 cb = cconj(bgv[j]);
-          const double2 rb = cconj(cmul(rho[j], bgv[j]));
-          const double2 sqe = cmul(cb, sf_q[j]);
-          const bool mirror = l0 + lb >= ny;  // kx > 0
-          for (int t0 = 0; t0 < ntype && t0 < 4; t0 += 2) {
-            double2 y[2];
-            for (int u = 0; u < 2; ++u) {
-              const int t = t0 + u;
-              y[u] = make_double2(0.0, 0.0);
-              if (t < ntype) {
-                const double qt = q_type[t] * ewf;
-                y[u].x = vtt[j][t] * rb.x + qt * sqe.x;
-                y[u].y = vtt[j][t] * rb.y + qt * sqe.y;
-              }
-            }
-            double2* w = ees.zy + (size_t)(t0 >> 1) * ees.gstride;
-            w[ep[j]] = make_double2(y[0].x - y[1].y, y[0].y + y[1].x);
-            if (mirror) w[em[j]] = make_double2(y[0].x + y[1].y, y[1].x - y[0].y);
-          }
-        }
-      } else if constexpr (FORCES) {
-        double2* c2 = cf + ((size_t)lb * nz + zz) * ntype;
-        for (int t = 0; t < ntype && t < 4; ++t) {
-          double2 ab = make_double2(0.0, 0.0);
-          if (cls[j] == 2) {
-            const double g2 = g2v[j];
-            const double ewf = fpi * exp(-g2 / falp2) / (g2 * vol);
-            const double qt = q_type[t];
-            ab.x = wn[j] * (rho[j].x * vtt[j][t] + sf_q[j].x * ewf * qt);
-            ab.y = wn[j] * (-rho[j].y * vtt[j][t] + sf_q[j].y * ewf * qt);
-          }
-          c2[t] = ab;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if (FORCES && !use_ees) {
-    // one warp per atom (type order), lanes over the block's (line, plane) points
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int ia = warp; ia < natm; ia += nwarp) {
-      int t = 0;
-      while (t + 1 < ntype && ia >= toff.off[t + 1]) ++t;
-      double fx = 0.0, fy = 0.0, fz = 0.0;
-      for (int e = lane; e < nb * nz; e += 32) {
-        const int lb = e / nz, zz = e - lb * nz;
-        const double2 ab = cf[((size_t)lb * nz + zz) * ntype + t];
-        if (ab.x == 0.0 && ab.y == 0.0) continue;
-        const int l = l0 + lb;
-        const int kx = l / ny;
-        int ky = l - kx * ny; if (2 * ky >= ny) ky -= ny;
-        int kz = zz; if (2 * kz >= nz) kz -= nz;
-        const double2 h = cmul(pxy[lb * natm + ia], phase[zoff[ia] + kz]);
-        const double comp = ab.x * h.y - ab.y * h.x;
-        fx += tpi_l * kx * comp;
-        fy += tpi_l * ky * comp;
-        fz += tpi_l * kz * comp;
-      }
-      fx = warp_sum_d(fx);
-      fy = warp_sum_d(fy);
-      fz = warp_sum_d(fz);
-      if (lane == 0) {
-        double* o = fpart + ((size_t)blockIdx.x * natm + atm_perm[ia]) * 3;
-        o[0] = fx; o[1] = fy; o[2] = fz;
-      }
-    }
-  }
-  double2* r2;
-  if constexpr (TP) {
-    zfft2<N1, N2, +1>(a, b, ldz, nb, tw);
-    r2 = a;
-  } else {
-    double2* other = (r == a) ? b : a;
-    r2 = fft_pingpong<+1>(r, other, ldz, nb, pz, tw);
-  }
-  for (int idx = threadIdx.x; idx < nz * OA_LB; idx += blockDim.x) {
-    const int zz = idx / OA_LB, lb = idx - zz * OA_LB;
-    if (lb < nb) dz[(size_t)zz * ldl_d + l0 + lb] = r2[lb * ldz + zz];
-  }
-  block_sum_n<3>(acc, sh);
-  if (threadIdx.x == 0) {
-    part[3 * blockIdx.x + 0] = acc[0];
-    part[3 * blockIdx.x + 1] = acc[1];
-    part[3 * blockIdx.x + 2] = acc[2];
   }
 }
 
@@ -812,6 +456,9 @@ k_rho_div_z(double2* __restrict__ dz, const double2* __restrict__ dzh, size_t fs
 
 cudaError_t oa_rho2_fwd(cudaStream_t s, int n, int nz, const double* rho, double scale, const double2* tw,
                         double2* dz, int ldl_d, int nf, size_t fin, size_t fout);
+cudaError_t oa_rho_zpass_plain(oa_ctx* c, cudaStream_t s, int nblk, double* part, double* fpart, const EesLocArgs& ees);
+cudaError_t oa_rho_zpass_forces(oa_ctx* c, cudaStream_t s, int nblk, double* part, double* fpart,
+                                const EesLocArgs& ees);
 cudaError_t oa_rho2_bwd(cudaStream_t s, int n, int nz, double2* dz, int ldl_d, const double2* tw,
                         const double* vxc, void* vks, int fp64, int nf, size_t fin, size_t fout);
 
@@ -861,9 +508,11 @@ cudaError_t oa_launch_rho_xc(oa_ctx* c, cudaStream_t s) {
 }
 
 int oa_rho_xc_nblk() { return 4 * 148; }
-int oa_rho_z_nblk(const oa_ctx* c) { return (c->nlines_d + OA_LB - 1) / OA_LB; }
+// blocks of the density z pass: sixteen lines with atom forces, else eight
+// (RhoZLB)
+int oa_rho_z_nblk(const oa_ctx* c) { return c->ions ? (c->nlines_d + 15) / 16 : (c->nlines_d + 7) / 8; }
 // offset of the GGA block partials (2 per block of k_rho_gga) in c->red
-size_t oa_rho_gga_red_off(const oa_ctx* c) { return (size_t)3 * oa_rho_xc_nblk() + 3 * (size_t)oa_rho_z_nblk(c); }
+size_t oa_rho_gga_red_off(const oa_ctx* c) { return (size_t)3 * oa_rho_xc_nblk() + 3 * (size_t)((c->nlines_d + 7) / 8); }
 
 cudaError_t oa_launch_phase_tables(oa_ctx* c, cudaStream_t s) {
   const double tpi_l = 2.0 * 3.14159265358979323846 / c->box;
@@ -918,7 +567,7 @@ static cudaError_t rho_xy_bwd(oa_ctx* c, cudaStream_t s, double2* src, const dou
 static cudaError_t gga_z(oa_ctx* c, cudaStream_t s, int div) {
   const double tpi_l = 2.0 * 3.14159265358979323846 / c->box;
   const size_t fst = (size_t)c->nz * c->ldl_d;
-  const int nbz = oa_rho_z_nblk(c);
+  const int nbz = (c->nlines_d + OA_LB - 1) / OA_LB;
   auto go = [&](auto grad_k, auto div_k, int ld) -> cudaError_t {
     const size_t sm = (align_up_r(c->nz, 2) + (size_t)3 * OA_LB * ld) * sizeof(double2);
     if (sm > (size_t)OA_MAX_SMEM) return cudaErrorNotSupported;
@@ -939,8 +588,7 @@ static cudaError_t gga_z(oa_ctx* c, cudaStream_t s, int div) {
   switch (c->nz) {
 #define OA_GZ(NN, A, B) \
   case NN: e = go(k_rho_grad_z<A, B>, k_rho_div_z<A, B>, gga_zbuf_ld<A, B>(c->nz)); break;
-    OA_GZ(12, 4, 3) OA_GZ(20, 4, 5) OA_GZ(24, 6, 4) OA_GZ(36, 6, 6) OA_GZ(40, 8, 5) OA_GZ(64, 8, 8)
-    OA_GZ(96, 12, 8) OA_GZ(108, 12, 9) OA_GZ(160, 16, 10)
+    OA_LENGTHS_ALL(OA_GZ)
 #undef OA_GZ
     default: e = cudaErrorNotSupported; break;
   }
@@ -962,14 +610,11 @@ static cudaError_t gga_front(oa_ctx* c, cudaStream_t s) {
 }
 
 cudaError_t oa_launch_rho_fft_hart(oa_ctx* c, cudaStream_t s) {
-  const double tpi_l = 2.0 * 3.14159265358979323846 / c->box;
   cudaError_t e;
   // phase tables exp(i 2 pi k x / L) (a native step makes them first of all)
   if (!c->phase_done && (e = oa_launch_phase_tables(c, s)) != cudaSuccess) return e;
   if ((e = rho_xy_fwd(c, s, c->rho, c->vol / c->npts, (double2*)c->dz, 1, 0, 0)) != cudaSuccess) return e;
   if (c->gga && (e = gga_front(c, s)) != cudaSuccess) return e;
-  RhoTypeOff toff;
-  for (int t = 0; t < 5; ++t) toff.off[t] = c->type_off[t];
   const int nbz = oa_rho_z_nblk(c);
   const bool forces = c->ions != nullptr;
   EesLocArgs ees{};
@@ -985,36 +630,9 @@ cudaError_t oa_launch_rho_fft_hart(oa_ctx* c, cudaStream_t s) {
     ees.na = L->na; ees.nb = L->nb; ees.nc = L->nc;
     ees.gstride = (size_t)L->na * L->nb * L->nc;
   }
-  auto zpass = [&](auto kern, int ldb) -> cudaError_t {
-    size_t smz =
-        (align_up_r(c->nz, 2) + (size_t)OA_LB * (c->nz + 1) + (size_t)OA_LB * ldb + (size_t)OA_LB * c->natm) *
-            sizeof(double2) +
-        (size_t)c->natm * sizeof(int);  // zoff
-    if (forces) smz = align_up_r(smz, 16) + (size_t)OA_LB * c->nz * c->ntype * sizeof(double2);
-    if (smz > (size_t)OA_MAX_SMEM) return cudaErrorNotSupported;
-    cudaError_t e2 = oa_smem_limit(kern);
-    if (e2 != cudaSuccess) return e2;
-    kern<<<nbz, OA_NTHREADS, smz, s>>>((double2*)c->dz, c->ldl_d, c->nlines_d, c->nx, c->ny, c->nz,
-                                       c->plan_z, c->tw_z, tpi_l, c->vol, c->ecut_rho,
-                                       4.0 * c->alp_ewd * c->alp_ewd, c->gzvps_sum / c->vol,
-                                       c->natm, c->ntype, c->atm_perm, toff, c->q_type, c->phase, c->kmax_tab,
-                                       c->spl, c->nspl, c->spl_gmin, c->spl_dg,
-                                       c->red + 3 * oa_rho_xc_nblk(), forces ? c->ions->fpart : nullptr, ees);
-    return cudaGetLastError();
-  };
-  auto ldb2 = [&](int n1, int n2) { const int p = (n1 * (n2 | 1)) | 1; return p > c->nz + 1 ? p : c->nz + 1; };
-  switch (c->nz) {
-#define OA_ZP(NN, A, B)                                                                      \
-  case NN:                                                                                   \
-    e = forces ? zpass(k_rho_zpass<A, B, true>, ldb2(A, B)) : zpass(k_rho_zpass<A, B, false>, ldb2(A, B)); \
-    break;
-    OA_ZP(12, 4, 3) OA_ZP(20, 4, 5) OA_ZP(24, 6, 4) OA_ZP(36, 6, 6) OA_ZP(40, 8, 5) OA_ZP(64, 8, 8)
-    OA_ZP(96, 12, 8) OA_ZP(108, 12, 9) OA_ZP(160, 16, 10)
-#undef OA_ZP
-    default: e = cudaErrorNotSupported; break;
-  }
-  if (e == cudaErrorNotSupported)
-    e = forces ? zpass(k_rho_zpass<0, 0, true>, c->nz + 1) : zpass(k_rho_zpass<0, 0, false>, c->nz + 1);
+  double* part = c->red + 3 * oa_rho_xc_nblk();
+  e = forces ? oa_rho_zpass_forces(c, s, nbz, part, c->ions->fpart, ees)
+             : oa_rho_zpass_plain(c, s, nbz, part, nullptr, ees);
   if (e != cudaSuccess) return e;
   // EES: the force grids back to real space and the atom forces from them
   if (c->eesl && forces && (e = oa_launch_eesl_forces(c, s)) != cudaSuccess) return e;

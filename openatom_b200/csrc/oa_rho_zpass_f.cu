@@ -1,0 +1,6 @@
+// Density z pass with atom forces (oa_rho_zpass.cuh).
+#include "oa_rho_zpass.cuh"
+
+cudaError_t oa_rho_zpass_forces(oa_ctx* c, cudaStream_t s, int nblk, double* part, double* fpart, const EesLocArgs& ees) {
+  return rho_zpass<true>(c, s, nblk, part, fpart, ees);
+}
