@@ -21,7 +21,8 @@ cudaError_t oa_launch_pc_fwd(cudaStream_t s, const double* A, const double* B, i
 cudaError_t oa_launch_pc_bwd(cudaStream_t s, const double* M1, const double* X1, double a1_kx0, double a1_rest,
                              const double* M2, const double* X2, double a2, int n, long ncol, long kx0_cols,
                              double* out);
-cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* B, int n, double alpha, double* C);
+cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* B, int n, double alpha, double* C,
+                                 const OaPlaneOut* pc = nullptr, const OaPlaneOut* pa = nullptr);
 int oa_ns_grid(int n, int device);
 int oa_pencil_supported(int n);
 int oa_ns_cluster_size(int n);
@@ -55,8 +56,8 @@ int oa_tg_nb(int n);
 cudaError_t oa_tfwd(cudaStream_t s, int nt, const __nv_bfloat16* PA, int rows_a, const __nv_bfloat16* PB, int rows_b,
                     int m, int n, long K, long ldp, double alpha, float* part, int max_kb, double* C, int* err_flag,
                     int nsm, const int* cond = nullptr);
-cudaError_t oa_tbwd(cudaStream_t s, int nt, const __nv_bfloat16* PM1, const __nv_bfloat16* PX1, double a1_kx0,
-                    double a1_rest, const __nv_bfloat16* PM2, const __nv_bfloat16* PX2, double a2, int nj, int nk,
+cudaError_t oa_tbwd(cudaStream_t s, int nt, const __nv_bfloat16* PM1, const __nv_bfloat16* PX1, int rx1, double a1_kx0,
+                    double a1_rest, const __nv_bfloat16* PM2, const __nv_bfloat16* PX2, int rx2, double a2, int nj, int nk,
                     long ncol, long ldx, long kx0_cols, double* out, int* err_flag, const double* yadd = nullptr,
                     const int* cond = nullptr);
 cudaError_t oa_launch_pc_fwd_mn(cudaStream_t s, const double* A, const double* B, int m, int n, long K,
@@ -70,7 +71,7 @@ cudaError_t oa_launch_nl_sf(cudaStream_t s, const int* kx, const int* ky, const 
                             const OaPlaneOut* po);
 cudaError_t oa_launch_nl_zscale(cudaStream_t s, const double* Z, int nstate, int natm_nl, const int* nl_atm,
                                 const int* atm_type, const double* vnorm, double rvol, const double* occ, double* zt,
-                                double* enl);
+                                double* enl, OaPlaneOut po);
 
 static thread_local char g_err[512] = "";
 
@@ -129,6 +130,8 @@ struct oa_ctx_pc {
   int ns_cluster;     // cluster Newton-Schulz size (0: use the cooperative kernel)
   int* ns_status;    // [2] device
   double* ns_err;    // [1] device
+  const double *m_ready, *m_ready2;  // M1, M2 whose planes are in pl_ma, pl_mb (m_planes)
+  int m_nt, m_nk, m_nj;
   int* partner;      // [nkx0_red]
   int* mirror;       // [nkx0] redundant point of a unique one, else -1
   double* cmass;     // [ng]
@@ -1103,12 +1106,14 @@ static cudaError_t ensure_planes(oa_ctx* c, cudaStream_t s, int nt, int slot, co
 void oa_planes_step_begin(oa_ctx* c) {
   oa_ctx_pc* p = pcx(c);
   p->pl_cache = 1;
+  p->m_ready = nullptr;
   for (int q = 0; q < 3; ++q)
     if (q != PL_PSI) p->pl_key[q].valid = false;
 }
 void oa_planes_step_end(oa_ctx* c) {
   oa_ctx_pc* p = pcx(c);
   p->pl_cache = 0;
+  p->m_ready = nullptr;
   for (int q = 0; q < 3; ++q)
     if (q != PL_PSI) p->pl_key[q].valid = false;
 }
@@ -1119,7 +1124,8 @@ static bool plane_out(oa_ctx* c, int slot, int rows, int nt, OaPlaneOut* po) {
   oa_ctx_pc* p = pcx(c);
   const int nb = oa_tg_nb(rows);
   if (!p->pl_big[slot] || !(nt == 2 || nt == 3)) return false;
-  const int rp = oa_tg_rows_pad(rows, nb);
+  // psi is the first operand of the forward products, whose tiles have 128 rows
+  const int rp = oa_tg_rows_pad(rows, slot == PL_PSI ? 128 : nb);
   if (rp > p->pl_rows || 2L * c->ng > p->pl_ld) return false;
   *po = OaPlaneOut{p->pl_big[slot], rp, p->pl_ld, nt};
   return true;
@@ -1128,6 +1134,29 @@ static void plane_mark(oa_ctx* c, int slot, const double* src, int rows, int row
   auto& k = pcx(c)->pl_key[slot];
   k.src = src; k.rows = rows; k.rows_pad = rows_pad; k.nt = nt; k.K = 2L * c->ng; k.kx0 = 0; k.w = 1.0;
   k.valid = true;
+}
+
+// The planes of M1 (and M2) of the next mixed_bwd product of this step, to be
+// written by the kernel that makes M1 (which reads M2): rows up to nkp,
+// leading size ldm, zero beyond nk x nj.  False: mixed_bwd splits them itself.
+static bool m_planes(oa_ctx* c, const double* M1, const double* M2, int nk, int nj, int nt, OaPlaneOut* p1,
+                     OaPlaneOut* p2) {
+  oa_ctx_pc* p = pcx(c);
+  const int nkp = oa_tg_rows_pad(nk, 32), ldm = oa_tg_rows_pad(nj, oa_tg_nb(nj));
+  if (!p->pl_cache || !(nt == 2 || nt == 3) || nkp > p->pl_rows || ldm > p->pl_rows) return false;
+  *p1 = OaPlaneOut{p->pl_ma, nkp, ldm, nt};
+  if (M2) *p2 = OaPlaneOut{p->pl_mb, nkp, ldm, nt};
+  p->m_ready = M1; p->m_ready2 = M2; p->m_nt = nt; p->m_nk = nk; p->m_nj = nj;
+  return true;
+}
+
+// Gamma = T Lambda of a mixed native step, with the planes of Gamma and T
+// that the backward product reads next
+oa_status oa_gamma_planes(oa_ctx* c, cudaStream_t s, const double* T, const double* lam, int nt, double* gam) {
+  OaPlaneOut pc{nullptr, 0, 0, 0}, pa{nullptr, 0, 0, 0};
+  m_planes(c, gam, T, c->nstate, c->nstate, nt, &pc, &pa);
+  OA_CUDA_TRY(oa_launch_small_gemm(s, T, lam, c->nstate, 1.0, gam, &pc, &pa));
+  return OA_OK;
 }
 
 // the next force z pass (oa_launch_state_zbwd) also writes the planes of F
@@ -1193,24 +1222,27 @@ static cudaError_t mixed_bwd(oa_ctx* c, cudaStream_t s, int nt, const double* M1
                              const int* cond) {
   oa_ctx_pc* p = pcx(c);
   const int mx = c->nstate > c->natm_nl ? c->nstate : c->natm_nl;
-  int nkp = oa_tg_rows_pad(nk, 32);
-  {
-    // planes of X1 already held with more zero rows (a multiple of 32) serve as they are
-    const auto& k = p->pl_key[s1];
-    if (p->pl_cache && k.valid && k.src == X1 && k.rows == nk && k.nt == nt && k.K == ncol && k.kx0 == 0 &&
-        k.rows_pad > nkp && k.rows_pad % 32 == 0 && k.rows_pad <= p->pl_rows)
-      nkp = k.rows_pad;
-  }
+  const int nkp = oa_tg_rows_pad(nk, 32);  // rows of the M planes and of the K loop
+  // planes of X already held with more zero rows serve as they are
+  auto held = [&](int slot, const double* X) {
+    const auto& k = p->pl_key[slot];
+    return p->pl_cache && k.valid && k.src == X && k.rows == nk && k.nt == nt && k.K == ncol && k.kx0 == 0 &&
+                   k.rows_pad > nkp && k.rows_pad <= p->pl_rows ? k.rows_pad : nkp;
+  };
+  const int rx1 = held(s1, X1), rx2 = M2 ? held(s2, X2) : 0;
   const int ldm = oa_tg_rows_pad(nj, oa_tg_nb(nj));  // M planes: leading size of whole N tiles, zero beyond nj
+  // M planes that the producer of M1 wrote (oa_m_planes) serve this product only
+  const bool mready = p->m_ready == M1 && p->m_ready2 == M2 && p->m_nt == nt && p->m_nk == nk && p->m_nj == nj;
+  p->m_ready = nullptr;
   if (nj <= mx && nk <= mx && ncol <= p->pl_ld && ldm <= p->pl_rows && nkp <= p->pl_rows && (!M2 || s1 != s2)) {
     bf16 *pm1 = (bf16*)p->pl_ma, *pm2 = (bf16*)p->pl_mb;
-    cudaError_t e = ensure_planes(c, s, nt, s1, X1, nk, nkp, ncol, 0, 1.0, cond);
-    if (e == cudaSuccess) e = oa_split_kc(s, nt, M1, nk, nkp, nj, nj, 0, 1.0, pm1, ldm, cond);
-    if (e == cudaSuccess && M2) e = ensure_planes(c, s, nt, s2, X2, nk, nkp, ncol, 0, 1.0, cond);
-    if (e == cudaSuccess && M2) e = oa_split_kc(s, nt, M2, nk, nkp, nj, nj, 0, 1.0, pm2, ldm, cond);
+    cudaError_t e = ensure_planes(c, s, nt, s1, X1, nk, rx1, ncol, 0, 1.0, cond);
+    if (e == cudaSuccess && !mready) e = oa_split_kc(s, nt, M1, nk, nkp, nj, nj, 0, 1.0, pm1, ldm, cond);
+    if (e == cudaSuccess && M2) e = ensure_planes(c, s, nt, s2, X2, nk, rx2, ncol, 0, 1.0, cond);
+    if (e == cudaSuccess && M2 && !mready) e = oa_split_kc(s, nt, M2, nk, nkp, nj, nj, 0, 1.0, pm2, ldm, cond);
     if (e != cudaSuccess) return e;
-    e = oa_tbwd(s, nt, pm1, (const bf16*)p->pl_big[s1], a1_kx0, a1_rest, M2 ? pm2 : nullptr,
-                M2 ? (const bf16*)p->pl_big[s2] : nullptr, a2, nj, nkp, ncol, p->pl_ld, kx0_cols, out, p->err_flag,
+    e = oa_tbwd(s, nt, pm1, (const bf16*)p->pl_big[s1], rx1, a1_kx0, a1_rest, M2 ? pm2 : nullptr,
+                M2 ? (const bf16*)p->pl_big[s2] : nullptr, rx2, a2, nj, nkp, ncol, p->pl_ld, kx0_cols, out, p->err_flag,
                 yadd, cond);
     if (e != cudaErrorNotSupported) return e;
   }
@@ -1390,8 +1422,10 @@ extern "C" oa_status oa_gpu_nl_sf(oa_ctx* c, void* stream, const double* psi, in
     OA_CUDA_TRY(oa_launch_pc_fwd_mn(s, psi, (const double*)c->sf, n, na, K, 0, 1.0, 1.0, p->part, p->nkb, c->zmat));
   else
     OA_CUDA_TRY(mixed_fwd(c, s, nterm, psi, (const double*)c->sf, n, na, K, 0, 1.0, 1.0, c->zmat, PL_PSI, PL_SF));
+  OaPlaneOut pz{nullptr, 0, 0, 0};
+  if (nterm > 0) m_planes(c, c->zt, nullptr, na, n, nterm, &pz, nullptr);
   OA_CUDA_TRY(oa_launch_nl_zscale(s, c->zmat, n, na, c->nl_atm, c->atm_type, c->nl_vnorm, 1.0 / c->vol, c->occ,
-                                  c->zt, c->enl));
+                                  c->zt, c->enl, pz));
   if (nterm == 0)
     OA_CUDA_TRY(oa_launch_pc_bwd_jk(s, c->zt, (const double*)c->sf, 1.0, 1.0, nullptr, nullptr, 0.0, n, na, K, 0,
                                     fnl_out));

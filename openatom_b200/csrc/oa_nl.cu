@@ -55,8 +55,17 @@ __global__ void k_nl_sf(const int* __restrict__ kx, const int* __restrict__ ky, 
 __global__ void __launch_bounds__(128)
 k_nl_zscale(const double* __restrict__ Z, int nstate, int natm_nl, const int* __restrict__ nl_atm,
             const int* __restrict__ atm_type, const double* __restrict__ vnorm, double rvol,
-            const double* __restrict__ occ, double* __restrict__ zt, double* __restrict__ enl) {
+            const double* __restrict__ occ, double* __restrict__ zt, double* __restrict__ enl, OaPlaneOut po) {
   const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (po.P) {
+    // also the bf16 planes of zt, zero in the padding rows and columns
+    if (s >= po.ldp) return;
+    for (int a = lane; a < po.rows_pad; a += 32) {
+      const bool in = a < natm_nl && s < nstate;
+      const double z = in ? -2.0 * (vnorm[atm_type[nl_atm[a]]] * rvol) * Z[(size_t)s * natm_nl + a] : 0.0;
+      oa_plane_put(po, a, s, z);
+    }
+  }
   if (s >= nstate) return;
   double e = 0.0;
   for (int a = lane; a < natm_nl; a += 32) {
@@ -83,8 +92,9 @@ cudaError_t oa_launch_nl_sf(cudaStream_t s, const int* kx, const int* ky, const 
 
 cudaError_t oa_launch_nl_zscale(cudaStream_t s, const double* Z, int nstate, int natm_nl, const int* nl_atm,
                                 const int* atm_type, const double* vnorm, double rvol, const double* occ, double* zt,
-                                double* enl) {
-  k_nl_zscale<<<(nstate + 3) / 4, 128, 0, s>>>(Z, nstate, natm_nl, nl_atm, atm_type, vnorm, rvol, occ, zt, enl);
+                                double* enl, OaPlaneOut po) {
+  const int cols = po.P ? (int)po.ldp : nstate;
+  k_nl_zscale<<<(cols + 3) / 4, 128, 0, s>>>(Z, nstate, natm_nl, nl_atm, atm_type, vnorm, rvol, occ, zt, enl, po);
   return cudaGetLastError();
 }
 

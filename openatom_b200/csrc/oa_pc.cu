@@ -186,7 +186,7 @@ k_pc_bwd_f64(const double* __restrict__ M1, const double* __restrict__ X1, doubl
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int n, double alpha,
-             double* __restrict__ C) {
+             double* __restrict__ C, OaPlaneOut pc, OaPlaneOut pa) {
   __shared__ double sA[16][17], sB[16][17];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int i0 = blockIdx.y * 16, j0 = blockIdx.x * 16;
@@ -203,6 +203,10 @@ k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int n, 
   }
   const int i = i0 + ty, j = j0 + tx;
   if (i < n && j < n) C[(size_t)i * n + j] = alpha * acc;
+  // bf16 planes of C and of A, zero in the padding rows and columns (the
+  // backward product reads them next; their split kernels were 3-4 us each)
+  if (pc.P && i < pc.rows_pad && j < pc.ldp) oa_plane_put(pc, i, j, i < n && j < n ? alpha * acc : 0.0);
+  if (pa.P && i < pa.rows_pad && j < pa.ldp) oa_plane_put(pa, i, j, i < n && j < n ? A[(size_t)i * n + j] : 0.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -609,9 +613,18 @@ cudaError_t oa_launch_pc_bwd(cudaStream_t s, const double* M1, const double* X1,
   return oa_launch_pc_bwd_jk(s, M1, X1, a1_kx0, a1_rest, M2, X2, a2, n, n, ncol, kx0_cols, out);
 }
 
-cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* B, int n, double alpha, double* C) {
-  dim3 grid((n + 15) / 16, (n + 15) / 16);
-  k_small_gemm<<<grid, 256, 0, s>>>(A, B, n, alpha, C);
+// pc, pa (optional): bf16 planes of C and of A written in the same pass
+cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* B, int n, double alpha, double* C,
+                                 const OaPlaneOut* pc, const OaPlaneOut* pa) {
+  const OaPlaneOut none{nullptr, 0, 0, 0}, c = pc ? *pc : none, a = pa ? *pa : none;
+  int rows = n, cols = n;
+  for (const OaPlaneOut* q : {&c, &a})
+    if (q->P) {
+      rows = q->rows_pad > rows ? q->rows_pad : rows;
+      cols = q->ldp > cols ? (int)q->ldp : cols;
+    }
+  dim3 grid((cols + 15) / 16, (rows + 15) / 16);
+  k_small_gemm<<<grid, 256, 0, s>>>(A, B, n, alpha, C, c, a);
   return cudaGetLastError();
 }
 

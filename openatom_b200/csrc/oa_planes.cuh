@@ -30,6 +30,19 @@ __device__ __forceinline__ void oa_bf16_digits(double v, int nt, __nv_bfloat16* 
   }
 }
 
+// planes of the element (r, c)
+__device__ __forceinline__ void oa_plane_put(const OaPlaneOut& po, int r, long c, double x) {
+  __nv_bfloat16 h[3];
+  oa_bf16_digits(x, po.nt, h);
+  __nv_bfloat16* base = (__nv_bfloat16*)po.P + oa_plane_at(r, c, po.rows_pad);
+  const size_t pstride = (size_t)po.rows_pad * po.ldp;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    if (q >= po.nt) break;
+    base[q * pstride] = h[q];
+  }
+}
+
 // planes of the pair (x, y) at row r, columns c and c + 1 (c even)
 __device__ __forceinline__ void oa_plane_put2(const OaPlaneOut& po, int r, long c, double x, double y) {
   __nv_bfloat16 hx[3], hy[3];

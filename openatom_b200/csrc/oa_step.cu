@@ -35,6 +35,7 @@ oa_status oa_gpu_integrate(oa_ctx* ctx, void* stream, const double* force, doubl
 }
 
 int oa_ns_capturable(oa_ctx* c);
+oa_status oa_gamma_planes(oa_ctx* c, cudaStream_t s, const double* T, const double* lam, int nt, double* gam);
 oa_status oa_vks_apply(oa_ctx* c, cudaStream_t s, const double* psi, int recompute_fwd, const double* fnl,
                        cudaEvent_t fnl_ready, double* force, double* eke_out);
 oa_status oa_integrate_sel(oa_ctx* c, cudaStream_t s, const double* force, double* vpsi, double* psi,
@@ -187,7 +188,7 @@ static oa_status launch_step_a(oa_ctx* c, cudaStream_t s, oa_cp_state* st, int c
   // constraint force (computeLambdaAndCg): Lambda, Gamma = T Lambda, F' = F T - Psi Gamma
   if (nt) {
     OA_STEP_TRY(oa_gpu_pc_forward_mixed(c, s, st->psi, w->F, 1.0, 1.0, nt, w->lam));
-    OA_STEP_TRY(oa_gpu_small_gemm(c, s, st->T, w->lam, 1.0, w->gam));
+    OA_STEP_TRY(oa_gamma_planes(c, s, st->T, w->lam, nt, w->gam));
     OA_STEP_TRY(oa_gpu_pc_backward_mixed(c, s, w->gam, st->psi, -0.5, -1.0, st->T, w->F, 1.0, nt, w->F2));
   } else {
     OA_STEP_TRY(oa_gpu_pc_forward(c, s, st->psi, w->F, 1.0, 1.0, w->lam));

@@ -107,6 +107,23 @@ __device__ __forceinline__ void tg_tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// two such loads in flight, one wait
+__device__ __forceinline__ void tg_tmem_ld16x2(uint32_t ta, uint32_t tb, float* u, float* v) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+        "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]),
+        "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23]),
+        "=&r"(r[24]), "=&r"(r[25]), "=&r"(r[26]), "=&r"(r[27]), "=&r"(r[28]), "=&r"(r[29]), "=&r"(r[30]), "=&r"(r[31])
+      : "r"(ta), "r"(tb)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { u[i] = __uint_as_float(r[i]); v[i] = __uint_as_float(r[16 + i]); }
+}
+
 // ---------------------------------------------------------------------------
 // FP64 [rows][K] (row stride ldx) -> planes P[q][ldp/64][rows_pad][64],
 // columns k < kx0_cols scaled by w_kx0 first; padding columns [K, ldp) and
@@ -348,7 +365,11 @@ k_tfwd_reduce(const float* __restrict__ part, int nkb, size_t nn, double alpha, 
 //   accf[b]  : accumulator b complete           (MMA commit -> epilogue)
 //   acce[b]  : accumulator b read out           (4 epilogue warps -> MMA)
 // ---------------------------------------------------------------------------
-#define TB_THREADS 192
+// TMA producer, MMA issuer, eight epilogue warps.  With four the epilogue
+// bound the kernel (one warp per scheduler, each waiting for its own TMEM
+// loads and stores): 58 us at 128 states, 40115 coefficients
+#define TB_EPI 8
+#define TB_THREADS (64 + 32 * TB_EPI)
 
 __device__ __forceinline__ void tg_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(tg_s32(bar)) : "memory");
@@ -381,7 +402,7 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
   const int nslab = nterm * kch;
   if (tid == 0) {
     for (int s = 0; s < stages; ++s) { tg_bar_init(&full[s], 1); tg_bar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { tg_bar_init(&accf[b], 1); tg_bar_init(&acce[b], 4); }
+    for (int b = 0; b < 2; ++b) { tg_bar_init(&accf[b], 1); tg_bar_init(&acce[b], TB_EPI); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *okflag = 1;
   }
@@ -470,9 +491,11 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
       if (!ok) *okflag = 0;
     }
   } else {
-    // epilogue: TMEM lane quarter q = warp & 3 holds columns c0 + 32 q ..
+    // epilogue: TMEM lane quarter q = warp & 3 holds columns c0 + 32 q ..;
+    // the two warps of a quarter take half of the output rows each
     const int q = warp & 3;
     const int row = q * 32 + lane;
+    const int jh = ((warp - 2) >> 2) * (NB / 2);
     for (int i = 0; i < my_tiles; ++i) {
       const int b = i & 1;
       if (!tg_wait(&accf[b], (uint32_t)((i >> 1) & 1))) { *okflag = 0; break; }
@@ -480,30 +503,42 @@ k_tbwd(const __grid_constant__ CUtensorMap tX1, const __grid_constant__ CUtensor
       if (!*okflag) break;
       const int tile = (int)blockIdx.x + i * (int)gridDim.x, ct = njt == 1 ? tile : tile / njt;
       const long c = (long)ct * TG_M + row;
-      const int jb = (tile - ct * njt) * NB;  // first output row of the tile
-      const int nje = nj - jb;                // output rows from there
-      double* oc = out + (size_t)jb * ncol + c;
-      const double* yc = yadd ? yadd + (size_t)jb * ncol + c : nullptr;
+      const int jb = (tile - ct * njt) * NB + jh;  // first output row
+      const int nje = nj - jb;                     // output rows from there
+      double* o = out + (size_t)jb * ncol + c;
+      const double* y = yadd ? yadd + (size_t)jb * ncol + c : nullptr;
       const double a1 = (c < kx0_cols) ? a1_kx0 : a1_rest;
-      const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * NBP);
-      for (int q0 = 0; q0 < NB; q0 += 16) {
+      const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * NBP + jh);
+      for (int q0 = 0; q0 < NB / 2 && q0 < nje; q0 += 16) {
         float v1[16], v2[16];
-        tg_tmem_ld16(tbase + (uint32_t)q0, v1);
-        if (nterm == 2) tg_tmem_ld16(tbase + (uint32_t)(NBP + q0), v2);
+        if (nterm == 2) {
+          tg_tmem_ld16x2(tbase + (uint32_t)q0, tbase + (uint32_t)(NBP + q0), v1, v2);
+        } else {
+          tg_tmem_ld16(tbase + (uint32_t)q0, v1);
+        }
         if (c < ncol) {
-          // yadd may be out itself: all 16 reads go before the writes
-          double ya[16];
-#pragma unroll
-          for (int e = 0; e < 16; ++e) ya[e] = (yc && q0 + e < nje) ? yc[(size_t)(q0 + e) * ncol] : 0.0;
+          double r[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const int j = q0 + e;
-            if (j < nje) {
-              double r = a1 * (double)v1[e];
-              if (nterm == 2) r += a2 * (double)v2[e];
-              oc[(size_t)j * ncol] = r + ya[e];
-            }
+            r[e] = a1 * (double)v1[e];
+            if (nterm == 2) r[e] += a2 * (double)v2[e];
           }
+          // yadd may be out itself: all 16 reads go before the writes
+          if (y) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              if (q0 + e < nje) r[e] += y[(size_t)e * ncol];
+            y += (size_t)16 * ncol;
+          }
+          if (q0 + 16 <= nje) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) o[(size_t)e * ncol] = r[e];
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              if (q0 + e < nje) o[(size_t)e * ncol] = r[e];
+          }
+          o += (size_t)16 * ncol;
         }
       }
       tg_tc_before();
@@ -619,23 +654,24 @@ cudaError_t oa_tfwd(cudaStream_t s, int nt, const bf16* PA, int rows_a, const bf
 }
 
 // out[j][c] = a1(c) sum_k M1[k][j] X1[k][c] + a2 sum_k M2[k][j] X2[k][c]
-// (+ yadd[j][c], which may be out itself) from X planes (rows nk, leading
-// size ldx) and M planes (rows nk, leading size nj rounded up to the N
+// (+ yadd[j][c], which may be out itself) from X planes (rows rx1, rx2 >= nk,
+// leading size ldx) and M planes (rows nk, leading size nj rounded up to the N
 // tile oa_tg_nb(nj), zero beyond nj); nk a multiple of 32 (planes padded with zero rows).  cond: optional device flag, nothing runs
 // when it is 0.
-cudaError_t oa_tbwd(cudaStream_t s, int nt, const bf16* PM1, const bf16* PX1, double a1_kx0, double a1_rest,
-                    const bf16* PM2, const bf16* PX2, double a2, int nj, int nk, long ncol, long ldx, long kx0_cols,
+cudaError_t oa_tbwd(cudaStream_t s, int nt, const bf16* PM1, const bf16* PX1, int rx1, double a1_kx0, double a1_rest,
+                    const bf16* PM2, const bf16* PX2, int rx2, double a2, int nj, int nk, long ncol, long ldx, long kx0_cols,
                     double* out, int* err_flag, const double* yadd, const int* cond) {
   const int nb = oa_tg_nb(nj);
-  if (((PM2 == nullptr) != (PX2 == nullptr)) || nk < TG_KS || (nk % TG_KS)) return cudaErrorNotSupported;
+  if (((PM2 == nullptr) != (PX2 == nullptr)) || nk < TG_KS || (nk % TG_KS) || rx1 < nk || (PX2 && rx2 < nk))
+    return cudaErrorNotSupported;
   const int stages = tg_stages(nt, nb, false);
   if (stages < 2) return cudaErrorNotSupported;
   const int njt = (nj + nb - 1) / nb;
   CUtensorMap tx1, tm1, tx2, tm2;
-  if (!tg_map(&tx1, PX1, nt, nk, ldx, TG_KS) || !tg_map(&tm1, PM1, nt, nk, njt * nb, TG_KS)) return cudaErrorNotSupported;
+  if (!tg_map(&tx1, PX1, nt, rx1, ldx, TG_KS) || !tg_map(&tm1, PM1, nt, nk, njt * nb, TG_KS)) return cudaErrorNotSupported;
   const int nterm = PM2 ? 2 : 1;
   if (nterm == 2) {
-    if (!tg_map(&tx2, PX2, nt, nk, ldx, TG_KS) || !tg_map(&tm2, PM2, nt, nk, njt * nb, TG_KS)) return cudaErrorNotSupported;
+    if (!tg_map(&tx2, PX2, nt, rx2, ldx, TG_KS) || !tg_map(&tm2, PM2, nt, nk, njt * nb, TG_KS)) return cudaErrorNotSupported;
   } else {
     tx2 = tx1; tm2 = tm1;
   }
