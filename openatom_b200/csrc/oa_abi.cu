@@ -125,7 +125,7 @@ cudaError_t oa_oz_rotate(oa_oz* z, cudaStream_t s, const double* T, const double
 struct oa_ctx_pc {
   double* part;      // split-K partials
   int nkb;
-  double* ns_work;   // 5 n^2 + grid
+  double* ns_work;   // 5 n^2 + 2 grid
   int ns_grid;        // cooperative Newton-Schulz blocks
   int ns_cluster;     // cluster Newton-Schulz size (0: use the cooperative kernel)
   int* ns_status;    // [2] device
@@ -469,7 +469,7 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
                                  sizeof(double)));
     p->ns_grid = oa_ns_grid(d->nstate, c->device);
     p->ns_cluster = oa_ns_cluster_size(d->nstate);
-    TRY(cudaMalloc(&p->ns_work, ((size_t)5 * d->nstate * d->nstate + p->ns_grid + 32) * sizeof(double)));
+    TRY(cudaMalloc(&p->ns_work, ((size_t)5 * d->nstate * d->nstate + 2 * p->ns_grid + 32) * sizeof(double)));
     TRY(cudaMalloc(&p->ns_status, 4 * sizeof(int)));  // [2] status, [3] ticket of the step record
     TRY(cudaMemset(p->ns_status, 0, 4 * sizeof(int)));
     TRY(cudaMalloc(&p->ns_err, 2 * sizeof(double)));

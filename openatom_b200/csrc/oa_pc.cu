@@ -218,100 +218,149 @@ k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int n, 
 //   status[1] = 1 if converged; errv[0] = err.
 // ---------------------------------------------------------------------------
 #define NS_TS 32
+#define NS_LD (NS_TS + 4)   // fragment loads on different banks
+#define NS_STAGES 3
+#define NS_SMEM (NS_STAGES * 2 * NS_TS * NS_LD * sizeof(double))
 
-__device__ void ns_tile_gemm(const double* __restrict__ X, const double* __restrict__ Y, int n, double alpha,
-                             double diag, double* __restrict__ Z, int tile, double* sX, double* sY,
-                             const double* __restrict__ Aold, double* err_acc) {
-  // Z[tile] = alpha * X Y + diag * I ; optional err += (Aold - Z)^2 on the tile
-  const int nt = (n + NS_TS - 1) / NS_TS;
-  const int ti = tile / nt, tj = tile - ti * nt;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int k0 = 0; k0 < n; k0 += NS_TS) {
-    __syncthreads();
-    for (int r = ty; r < NS_TS; r += 8) {
-      const int i = ti * NS_TS + r, k = k0 + tx;
-      sX[r * (NS_TS + 1) + tx] = (i < n && k < n) ? X[(size_t)i * n + k] : 0.0;
-      const int kk = k0 + r, j = tj * NS_TS + tx;
-      sY[r * (NS_TS + 1) + tx] = (kk < n && j < n) ? Y[(size_t)kk * n + j] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int k = 0; k < NS_TS; ++k) {
-      const double y = sY[k * (NS_TS + 1) + tx];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] += sX[(ty + 8 * q) * (NS_TS + 1) + k] * y;
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = ti * NS_TS + ty + 8 * q, j = tj * NS_TS + tx;
-    if (i < n && j < n) {
-      double v = alpha * acc[q] + ((i == j) ? diag : 0.0);
-      Z[(size_t)i * n + j] = v;
-      if (Aold) { const double d = Aold[(size_t)i * n + j] - v; *err_acc += d * d; }
-    }
-  }
+// two doubles (one for odd n) global -> shared past the L1 (other blocks wrote
+// them), zeros when not valid; the wide form in the background
+__device__ __forceinline__ void ns_cp(double* dst, const double* src, bool wide, bool valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+  else *dst = valid ? __ldcg(src) : 0.0;
 }
 
-__global__ void __launch_bounds__(256)
+// Z[tile] = alpha * X Y + diag * I ; optional err += (Aold - Z)^2 on the tile.
+// A 32 x 32 tile by 8 warps of 8 x 16 (DMMA), slabs of 32 k through a ring of
+// three; each warp keeps even and odd k steps in separate accumulators, four
+// independent chains.
+__device__ void ns_tile_gemm(const double* X, const double* Y, int n, double alpha, double diag, double* Z, int tile,
+                             double* sm, const double* Aold, double* err_acc) {
+  const int nt = (n + NS_TS - 1) / NS_TS;
+  const int ti = tile / nt, tj = tile - ti * nt;
+  const int i0 = ti * NS_TS, j0 = tj * NS_TS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wr = (warp >> 1) * 8, wc = (warp & 1) * 16;
+  const bool wide = (n & 1) == 0;
+  auto issue = [&](int s) {
+    const int k0 = s * NS_TS;
+    double* sx = sm + (s % NS_STAGES) * 2 * NS_TS * NS_LD;
+    double* sy = sx + NS_TS * NS_LD;
+    const int w = wide ? 2 : 1, per = NS_TS / w;
+    for (int q = threadIdx.x; q < NS_TS * per; q += 256) {
+      const int r = q / per, c = (q - r * per) * w;
+      const bool vx = i0 + r < n && k0 + c < n, vy = k0 + r < n && j0 + c < n;
+      ns_cp(sx + r * NS_LD + c, vx ? X + (size_t)(i0 + r) * n + k0 + c : X, wide, vx);
+      ns_cp(sy + r * NS_LD + c, vy ? Y + (size_t)(k0 + r) * n + j0 + c : Y, wide, vy);
+    }
+  };
+  double acc[2][2][2] = {};  // [k parity][column tile][element]
+  for (int s = 0; s < NS_STAGES - 1; ++s) {
+    if (s < nt) issue(s);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  for (int s = 0; s < nt; ++s) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(NS_STAGES - 2) : "memory");
+    __syncthreads();
+    if (s + NS_STAGES - 1 < nt) issue(s + NS_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const double* sx = sm + (s % NS_STAGES) * 2 * NS_TS * NS_LD + (wr + (lane >> 2)) * NS_LD + (lane & 3);
+    const double* sy = sm + ((s % NS_STAGES) * 2 + 1) * NS_TS * NS_LD + (lane & 3) * NS_LD + wc + (lane >> 2);
+#pragma unroll
+    for (int k4 = 0; k4 < NS_TS / 4; ++k4) {
+      const double a = sx[k4 * 4], b0 = sy[k4 * 4 * NS_LD], b1 = sy[k4 * 4 * NS_LD + 8];
+      dmma_8x8x4(acc[k4 & 1][0][0], acc[k4 & 1][0][1], a, b0);
+      dmma_8x8x4(acc[k4 & 1][1][0], acc[k4 & 1][1][1], a, b1);
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();  // the next tile refills the ring
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = i0 + wr + (lane >> 2), j = j0 + wc + b * 8 + 2 * (lane & 3) + e;
+      if (i < n && j < n) {
+        const double v = alpha * (acc[0][b][e] + acc[1][b][e]) + ((i == j) ? diag : 0.0);
+        Z[(size_t)i * n + j] = v;
+        if (Aold) { const double d = __ldcg(Aold + (size_t)i * n + j) - v; *err_acc += d * d; }
+      }
+    }
+}
+
+// More than 128 states (or an odd count above 48).  What bounds it are the grid
+// barriers and the chain of small products, three per iteration: a barrier after
+// C and one after the two others, which run side by side on twice the blocks.
+// Against FMA tiles, one after the other, with three barriers and a serial sum
+// of the error partials: 199 states 325 -> 205 us, 260 390 -> 130, 512 777 -> 311.
+__global__ void __launch_bounds__(256, 4)
 k_ortho_ns(const double* __restrict__ S, int n, double bscale, double tol, int max_iter,
-           double* __restrict__ A0, double* __restrict__ A1, double* __restrict__ B0, double* __restrict__ B1,
-           double* __restrict__ Cm, double* __restrict__ errpart, double* __restrict__ T,
+           double* A0, double* A1, double* B0, double* B1, double* Cm, double* errpart, double* __restrict__ T,
            int* __restrict__ status, double* __restrict__ errv) {
   cg::grid_group grid = cg::this_grid();
-  __shared__ double sX[NS_TS * (NS_TS + 1)];
-  __shared__ double sY[NS_TS * (NS_TS + 1)];
+  extern __shared__ __align__(16) double ns_sm[];
   __shared__ double sred[32];
-  __shared__ int sdone;
   const int nt = (n + NS_TS - 1) / NS_TS;
   const int ntiles = nt * nt;
   const size_t nn = (size_t)n * n;
-  // init: A = I, B = S * bscale; max |S - I/bscale| (Ortho::array_diag_max,
-  // ortho.h:282-310) for the PsiV tolerance check
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // init: A = I, B = S * bscale, the first C = 3I - B; max |S - I/bscale|
+  // (Ortho::array_diag_max, ortho.h:282-310) for the PsiV tolerance check
   double dmax = 0.0;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (size_t)gridDim.x * blockDim.x) {
     const int r = (int)(i / n), c = (int)(i - (size_t)r * n);
-    A0[i] = (r == c) ? 1.0 : 0.0;
-    B0[i] = S[i] * bscale;
-    const double dv = fabs(S[i] - ((r == c) ? 1.0 / bscale : 0.0));
+    const double sv = S[i], b = sv * bscale;
+    B0[i] = b;
+    Cm[i] = ((r == c) ? 3.0 : 0.0) - b;
+    const double dv = fabs(sv - ((r == c) ? 1.0 / bscale : 0.0));
     dmax = dv > dmax ? dv : dmax;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = dmax;
+  if (lane == 0) sred[warp] = dmax;
   __syncthreads();
+  double* maxpart = errpart + gridDim.x;
   if (threadIdx.x == 0) {
     double m = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, sred[w]);
-    errpart[blockIdx.x] = m;
+    maxpart[blockIdx.x] = m;
   }
   grid.sync();
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && warp == 0) {
     double m = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) m = fmax(m, errpart[b]);
-    errv[1] = m;
+    for (int b = lane; b < (int)gridDim.x; b += 32) m = fmax(m, __ldcg(maxpart + b));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) errv[1] = m;
   }
-  grid.sync();
   double* A = A0; double* An = A1; double* B = B0; double* Bn = B1;
   int it = 0;
   double err = 1.0;
   while (true) {
-    // C = 3I - A B
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-      ns_tile_gemm(A, B, n, -1.0, 3.0, Cm, t, sX, sY, nullptr, nullptr);
-    grid.sync();
-    // Bn = B C / 2 ; An = C A / 2 with error partials
-    double e_loc = 0.0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      ns_tile_gemm(B, Cm, n, 0.5, 0.0, Bn, t, sX, sY, nullptr, nullptr);
-      ns_tile_gemm(Cm, A, n, 0.5, 0.0, An, t, sX, sY, A, &e_loc);
+    // C = 3I - A B (the first is made above)
+    if (it > 0) {
+      for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
+        ns_tile_gemm(A, B, n, -1.0, 3.0, Cm, t, ns_sm, nullptr, nullptr);
+      grid.sync();
     }
+    // Bn = B C / 2 ; An = C A / 2 with error partials (C / 2 while A = I)
+    double e_loc = 0.0;
+    for (int t = blockIdx.x; t < (it > 0 ? 2 : 1) * ntiles; t += gridDim.x) {
+      if (t < ntiles) ns_tile_gemm(B, Cm, n, 0.5, 0.0, Bn, t, ns_sm, nullptr, nullptr);
+      else ns_tile_gemm(Cm, A, n, 0.5, 0.0, An, t - ntiles, ns_sm, A, &e_loc);
+    }
+    if (it == 0)
+      for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (size_t)gridDim.x * blockDim.x) {
+        const int r = (int)(i / n), c = (int)(i - (size_t)r * n);
+        const double v = 0.5 * __ldcg(Cm + i), d = ((r == c) ? 1.0 : 0.0) - v;
+        An[i] = v;
+        e_loc += d * d;
+      }
     // deterministic per-block partial
     double v = e_loc;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = v;
+    if (lane == 0) sred[warp] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
       double s = 0.0;
@@ -320,22 +369,18 @@ k_ortho_ns(const double* __restrict__ S, int n, double bscale, double tol, int m
     }
     grid.sync();
     ++it;
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int b = 0; b < (int)gridDim.x; ++b) s += errpart[b];
-      err = sqrt(s / (double)nn);
-      sdone = !(err > tol && it < max_iter);
-      sred[0] = err;
-    }
-    __syncthreads();
-    err = sred[0];
-    const int done = sdone;
+    // every warp sums the partials in the same order; they are rewritten
+    // only after the barrier behind the next C
+    double s = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(errpart + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    err = sqrt(s / (double)nn);
     { double* t = A; A = An; An = t; t = B; B = Bn; Bn = t; }
-    if (done) break;
-    // errpart is rewritten next iteration only after the next grid.sync
-    grid.sync();
+    if (!(err > tol && it < max_iter)) break;
   }
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (size_t)gridDim.x * blockDim.x) T[i] = A[i];
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (size_t)gridDim.x * blockDim.x)
+    T[i] = __ldcg(A + i);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     status[0] = it;
     status[1] = (err <= tol) ? 1 : 0;
@@ -643,10 +688,11 @@ cudaError_t oa_launch_step_record(cudaStream_t s, const OaSumJobs& J, const int*
 int oa_ns_grid(int n, int device) {
   const int nt = (n + NS_TS - 1) / NS_TS;
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ortho_ns, 256, 0);
+  if (oa_smem_limit(k_ortho_ns) != cudaSuccess) cudaGetLastError();
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ortho_ns, 256, NS_SMEM);
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  int g = nt * nt;
+  int g = 2 * nt * nt;  // B C and C A side by side
   const int cap = per_sm * nsm;
   if (g > cap) g = cap;
   if (g < 1) g = 1;
@@ -661,7 +707,7 @@ cudaError_t oa_launch_ortho_ns_cluster(cudaStream_t s, const double* S, int n, d
 // grid > 0: cooperative kernel on grid blocks; grid < 0: the cluster kernel
 // (oa_ns.cu) on a cluster of -grid blocks
 cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
-                               double* work /* 5 n^2 + grid */, double* T, int* status, double* errv, int grid) {
+                               double* work /* 5 n^2 + 2 grid */, double* T, int* status, double* errv, int grid) {
   // few states: one block (oa_ns.cu)
   const cudaError_t eb = oa_launch_ortho_ns_block(s, S, n, bscale, tol, max_iter, T, status, errv);
   if (eb != cudaErrorNotSupported) return eb;
@@ -671,7 +717,9 @@ cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bs
   double* errpart = Cm + nn;
   void* args[] = {(void*)&S, (void*)&n, (void*)&bscale, (void*)&tol, (void*)&max_iter, (void*)&A0, (void*)&A1,
                   (void*)&B0, (void*)&B1, (void*)&Cm, (void*)&errpart, (void*)&T, (void*)&status, (void*)&errv};
-  return cudaLaunchCooperativeKernel((void*)k_ortho_ns, dim3(grid), dim3(256), args, 0, s);
+  const cudaError_t el = oa_smem_limit(k_ortho_ns);
+  if (el != cudaSuccess) return el;
+  return cudaLaunchCooperativeKernel((void*)k_ortho_ns, dim3(grid), dim3(256), args, NS_SMEM, s);
 }
 
 cudaError_t oa_launch_integrate(cudaStream_t s, const double2* F, double2* V, double2* P, const double2* P_in,
