@@ -1,7 +1,6 @@
 """Autotuner of the runtime tile and schedule choices of a context
-(oa_tuning: state groups of the per-state and state-pair plane kernels,
-split-K blocks of the FP64 products, the FFT path) per system size and
-precision.
+(oa_tuning: groups of the state-pair plane kernels, split-K blocks of the
+FP64 products, the FFT path) per system size and precision.
 
 For each system it runs coordinate descent over the knobs: every candidate
 value is set (oa_gpu_set_tuning) on a fresh context started from the same
@@ -77,7 +76,7 @@ def knobs_for(precision: str) -> tuple:
     stays at the built-in choice, the largest the partials allow)."""
     if precision == "mixed":
         return ("group_pair", "dgemm_kblocks")
-    return ("group_state", "dgemm_kblocks", "fft_path")
+    return ("group_pair", "dgemm_kblocks", "fft_path")
 
 
 def _time_steps(torch, drv, st, steps: int, reps: int) -> float:
