@@ -318,50 +318,62 @@ cudaError_t oa_dgemm_fwd(cudaStream_t s, const double* A, const double* B, int m
 // bwMultiplyDynOrthoT, ckPairCalculator.C:1201-1468, 1710-2031):
 //   out[j][c] = a1(c) sum_k M1[k][j] X1[k][c] + a2 sum_k M2[k][j] X2[k][c]
 //   a1(c) = a1_kx0 for c < kx0_cols, else a1_rest
-// CTA tile: 128 rows j x 64 columns c, all k; 8 warps of 32 x 32.  The M and
-// X slabs of 16 k rows move through a 4-stage cp.async ring; the two terms
-// run as one slab sequence.  The first term's sum is scaled by a1(c) in
-// registers once it is complete; the second term's M fragments are scaled
-// by a2 as they are read, so one accumulator set serves both terms.
+// CTA tile: TJ rows j x 64 columns c, all k; one warp per 32 x 32.  TJ is 32
+// up to 32 states, else 64 (row tiles of 64 beyond).  A tile's load, product
+// and epilogue follow one another, so it takes several small blocks per SM to
+// keep the FP64 tensor pipe busy through the others' epilogues.  Measured
+// against 128-row tiles of eight warps, two per SM: 32 states, 8276
+// coefficients, rotation with velocity and planes 15.8 -> 8.5 us (six of eight
+// warps had no rows); 56 states 40 -> 23; 128 states, 40115 coefficients 171 -> 130,
+// plain 95 -> 75 (mean of the two products of a step), two-term 198 -> 184; 512
+// states 4.72 -> 4.41 ms.  The M and X slabs of 16 k rows move through a cp.async
+// ring; the two terms run as one slab sequence.  The first term's sum is
+// scaled by a1(c) in registers once it is complete; the second term's M
+// fragments are scaled by a2 as they are read, so one accumulator set serves
+// both terms.
 // ---------------------------------------------------------------------------
-#define DB_TJ 128
 #define DB_TC 64
 #define DB_KS 16
-#define DB_LDM (DB_TJ + 4)
 #define DB_LDX (DB_TC + 4)
-#define DB_STAGES 4
-#define DB_THREADS 256
-#define DB_MSLAB (DB_KS * DB_LDM)
-#define DB_XSLAB (DB_KS * DB_LDX)
+template <int TJ> struct DbTile {
+  static constexpr int THREADS = TJ * 2;
+  static constexpr int BLOCKS = 256 / TJ;  // resident per SM
+  static constexpr int STAGES = 3;
+  static constexpr int LDM = TJ + 4;
+  static constexpr int MSLAB = DB_KS * LDM, XSLAB = DB_KS * DB_LDX;
+  static constexpr size_t SMEM = (size_t)STAGES * (MSLAB + XSLAB) * sizeof(double);
+};
 
+template <int TJ>
 __device__ __forceinline__ void db_load_slab(double* ms, double* xs, const double* __restrict__ M,
                                              const double* __restrict__ X, int nj, int nk, long ncol, int k0,
                                              long c0, int j0) {
+  typedef DbTile<TJ> D;
   if (nj & 1) {
     // odd nj: the rows of M are not 16-byte aligned; 8-byte pieces, 8 per thread
 #pragma unroll
-    for (int q = 0; q < (DB_KS * DB_TJ) / DB_THREADS; ++q) {
-      const int piece = threadIdx.x + q * DB_THREADS;
-      const int kk = piece >> 7, jj = piece & 127;
+    for (int q = 0; q < (DB_KS * TJ) / D::THREADS; ++q) {
+      const int piece = threadIdx.x + q * D::THREADS;
+      const int kk = piece / TJ, jj = piece % TJ;
       const int k = k0 + kk;
       const bool valid = (k < nk) && (j0 + jj < nj);
-      dg_cp8(ms + kk * DB_LDM + jj, valid ? M + (size_t)k * nj + j0 + jj : M, valid);
+      dg_cp8(ms + kk * D::LDM + jj, valid ? M + (size_t)k * nj + j0 + jj : M, valid);
     }
   } else {
-    // M rows k0..k0+15, all 128 j: 16 x 64 pieces of 16 B = 1024 -> 4 per thread
+    // M rows k0..k0+15, all TJ j: pieces of 16 B, 4 per thread
 #pragma unroll
-    for (int q = 0; q < (DB_KS * DB_TJ / 2) / DB_THREADS; ++q) {
-      const int piece = threadIdx.x + q * DB_THREADS;
-      const int kk = piece >> 6, jj = (piece & 63) * 2;
+    for (int q = 0; q < (DB_KS * TJ / 2) / D::THREADS; ++q) {
+      const int piece = threadIdx.x + q * D::THREADS;
+      const int kk = piece / (TJ / 2), jj = piece % (TJ / 2) * 2;
       const int k = k0 + kk;
       const bool valid = (k < nk) && (j0 + jj < nj);
-      dg_cp16(ms + kk * DB_LDM + jj, valid ? M + (size_t)k * nj + j0 + jj : M, valid);
+      dg_cp16(ms + kk * D::LDM + jj, valid ? M + (size_t)k * nj + j0 + jj : M, valid);
     }
   }
-  // X rows k0..k0+15, columns c0..c0+63: 16 x 32 pieces = 512 -> 2 per thread
+  // X rows k0..k0+15, columns c0..c0+63: 16 x 32 pieces
 #pragma unroll
-  for (int q = 0; q < (DB_KS * DB_TC / 2) / DB_THREADS; ++q) {
-    const int piece = threadIdx.x + q * DB_THREADS;
+  for (int q = 0; q < (DB_KS * DB_TC / 2) / D::THREADS; ++q) {
+    const int piece = threadIdx.x + q * D::THREADS;
     const int kk = piece >> 5, cc = (piece & 31) * 2;
     const int k = k0 + kk;
     const long c = c0 + cc;
@@ -376,9 +388,9 @@ __device__ __forceinline__ void db_load_slab(double* ms, double* xs, const doubl
 // *cond2 != 0; vel (optional, when *vcond != 0) receives the finite
 // difference (result - previous out) vscale, previous out read by the
 // thread that overwrites it.
-// EDGE: the last row tile has idle 32-row blocks (nj not a multiple of 128)
-template <bool TWO, bool EDGE>
-__global__ void __launch_bounds__(DB_THREADS, 2)
+// EDGE: the lower 32 rows of the last row tile hold no state
+template <int TJ, bool TWO, bool EDGE>
+__global__ void __launch_bounds__(DbTile<TJ>::THREADS, DbTile<TJ>::BLOCKS)
 k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double a1_kx0, double a1_rest,
             const double* __restrict__ M2, const double* __restrict__ X2, double a2, int nj, int nk, long ncol,
             long kx0_cols, double* out, const int* __restrict__ cond, const double* yadd, double* __restrict__ out2,
@@ -387,16 +399,17 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
   if (cond && *cond == 0) return;
   const bool dual = out2 && *cond2 != 0;
   const bool velo = vel && *vcond != 0;
+  typedef DbTile<TJ> D;
   extern __shared__ __align__(16) double db_smem[];
   double* Ms = db_smem;
-  double* Xs = db_smem + DB_STAGES * DB_MSLAB;
+  double* Xs = db_smem + D::STAGES * D::MSLAB;
   const long c0 = (long)blockIdx.x * DB_TC;
-  const int j0 = blockIdx.y * DB_TJ;  // rows j0 .. j0 + 127 of the output
+  const int j0 = blockIdx.y * TJ;  // first row of the output tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the row block of a warp pair rotates with the block: the idle blocks of
-  // an edge tile then fall on different SM sub-partitions in the two
-  // resident blocks
-  const int wj = (((warp >> 1) + (EDGE ? (blockIdx.x & 1) : 0)) & 3) * 32, wc = (warp & 1) * 32;
+  // an edge tile then fall on different SM sub-partitions in neighbouring
+  // blocks
+  const int wj = (((warp >> 1) + (EDGE ? (blockIdx.x & 1) : 0)) & (TJ / 32 - 1)) * 32, wc = (warp & 1) * 32;
   const bool live = !EDGE || j0 + wj < nj;
   const int nsl = (nk + DB_KS - 1) / DB_KS;
   const int ntot = TWO ? 2 * nsl : nsl;
@@ -406,10 +419,10 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
 #pragma unroll
     for (int b = 0; b < 4; ++b) { acc[a][b][0] = 0.0; acc[a][b][1] = 0.0; }
   auto issue = [&](int s) {
-    const int st = s % DB_STAGES;
+    const int st = s % D::STAGES;
     const bool second = TWO && s >= nsl;
     const int k0 = (second ? s - nsl : s) * DB_KS;
-    db_load_slab(Ms + st * DB_MSLAB, Xs + st * DB_XSLAB, second ? M2 : M1, second ? X2 : X1, nj, nk, ncol, k0, c0,
+    db_load_slab<TJ>(Ms + st * D::MSLAB, Xs + st * D::XSLAB, second ? M2 : M1, second ? X2 : X1, nj, nk, ncol, k0, c0,
                  j0);
   };
   // a1(c) for this thread's output columns
@@ -425,26 +438,26 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
       }
   };
 #pragma unroll
-  for (int s = 0; s < DB_STAGES - 1; ++s) {
+  for (int s = 0; s < D::STAGES - 1; ++s) {
     if (s < ntot) issue(s);
     dg_commit();
   }
   for (int s = 0; s < ntot; ++s) {
-    dg_wait<DB_STAGES - 2>();
+    dg_wait<D::STAGES - 2>();
     __syncthreads();
-    if (s + DB_STAGES - 1 < ntot) issue(s + DB_STAGES - 1);
+    if (s + D::STAGES - 1 < ntot) issue(s + D::STAGES - 1);
     dg_commit();
     if (TWO && s == nsl) scale_a1();
     const double sa = (TWO && s >= nsl) ? a2 : 1.0;
-    const double* ms = Ms + (s % DB_STAGES) * DB_MSLAB;
-    const double* xs = Xs + (s % DB_STAGES) * DB_XSLAB;
+    const double* ms = Ms + (s % D::STAGES) * D::MSLAB;
+    const double* xs = Xs + (s % D::STAGES) * D::XSLAB;
     if (live)
 #pragma unroll
     for (int k4 = 0; k4 < DB_KS; k4 += 4) {
       double af[4], bf[4];
       // A[j][k] = M[k][j] (row-major 8 x 4 fragment), B[k][c] = X[k][c]
 #pragma unroll
-      for (int q = 0; q < 4; ++q) af[q] = ms[(k4 + (lane & 3)) * DB_LDM + wj + q * 8 + (lane >> 2)] * sa;
+      for (int q = 0; q < 4; ++q) af[q] = ms[(k4 + (lane & 3)) * D::LDM + wj + q * 8 + (lane >> 2)] * sa;
 #pragma unroll
       for (int q = 0; q < 4; ++q) bf[q] = xs[(k4 + (lane & 3)) * DB_LDX + wc + q * 8 + (lane >> 2)];
 #pragma unroll
@@ -455,29 +468,42 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
   }
   dg_wait<0>();
   if (!TWO) scale_a1();
+  // the old out or yadd (which may be out) of eight pieces is read before any
+  // of them is written: read one at a time behind the writes they were a
+  // chain of sixteen L2 round trips, 8 of 13 us at 32 states
+  const double* pre = velo ? out : yadd;
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int j = j0 + wj + a * 8 + (lane >> 2);
-    if (j >= nj) continue;
+  for (int a2 = 0; a2 < 4; a2 += 2) {
+    double2 p[2][4];
+    if (pre) {
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const long c = c0 + wc + b * 8 + 2 * (lane & 3);
-      const size_t o = (size_t)j * ncol + c;
-      if (c + 1 < ncol) {
-        double2 v = make_double2(acc[a][b][0], acc[a][b][1]);
-        if (yadd) { const double2 y = *(const double2*)(yadd + o); v.x += y.x; v.y += y.y; }
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int j = j0 + wj + (a2 + a) * 8 + (lane >> 2);
+          const long c = c0 + wc + b * 8 + 2 * (lane & 3);
+          p[a][b] = make_double2(0.0, 0.0);
+          if (j < nj && c < ncol) p[a][b] = *(const double2*)(pre + (size_t)j * ncol + c);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const int j = j0 + wj + (a2 + a) * 8 + (lane >> 2);
+      if (j >= nj) continue;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const long c = c0 + wc + b * 8 + 2 * (lane & 3);  // even, as ncol is
+        const size_t o = (size_t)j * ncol + c;
+        if (c >= ncol) continue;
+        double2 v = make_double2(acc[a2 + a][b][0], acc[a2 + a][b][1]);
         if (velo) {
-          const double2 p = *(const double2*)(out + o);
-          *(double2*)(vel + o) = make_double2(fma(v.x, vscale, p.x * -vscale), fma(v.y, vscale, p.y * -vscale));
+          *(double2*)(vel + o) = make_double2(fma(v.x, vscale, p[a][b].x * -vscale), fma(v.y, vscale, p[a][b].y * -vscale));
+        } else if (pre) {
+          v.x += p[a][b].x;
+          v.y += p[a][b].y;
         }
         *(double2*)(out + o) = v;
         if (dual) *(double2*)(out2 + o) = v;
-      } else if (c < ncol) {
-        double v = acc[a][b][0];
-        if (yadd) v += yadd[o];
-        if (velo) vel[o] = fma(v, vscale, out[o] * -vscale);
-        out[o] = v;
-        if (dual) out2[o] = v;
       }
     }
   }
@@ -493,35 +519,31 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
         const int cl = wc + b * 8 + 2 * (lane & 3);
-        __nv_bfloat16 hx[3], hy[3];
-        oa_bf16_digits(acc[a][b][0], po.nt, hx);
-        oa_bf16_digits(acc[a][b][1], po.nt, hy);
+        __nv_bfloat162 h[3];
+        oa_bf16_digits2(acc[a][b][0], acc[a][b][1], po.nt, h);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
           if (q >= po.nt) break;
-          __nv_bfloat162 v2;
-          v2.x = hx[q];
-          v2.y = hy[q];
-          *reinterpret_cast<__nv_bfloat162*>(sp + ((size_t)q * DB_TJ + jl) * SPLD + cl) = v2;
+          *reinterpret_cast<__nv_bfloat162*>(sp + ((size_t)q * TJ + jl) * SPLD + cl) = h[q];
         }
       }
     }
-    __syncthreads();
+  __syncthreads();
     const size_t pstride = (size_t)po.rows_pad * po.ldp;
-    for (int i = threadIdx.x; i < po.nt * DB_TJ * (DB_TC / 8); i += DB_THREADS) {
-      const int q = i / (DB_TJ * (DB_TC / 8)), rem = i - q * (DB_TJ * (DB_TC / 8));
+    for (int i = threadIdx.x; i < po.nt * TJ * (DB_TC / 8); i += D::THREADS) {
+      const int q = i / (TJ * (DB_TC / 8)), rem = i - q * (TJ * (DB_TC / 8));
       const int jl = rem / (DB_TC / 8), ch = rem - jl * (DB_TC / 8);
       if (j0 + jl >= nj || c0 + ch * 8 >= po.ldp) continue;
       *reinterpret_cast<uint4*>((__nv_bfloat16*)po.P + q * pstride +
                                 oa_plane_at(j0 + jl, c0 + ch * 8, po.rows_pad)) =
-          *reinterpret_cast<const uint4*>(sp + ((size_t)q * DB_TJ + jl) * SPLD + ch * 8);
+          *reinterpret_cast<const uint4*>(sp + ((size_t)q * TJ + jl) * SPLD + ch * 8);
     }
   }
 }
 
 // Returns cudaErrorNotSupported when the shapes or pointers do not allow the
 // copies (odd ncol, unaligned pointers); an odd nj moves M in 8-byte pieces.
-// Outputs of more than 128 rows run as row tiles of 128 (grid y).
+// Outputs of more than 64 rows run as row tiles of 64 (grid y).
 // po (optional): bf16 planes of out written in the same pass (ncol even).
 cudaError_t oa_dgemm_bwd_ex(cudaStream_t s, const double* M1, const double* X1, double a1_kx0, double a1_rest,
                             const double* M2, const double* X2, double a2, int nj, int nk, long ncol, long kx0_cols,
@@ -535,18 +557,22 @@ cudaError_t oa_dgemm_bwd_ex(cudaStream_t s, const double* M1, const double* X1, 
                        (uintptr_t)(X2 ? X2 : X1) | (uintptr_t)yadd | (uintptr_t)out2 | (uintptr_t)vel;
   if (out2 && !cond2) return cudaErrorInvalidValue;
   if (nj <= 0 || (ncol & 1) || (al & 15) || nk <= 0 || (M2 && !X2)) return cudaErrorNotSupported;
-  const size_t sm = (size_t)DB_STAGES * (DB_MSLAB + DB_XSLAB) * sizeof(double);
-  // column tiles of 64 by row tiles of 128
-  dim3 grid((unsigned)((ncol + DB_TC - 1) / DB_TC), (unsigned)((nj + DB_TJ - 1) / DB_TJ));
-  auto go = [&](auto kern) -> cudaError_t {
+  // column tiles of 64 by row tiles of tj
+  auto go = [&](auto kern, int tj, int threads, size_t sm) -> cudaError_t {
     const cudaError_t e = oa_smem_limit(kern);
     if (e != cudaSuccess) return e;
-    kern<<<grid, DB_THREADS, sm, s>>>(M1, X1, a1_kx0, a1_rest, M2, X2, a2, nj, nk, ncol, kx0_cols, out, cond, yadd,
-                                      out2, cond2, pz, vel, vscale, vcond);
+    dim3 grid((unsigned)((ncol + DB_TC - 1) / DB_TC), (unsigned)((nj + tj - 1) / tj));
+    kern<<<grid, threads, sm, s>>>(M1, X1, a1_kx0, a1_rest, M2, X2, a2, nj, nk, ncol, kx0_cols, out, cond, yadd, out2,
+                                   cond2, pz, vel, vscale, vcond);
     return cudaGetLastError();
   };
-  if (nj % DB_TJ == 0) return M2 ? go(k_dgemm_bwd<true, false>) : go(k_dgemm_bwd<false, false>);
-  return M2 ? go(k_dgemm_bwd<true, true>) : go(k_dgemm_bwd<false, true>);
+#define OA_DB(TJ, EDGE)                                                                             \
+  return M2 ? go(k_dgemm_bwd<TJ, true, EDGE>, TJ, DbTile<TJ>::THREADS, DbTile<TJ>::SMEM)            \
+            : go(k_dgemm_bwd<TJ, false, EDGE>, TJ, DbTile<TJ>::THREADS, DbTile<TJ>::SMEM)
+  if (nj <= 32) OA_DB(32, false);
+  if (nj % 64 >= 1 && nj % 64 <= 32) OA_DB(64, true);
+  OA_DB(64, false);
+#undef OA_DB
 }
 
 cudaError_t oa_dgemm_bwd(cudaStream_t s, const double* M1, const double* X1, double a1_kx0, double a1_rest,

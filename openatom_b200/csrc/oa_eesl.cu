@@ -2,7 +2,7 @@
 // on one GPU: the B-spline grids of the atom types, their 3-D transform,
 // and the atom forces from the back-transformed force grids.  The g-space
 // part (energies, V_KS and the force transforms) runs inside the density z
-// pass (k_rho_zpass with EesLocArgs, oa_rho.cu).
+// pass (k_rho_zpass with EesLocArgs, oa_rho_zpass.cuh).
 //
 // Replaces:
 //   CPLOCAL::eesAtmBsplineRgrp + eesPackGridRchare (cp_hart_ext.C:641-990)  -> k_eesl_spread

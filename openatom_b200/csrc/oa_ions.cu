@@ -12,7 +12,7 @@
 //     ATOMINTEGRATE::integrate_nve_2nd_half / integrate_nve_1st_half
 //     (classical_physics/integrate/integration_drivers.C:17-85)             -> k_ion_integrate
 // The local pseudopotential and reciprocal Ewald forces come from the
-// density z pass (k_rho_zpass<..., true>, oa_rho.cu), one partial per z-pass
+// density z pass (k_rho_zpass<..., true>, oa_rho_zpass.cuh), one partial per z-pass
 // block, or with the EES local path from k_eesl_force (oa_eesl.cu) in the
 // first partial.
 #include <stdlib.h>
@@ -41,8 +41,10 @@ static __device__ void ion_block_sum3(double v[3], double* sh) {
 
 // F_a = -2 vnorm_a / V sum_g g (Y.x SF.y - Y.y SF.x), Y = sum_s Z[s][a] psi_s:
 // dZ/dR_a of SF_a(g) = w p y00 conj(e^{i g.R_a}) is -i g SF_a.  One block per
-// nonlocal atom; writes that atom's row of fnl (the others stay zero).
-__global__ void k_nl_sf_force(const double2* __restrict__ y, const double2* __restrict__ sf, int ng,
+// nonlocal atom; writes that atom's row of fnl (the others stay zero).  The
+// chain of loads of a thread bounds it: 1024 threads, four points in flight
+// (256 threads, one point: 54 us at 16 atoms and 16000 g-points).
+__global__ void __launch_bounds__(1024) k_nl_sf_force(const double2* __restrict__ y, const double2* __restrict__ sf, int ng,
                               const int* __restrict__ kx, const int* __restrict__ ky, const int* __restrict__ kz,
                               double tpi_l, const int* __restrict__ nl_atm, const int* __restrict__ atm_type,
                               const double* __restrict__ vnorm, double rvol, double* __restrict__ fnl) {
@@ -51,6 +53,7 @@ __global__ void k_nl_sf_force(const double2* __restrict__ y, const double2* __re
   const double2* ya = y + (size_t)a * ng;
   const double2* sa = sf + (size_t)a * ng;
   double f[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
   for (int i = threadIdx.x; i < ng; i += blockDim.x) {
     const double2 yy = ya[i], ss = sa[i];
     const double c = yy.x * ss.y - yy.y * ss.x;
@@ -219,7 +222,7 @@ cudaError_t oa_launch_nl_sf_force(oa_ctx* c, cudaStream_t s, const double* psi) 
   const long K = 2L * c->ng;
   e = oa_launch_pc_bwd_jk(s, c->zmat, psi, 1.0, 1.0, nullptr, nullptr, 0.0, c->natm_nl, c->nstate, K, 0, io->y);
   if (e != cudaSuccess) return e;
-  k_nl_sf_force<<<c->natm_nl, 256, 0, s>>>((const double2*)io->y, c->sf, c->ng, c->kx, c->ky, c->kz,
+  k_nl_sf_force<<<c->natm_nl, 1024, 0, s>>>((const double2*)io->y, c->sf, c->ng, c->kx, c->ky, c->kz,
                                            2.0 * 3.14159265358979323846 / c->box, c->nl_atm, c->atm_type,
                                            c->nl_vnorm, 1.0 / c->vol, io->fnl);
   return cudaGetLastError();

@@ -238,9 +238,9 @@ k_ortho_ns_cluster(const double* __restrict__ S, int n, double bscale, double to
 // new A, B in shared memory.  The products are short (32 states: 16 tiles of
 // 8 DMMAs), so what a cluster iteration costs is its two cluster barriers and
 // the L2 round trips between them; one block replaces them by block barriers.
-// Measured per call at 32 states (5 iterations): cluster 33 us, one block
-// 9 us; the products take over between 48 and 64 states, where one SM's FP64
-// tensor rate (2 us a product at 64) loses to sixteen SMs.
+// Measured per call at 32 states in a step: cluster 33 us, one block 14 us.  At
+// 64 states the products alone, on one SM's FP64 tensor pipe (2 us each), cost
+// what the cluster takes (35 us).
 // ---------------------------------------------------------------------------
 #define NSS_MAXN 48
 

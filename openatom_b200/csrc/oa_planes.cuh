@@ -19,14 +19,35 @@ __host__ __device__ __forceinline__ size_t oa_plane_at(int r, long c, int rows_p
   return ((size_t)(c >> 6) * rows_pad + r) * 64 + (size_t)(c & 63);
 }
 
-// the nt bf16 digits of v (nt <= 3)
+// the nt bf16 digits of v (nt <= 3): v is split into two FP32 parts first and
+// the digits are taken in FP32 (conversions from and to FP64 run at a quarter
+// of the FP32 rate), where the sum of the remainder and the low part rounds
+// 2^-33 below v, far under the last digit
 __device__ __forceinline__ void oa_bf16_digits(double v, int nt, __nv_bfloat16* h) {
+  float r = (float)v;
+  const float lo = (float)(v - (double)r);
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     if (q >= nt) break;
-    const __nv_bfloat16 b = __float2bfloat16_rn((float)v);
+    const __nv_bfloat16 b = __float2bfloat16_rn(r);
     h[q] = b;
-    v -= (double)__bfloat162float(b);
+    r -= __bfloat162float(b);
+    if (q == 0) r += lo;
+  }
+}
+
+// the digits of a pair, one conversion instruction for both
+__device__ __forceinline__ void oa_bf16_digits2(double x, double y, int nt, __nv_bfloat162* h) {
+  float rx = (float)x, ry = (float)y;
+  const float lx = (float)(x - (double)rx), ly = (float)(y - (double)ry);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    if (q >= nt) break;
+    const __nv_bfloat162 b = __floats2bfloat162_rn(rx, ry);
+    h[q] = b;
+    rx -= __low2float(b);
+    ry -= __high2float(b);
+    if (q == 0) { rx += lx; ry += ly; }
   }
 }
 
@@ -45,17 +66,15 @@ __device__ __forceinline__ void oa_plane_put(const OaPlaneOut& po, int r, long c
 
 // planes of the pair (x, y) at row r, columns c and c + 1 (c even)
 __device__ __forceinline__ void oa_plane_put2(const OaPlaneOut& po, int r, long c, double x, double y) {
-  __nv_bfloat16 hx[3], hy[3];
-  oa_bf16_digits(x, po.nt, hx);
-  oa_bf16_digits(y, po.nt, hy);
-  __nv_bfloat16* base = (__nv_bfloat16*)po.P + oa_plane_at(r, c, po.rows_pad);
+  __nv_bfloat162 h[3];
+  oa_bf16_digits2(x, y, po.nt, h);
+  const unsigned cu = (unsigned)c;  // a row has fewer than 2^32 columns
+  __nv_bfloat16* base =
+      (__nv_bfloat16*)po.P + ((size_t)(cu >> 6) * (unsigned)po.rows_pad + (unsigned)r) * 64 + (cu & 63u);
   const size_t pstride = (size_t)po.rows_pad * po.ldp;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     if (q >= po.nt) break;
-    __nv_bfloat162 v;
-    v.x = hx[q];
-    v.y = hy[q];
-    *reinterpret_cast<__nv_bfloat162*>(base + q * pstride) = v;
+    *reinterpret_cast<__nv_bfloat162*>(base + q * pstride) = h[q];
   }
 }

@@ -28,6 +28,13 @@
 // psi(r) is private to the two kernels: [pair][z][k2][row position][k1], the
 // order in which pass B holds it, so that stores and loads are contiguous.
 //
+// What bounds them: the shared-memory round trips and the instructions of the
+// register DFTs (DRAM traffic is psi(r) and the z-lines once).  Measured,
+// density / V_KS: 108^3, 128 states, FP32 287 / 286 us (one pair per block
+// iteration with block barriers between the passes: 305 / 331), FP64 554 / 542 us
+// (per-state planes: 1093 / 963); 120^3, 256 states, FP64 1.73 / 1.43 ms
+// (runtime-plan planes: 15.8 together); 80^3, 78 states, FP32 50 / 56 us.
+//
 // Shared-memory strides are chosen per length by enumeration over the access
 // patterns above (bank conflicts of 8- or 16-byte elements); the table is in
 // oa_pp_table.h.

@@ -232,8 +232,8 @@ k_rho2_bwd(const double2* __restrict__ dz, int ldl_d, const double2* __restrict_
 //             k_rho3_y<-1> (columns of dz in place)
 //   backward: k_rho3_y<+1>, k_rho3_x_bwd
 // Against the runtime-plan kernels (one block per plane, one stage of
-// radix <= 5 per shared-memory pass) at 160^3: forward 378 -> 90 us, backward
-// 465 -> 98 us.
+// radix <= 5 per shared-memory pass) at 120^3: forward 57 -> 18 us, backward
+// 65 -> 21 us.  At 160^3 the x kernels take 21 (forward) and 46 us (backward).
 // ---------------------------------------------------------------------------
 template <int N1, int N2> struct Rho3Cfg {
   static constexpr int N = N1 * N2, NKX = N / 2 + 1, NPAIR = (N + 1) / 2;

@@ -1,4 +1,4 @@
-// z pass of the density path (see oa_rho.cu): FFT(-) -> Hartree + local
+// z pass of the density path (oa_rho.cu launches it): FFT(-) -> Hartree + local
 // pseudopotential + Ewald (recip) in G -> FFT(+), LB z-lines per block.
 //
 // The structure factors S_t(g) = sum_{a in t} e^{i g.R_a} factorise per
@@ -8,8 +8,10 @@
 // [atom][kz].  Of the complex product the four real ones Re w Re z, Im w Im z,
 // Re w Im z, Im w Re z run on the FP64 tensor cores (8 lines x 8 kz tiles),
 // and their sums and differences give S at kz and at -kz.  A thread per point
-// was bound by the latency of its z-phase loads (two points per load): 82 us
-// at 108^3 with 96 atoms, 1050 us at 160^3 with 384.
+// was bound by the latency of its z-phase loads (two points per load).
+// Measured before -> now: 108^3 with 96 atoms 82 -> 58 us, 120^3 with 192 atoms
+// 196 (runtime transforms) -> 78 us, 160^3 with 384 atoms 1050 -> 611 us beside the
+// nonlocal branch, 64^3 with 24 atoms 17 -> 11 us.
 #pragma once
 #include "oa_rho_common.cuh"
 #include "oa_rdft.cuh"

@@ -1,7 +1,7 @@
 """Sizes off the presets: every kind of two-pass grid length (even and odd,
 with and without the band-pruned first DFT, the row-split FP64 density pass),
-odd state counts, state counts of several product tiles, and the one-block
-Newton-Schulz iteration, against the oracle."""
+odd state counts, state counts at the edges of the product tiles and of
+several tiles, and the three Newton-Schulz forms, against the oracle."""
 import math
 
 import numpy as np
@@ -87,7 +87,7 @@ def test_ees_pairs(n, nstate, order, scale, precision, tol):
     assert rel(f.cpu().numpy(), fr) < tol
 
 
-@pytest.mark.parametrize("nstate", [129, 150, 199, 256, 300])
+@pytest.mark.parametrize("nstate", [5, 31, 33, 64, 65, 100, 129, 150, 199, 256, 300])
 def test_products_of_several_tiles(nstate):
     """S (symmetric tiles), Lambda, the two-term backward product and the
     rotation: FP64 to rounding; split-BF16 to the rounding of FP32 sums of six
@@ -120,7 +120,7 @@ def test_products_of_several_tiles(nstate):
         assert rel(rot.cpu().numpy(), T.T @ s.psi) < 1e-12
 
 
-@pytest.mark.parametrize("nstate", [1, 2, 7, 8, 31, 32, 48, 50, 51])
+@pytest.mark.parametrize("nstate", [1, 2, 7, 8, 31, 32, 48, 50, 51, 130, 161, 199, 288])
 def test_newton_schulz_sizes(nstate):
     import torch
     from openatom_b200.gpu import CPContext
