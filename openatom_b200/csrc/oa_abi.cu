@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <vector>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include "oa_internal.h"
 
@@ -86,6 +87,24 @@ extern "C" const char* oa_gpu_last_error(void) { return g_err; }
     if (!(cond)) { oa_set_error(msg, __FILE__, __LINE__); return OA_ERR_BAD_ARG; } \
   } while (0)
 
+// unique id of the device's current CUDA context (0: unknown): it changes
+// when the device has been reset
+static unsigned long long context_id() {
+  typedef CUresult (*GetId)(CUcontext, unsigned long long*);
+  static const GetId get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    cudaGetLastError();
+    return (GetId)f;
+  }();
+  unsigned long long id = 0;
+  cudaFree(nullptr);  // makes the context current
+  return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 // open-addressing set of (kernel, device); a full probe sequence just means
 // that the limit is set again at that launch
 static std::atomic<uintptr_t> g_smem_set[1024];
@@ -109,6 +128,20 @@ void oa_smem_mark(const void* kernel) {
     uintptr_t v = 0;
     if (g_smem_set[(h + i) & 1023].compare_exchange_strong(v, k, std::memory_order_acq_rel) || v == k) return;
   }
+}
+
+// the raised limits end with a device's context: forget them when it is a new
+// one (or when that cannot be told)
+static void forget_stale_smem_limits() {
+  static std::atomic<unsigned long long> last[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long id = context_id();
+  if (id != 0 && dev < 64) {
+    const unsigned long long was = last[dev].exchange(id, std::memory_order_acq_rel);
+    if (was == id || was == 0) return;  // unchanged, or nothing raised on this device yet
+  }
+  for (auto& v : g_smem_set) v.store(0, std::memory_order_release);
 }
 
 // FP64-accurate int8 tensor-core products of the mixed form (oa_ozaki.cu)
@@ -272,7 +305,7 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
   OA_ARG_CHECK(d->natm == 0 || d->atm_type, "null atm_type");
   for (int a = 0; a < d->natm; ++a) OA_ARG_CHECK(d->atm_type[a] >= 0 && d->atm_type[a] < d->ntype, "atom type out of range");
   *out = nullptr;
-  for (auto& v : g_smem_set) v.store(0, std::memory_order_release);
+  forget_stale_smem_limits();
   oa_ctx_full* F = (oa_ctx_full*)calloc(1, sizeof(oa_ctx_full));
   if (!F) return OA_ERR_CUDA;
   oa_ctx* c = &F->c;

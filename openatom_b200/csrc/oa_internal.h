@@ -12,9 +12,8 @@
 #define OA_MAX_SMEM (227 * 1024)
 
 // Kernels whose dynamic shared-memory limit has been raised on the current
-// device (oa_abi.cu).  The limit lasts as long as the device's context: every
-// oa_gpu_init forgets the set, so that contexts made after a device reset
-// raise it again.
+// device (oa_abi.cu).  The limit lasts as long as the device's context: an
+// oa_gpu_init that finds a new context (after a device reset) forgets the set.
 bool oa_smem_raised(const void* kernel);
 void oa_smem_mark(const void* kernel);
 
