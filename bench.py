@@ -698,7 +698,7 @@ def run_ours(args):
 # the plane kernels on the 32-water workload, copied from one ncu capture of
 # the same kernels (the run itself cannot read DRAM counters); None for other
 # workloads.
-TRAFFIC_W32 = {"state_plane_density": 755.4e6, "state_plane_vks": 748.0e6}
+TRAFFIC_W32 = {"state_plane_density": 793.6e6, "state_plane_vks": 744.7e6}
 
 
 def roofline(sysm, drv, kt, config=None):

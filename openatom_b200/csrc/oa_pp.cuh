@@ -1,5 +1,6 @@
 // State-pair plane kernels of the state FFT path, for every grid length with
-// a two-pass factorisation N = N1 N2 (oa_rdft.cuh) and both precision forms:
+// a two-pass factorisation N = N1 N2 (oa_rdft.cuh) and both precision forms
+// (FP64 without 125, 150 and 160, whose planes do not fit):
 //   k_pp_density  z-line rows -> psi(r) of two states -> density sum, psi(r) stored
 //   k_pp_vks      stored psi(r) V_KS -> z-line rows
 //
