@@ -341,6 +341,7 @@ k_rho_zpass(double2* __restrict__ dz, int ldl_d, int nlines_d, int nx, int ny, i
         o[0] = fx; o[1] = fy; o[2] = fz;
       }
     }
+    __syncthreads();  // cf0 is the buffer that the inverse transform writes first
   }
   double2* r2;
   if constexpr (TP) {

@@ -118,6 +118,36 @@ def test_ion_dynamics_ees_nonlocal_fp64(preset, nstate, order):
     d.ctx.close()
 
 
+# z lengths whose inverse transform is written by every warp of a z-pass block
+# from its first pass on (125 = 5 x 25, and the runtime plan at 162), and one
+# whose first pass takes the low warps only
+@pytest.mark.parametrize("nz,types", [(125, (19, 2)), (162, (19, 2)), (64, (19, 2)), (125, (21, 0)), (162, (3, 18))])
+def test_local_forces_of_uneven_atoms(nz, types):
+    """Atom forces with most atoms of one type and a count that is no
+    multiple of a block's warps: the first half kick against the oracle, and
+    the same bits from run to run."""
+    import dataclasses
+    from openatom_b200.gpu import CPDriver
+    s = make_system("w8", seed=47, nstate=3, nfft=(40, 40, nz), ecut_ry=20.0, dt=5.0)
+    n = sum(types)
+    typ = np.repeat([0, 1], types)
+    s = dataclasses.replace(s, pos=s.pos[:n].copy(), atm_type=typ, q=np.where(typ == 0, 6.0, 1.0))
+    m = O.atom_masses(s)
+    runs = []
+    for _ in range(4):
+        d = CPDriver(s, "fp64")
+        d.ctx.set_ions(m)
+        d.run_native(d.native_state(), 1)
+        runs.append(d.ctx.get_ions()[1])
+        d.ctx.close()
+    for v in runs[1:]:
+        assert np.array_equal(v, runs[0])
+    so = copy.deepcopy(s)
+    ions = O.IonState(so)
+    O.cp_step(O.CPState(so), so, norb_tol=0.003, ions=ions)
+    assert np.max(np.abs(runs[0] - ions.v)) <= 1e-10 * np.max(np.abs(ions.v))
+
+
 def test_ion_dynamics_refuses_host_positions():
     from openatom_b200.gpu import CPDriver, OaError
     s, m, vel = _start("w2", None, 44)
