@@ -201,8 +201,9 @@ oa_status oa_gpu_check(oa_ctx *ctx, void *stream);
 /* Failure-detection test hook, no counterpart in the reference (its
  * failures end in CkAbort / EXIT).  kind 1: the next split-BF16 forward
  * product skips the loads of one pipeline stage in one block, so that
- * block's bounded wait runs out and oa_gpu_check reports it; kind 0 clears
- * the hook.  Acts on the current device. */
+ * block's bounded wait runs out and oa_gpu_check reports it (acts on the
+ * current device); kind 2: the next graph capture of this context's native
+ * step is reported as failed on the host; kind 0 clears the hooks. */
 oa_status oa_gpu_fault_inject(oa_ctx *ctx, int kind);
 
 /* Small dense C = alpha A B (N x N), e.g. Gamma = T Lambda (ortho.C:565-570). */

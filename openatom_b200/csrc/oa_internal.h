@@ -177,6 +177,7 @@ struct oa_ctx {
   oa_eesl *eesl;          // EES local path, after oa_gpu_set_ees_local
   int eesl_gen;           // bumped by every oa_gpu_set_ees_local (captured graphs depend on it)
   int fft_runtime;        // oa_tuning fft_path 2: runtime-plan transforms for the state path
+  int fail_capture;       // oa_gpu_fault_inject 2: the next capture of a native step is reported as failed
   int phase_done;         // inside a native step: the phase tables are this step's
   int rho_groups_cap;     // groups the density partials are allocated for
   int nq2_cap;            // entries of qpart2 allocated
@@ -215,10 +216,24 @@ cudaError_t oa_launch_phase_tables(oa_ctx* c, cudaStream_t s);
 #define OA_CUDA_TRY(x)                                  \
   do {                                                  \
     cudaError_t e_ = (x);                               \
-    if (e_ != cudaSuccess) { oa_set_error(cudaGetErrorString(e_), __FILE__, __LINE__); return OA_ERR_CUDA; } \
+    if (e_ != cudaSuccess) {                            \
+      oa_set_error(cudaGetErrorString(e_), __FILE__, __LINE__); \
+      cudaGetLastError(); /* reported here: not the next launch's error */ \
+      return OA_ERR_CUDA;                               \
+    }                                                   \
   } while (0)
 
 void oa_set_error(const char* msg, const char* file, int line);
+
+void oa_planes_step_begin(oa_ctx* c);
+void oa_planes_step_end(oa_ctx* c);
+// A native step's launches (or their capture): the plane reuse and the sums
+// at the end of the step are on for its life only, however it ends.
+struct StepScope {
+  oa_ctx* c;
+  explicit StepScope(oa_ctx* ctx) : c(ctx) { oa_planes_step_begin(c); }
+  ~StepScope() { oa_planes_step_end(c); }
+};
 
 // stage launchers (return cudaError_t)
 cudaError_t oa_launch_state_zfwd(oa_ctx* c, cudaStream_t s, const double2* psi, int s0, int ns);

@@ -148,11 +148,20 @@ void oa_step_free(oa_ctx* c) {
 
 #define OA_STEP_TRY(x) do { oa_status st_ = (x); if (st_ != OA_OK) return st_; } while (0)
 
-void oa_planes_step_begin(oa_ctx* c);
-void oa_planes_step_end(oa_ctx* c);
 void oa_planes_force_begin(oa_ctx* c, int nt);
 void oa_planes_force_end(oa_ctx* c, const double* F);
 oa_status oa_planes_psi_refresh(oa_ctx* c, cudaStream_t s, const double* psi, int nt);
+
+// The nonlocal branch of a step: an error between fork and join still orders
+// its stream before what `s` runs next (both use the context's scratch).
+struct SideBranch {
+  cudaStream_t s, side;
+  cudaEvent_t join;
+  bool joined;
+  ~SideBranch() {
+    if (!joined && cudaEventRecord(join, side) == cudaSuccess) cudaStreamWaitEvent(s, join, 0);
+  }
+};
 
 // Launches of one step up to S (part A); no host synchronisation.  In the
 // mixed form the bf16 planes of psi come from the previous step's Psi T and
@@ -170,6 +179,7 @@ static oa_status launch_step_a(oa_ctx* c, cudaStream_t s, oa_cp_state* st, int c
   OA_CUDA_TRY(oa_launch_state_plane_density(c, s));
   OA_CUDA_TRY(cudaEventRecord(w->fork, s));
   OA_CUDA_TRY(cudaStreamWaitEvent(w->side, w->fork, 0));
+  SideBranch branch{s, w->side, w->join, false};
   OA_CUDA_TRY(oa_launch_rho_xc(c, s));
   c->phase_done = 1;
   const oa_status rv = oa_gpu_vks_build(c, s, nullptr);
@@ -185,6 +195,7 @@ static oa_status launch_step_a(oa_ctx* c, cudaStream_t s, oa_cp_state* st, int c
   const oa_status rf = oa_vks_apply(c, s, st->psi, 0, w->Fnl, w->join, w->F, nullptr);
   oa_planes_force_end(c, w->F);
   OA_STEP_TRY(rf);
+  branch.joined = true;
   // constraint force (computeLambdaAndCg): Lambda, Gamma = T Lambda, F' = F T - Psi Gamma
   if (nt) {
     OA_STEP_TRY(oa_gpu_pc_forward_mixed(c, s, st->psi, w->F, 1.0, 1.0, nt, w->lam));
@@ -277,11 +288,11 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
         if (w->exec) { cudaGraphExecDestroy(w->exec); w->exec = nullptr; }
         if (w->exec2) { cudaGraphExecDestroy(w->exec2); w->exec2 = nullptr; }
         int nker = ns_in_graph ? 0 : 1;  // the Newton-Schulz launch between the two graphs
+        StepScope scope(c);
         for (int part = 0; part < (ns_in_graph ? 1 : 2); ++part) {
           cudaGraph_t g = nullptr;
           OA_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
           oa_status r = OA_OK;
-          if (part == 0) oa_planes_step_begin(c);
           if (ns_in_graph) {
             r = launch_step_a(c, s, st, 1);
             if (r == OA_OK) r = launch_step_ns(c, s, st);
@@ -289,10 +300,14 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
           } else {
             r = part == 0 ? launch_step_a(c, s, st, 1) : launch_step_b(c, s, st);
           }
-          if (ns_in_graph || part == 1 || r != OA_OK) oa_planes_step_end(c);
           cudaError_t ce = cudaStreamEndCapture(s, &g);
-          if (r != OA_OK) { if (g) cudaGraphDestroy(g); return r; }
-          if (ce != cudaSuccess) { oa_set_error(cudaGetErrorString(ce), __FILE__, __LINE__); return OA_ERR_CUDA; }
+          if (c->fail_capture) { c->fail_capture = 0; ce = cudaErrorStreamCaptureInvalidated; }
+          if (r != OA_OK || ce != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            if (r == OA_OK) oa_set_error(cudaGetErrorString(ce), __FILE__, __LINE__);
+            return r != OA_OK ? r : OA_ERR_CUDA;
+          }
           {
             size_t nn = 0;
             if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
@@ -306,7 +321,7 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
           }
           ce = cudaGraphInstantiate(part == 0 ? &w->exec : &w->exec2, g, 0);
           cudaGraphDestroy(g);
-          if (ce != cudaSuccess) { oa_set_error(cudaGetErrorString(ce), __FILE__, __LINE__); return OA_ERR_CUDA; }
+          OA_CUDA_TRY(ce);
         }
         memcpy(w->key, key, sizeof(key));
         w->graph_kernels = nker;
@@ -320,12 +335,10 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
         OA_CUDA_TRY(cudaGraphLaunch(w->exec2, s));
       }
     } else {
-      oa_planes_step_begin(c);
-      oa_status r = launch_step_a(c, s, st, complete_prev);
-      if (r == OA_OK) r = launch_step_ns(c, s, st);
-      if (r == OA_OK) r = launch_step_b(c, s, st);
-      oa_planes_step_end(c);
-      OA_STEP_TRY(r);
+      StepScope scope(c);
+      OA_STEP_TRY(launch_step_a(c, s, st, complete_prev));
+      OA_STEP_TRY(launch_step_ns(c, s, st));
+      OA_STEP_TRY(launch_step_b(c, s, st));
     }
   }
   OA_STEP_TRY(oa_psi_t_settle(c, s, st->psi, st->psi_t, w->flag));
@@ -361,12 +374,10 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
 // kernels of different systems fill the GPU together.
 // ---------------------------------------------------------------------------
 static oa_status batch_launch_one(oa_ctx* c, cudaStream_t s, oa_cp_state* st, int complete_prev) {
-  oa_planes_step_begin(c);
-  oa_status r = launch_step_a(c, s, st, complete_prev);
-  if (r == OA_OK) r = launch_step_ns(c, s, st);
-  if (r == OA_OK) r = launch_step_b(c, s, st);
-  oa_planes_step_end(c);
-  return r;
+  StepScope scope(c);
+  OA_STEP_TRY(launch_step_a(c, s, st, complete_prev));
+  OA_STEP_TRY(launch_step_ns(c, s, st));
+  return launch_step_b(c, s, st);
 }
 
 extern "C" oa_status oa_gpu_cp_run_batch(oa_ctx** ctxs, oa_cp_state** states, int nsys, void* stream, int nsteps,
@@ -414,6 +425,7 @@ extern "C" oa_status oa_gpu_cp_run_batch(oa_ctx** ctxs, oa_cp_state** states, in
   oa_status ret = OA_OK;
   auto fail = [&](cudaError_t e, int line) {
     oa_set_error(cudaGetErrorString(e), __FILE__, line);
+    cudaGetLastError();  // reported here: not the next launch's error
     ret = OA_ERR_CUDA;
   };
   cudaError_t ce = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
@@ -461,7 +473,7 @@ extern "C" oa_status oa_gpu_cp_run_batch(oa_ctx** ctxs, oa_cp_state** states, in
         }
         const oa_status r = step_all(true);
         ce = cudaStreamEndCapture(s, &g);
-        if (r != OA_OK) { if (g) cudaGraphDestroy(g); ret = r; break; }
+        if (r != OA_OK) { if (g) cudaGraphDestroy(g); cudaGetLastError(); ret = r; break; }
         if (ce != cudaSuccess) { fail(ce, __LINE__); break; }
         size_t nn = 0;
         if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {

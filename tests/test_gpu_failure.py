@@ -7,7 +7,9 @@ CkAbort / EXIT: ortho.C:129-133, cp_lowdin.C:246-252):
   the context gives the right product on the next call;
 * a non-finite coefficient and a singular overlap matrix injected from the
   host: the native run returns OA_ERR_NONFINITE / OA_ERR_NOT_CONVERGED and
-  names the first failing step."""
+  names the first failing step;
+* a step capture reported as failed by a host hook: the stage calls that
+  follow sum their energies, and the next native run captures again."""
 import time
 
 import numpy as np
@@ -77,3 +79,37 @@ def test_singular_overlap_names_the_step():
         d.run_native(st, 2)
     assert ei.value.status in (OA_ERR_NONFINITE, OA_ERR_NOT_CONVERGED)
     assert "step 1 of 2" in str(ei.value)
+
+
+@pytest.mark.parametrize("nstate", [8, 49])
+def test_failed_capture_leaves_the_context_usable(nstate):
+    """One graph per step (8 states) and two around the cooperative
+    Newton-Schulz launch (49 states: the first one's capture fails)."""
+    import torch
+    from openatom_b200.gpu import CPDriver, OaError, OA_ERR_CUDA
+    s = make_system("w2", seed=34, nstate=nstate, dt=0.5, pseudo="analytic")
+    d, ref = CPDriver(s, "fp64"), CPDriver(s, "fp64")
+    st, sr = d.native_state(use_graph=True), ref.native_state(use_graph=True)
+    d.run_native(st, 1)
+    ref.run_native(sr, 1)
+    it = st.iteration
+    d.ctx.fault_inject(2)
+    with pytest.raises(OaError) as ei:
+        d.run_native(st, 2)
+    assert ei.value.status == OA_ERR_CUDA
+    # stage calls of other coefficients: their own energies
+    d.psi.mul_(0.9)
+    ref.psi.mul_(0.9)
+    d.forces()
+    ref.forces()
+    got, want = d.ctx.energies(), ref.ctx.energies()
+    for k in ("EKE", "EHART", "EEXT", "EEXC", "ENL"):
+        assert got[k] == want[k], k
+    # and the run goes on
+    d.psi.div_(0.9)
+    ref.psi.copy_(d.psi)
+    torch.cuda.synchronize()
+    st.iteration = it
+    for g, r in zip(d.run_native(st, 2), ref.run_native(sr, 2)):
+        for k in ("EKE", "EHART", "EEXT", "EEXC", "ENL", "FICT_KE"):
+            assert g[k] == r[k], k
