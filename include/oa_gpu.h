@@ -349,9 +349,9 @@ oa_status oa_gpu_cp_run(oa_ctx *ctx, void *stream, oa_cp_state *state, int nstep
  * back.  Results are those of oa_gpu_cp_run on each system alone.  The
  * reference runs such sets as separate instances (UberCollection /
  * InstanceController, main/InstanceController.C).  energies_out (optional,
- * host [nsys][nsteps][14]).  Needs at most 128 states per system (the whole
- * step captured); a Newton-Schulz failure names the first failing system
- * and step. */
+ * host [nsys][nsteps][14]).  Needs at most 48 states per system, or an even
+ * number up to 128 (the whole step captured); a Newton-Schulz failure names
+ * the first failing system and step. */
 oa_status oa_gpu_cp_run_batch(oa_ctx **ctxs, oa_cp_state **states, int nsys, void *stream, int nsteps,
                               double *energies_out);
 

@@ -27,6 +27,7 @@ cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* 
 int oa_ns_grid(int n, int device);
 int oa_pencil_supported(int n);
 int oa_ns_cluster_size(int n);
+int oa_ns_one_block(int n);
 cudaError_t oa_launch_ortho_ns(cudaStream_t s, const double* S, int n, double bscale, double tol, int max_iter,
                                double* work, double* T, int* status, double* errv, int grid);
 int oa_integrate_nblk(int ng, int nstate);
@@ -207,8 +208,10 @@ static oa_ctx_pc* pcx(oa_ctx* c) { return &reinterpret_cast<oa_ctx_full*>(c)->pc
 // kernel, else the cooperative grid
 static int ns_launch_grid(const oa_ctx_pc* p) { return p->ns_cluster > 0 ? -p->ns_cluster : p->ns_grid; }
 
-// whether the Newton-Schulz launch can be captured in a CUDA graph
-int oa_ns_capturable(oa_ctx* c) { return pcx(c)->ns_cluster > 0; }
+// whether the Newton-Schulz launch can be captured in a CUDA graph: the
+// one-block and the cluster kernel can, the cooperative one is launched
+// outside (oa_launch_ortho_ns chooses)
+int oa_ns_capturable(oa_ctx* c) { return oa_ns_one_block(c->nstate) || pcx(c)->ns_cluster > 0; }
 
 static bool make_plan(int n, OaFftPlan* p) {
   p->n = n;

@@ -244,6 +244,8 @@ k_ortho_ns_cluster(const double* __restrict__ S, int n, double bscale, double to
 // ---------------------------------------------------------------------------
 #define NSS_MAXN 48
 
+int oa_ns_one_block(int n) { return n <= NSS_MAXN; }
+
 __device__ __forceinline__ void nss_tile(const double* X, const double* Y, int ld, int np, int rt, int ct, double& d0,
                                          double& d1) {
   const int lane = threadIdx.x & 31;

@@ -73,8 +73,8 @@ struct oa_step_scratch {
   cudaGraphExec_t exec;   // PsiV reset .. S
   cudaGraphExec_t exec2;  // Psi T + the step record
   const void* key[9];
-  int key_nterm;
-  double key_dt, key_tol;
+  int key_nterm, key_ns_iter;
+  double key_dt, key_tol, key_ns_tol;
   int graph_kernels;      // kernel launches of one graphed step (graph nodes + launches outside)
 };
 
@@ -222,7 +222,7 @@ static oa_status launch_step_a(oa_ctx* c, cudaStream_t s, oa_cp_state* st, int c
   return OA_OK;
 }
 
-// Newton-Schulz: one cooperative launch (kept out of the captured graphs)
+// Newton-Schulz (in the captured step where oa_ns_capturable)
 static oa_status launch_step_ns(oa_ctx* c, cudaStream_t s, oa_cp_state* st) {
   oa_step_scratch* w = step_scratch(c);
   double *work, *errv, *dev_e, *hv, *eye;
@@ -267,8 +267,8 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
                         (const void*)(uintptr_t)c->xc_gen, (const void*)(uintptr_t)c->eesl_gen};
   // the legacy default stream cannot be captured: launch eagerly there
   const bool capturable = s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread;
-  // the cluster Newton-Schulz kernel is an ordinary launch: then the whole
-  // step is one graph; the cooperative one splits it in two
+  // the one-block and the cluster Newton-Schulz kernel are ordinary launches:
+  // then the whole step is one graph; the cooperative one splits it in two
   const bool ns_in_graph = oa_ns_capturable(c) != 0;
   if (pos_host && c->ions) {
     oa_set_error("pos_host with ion dynamics on: the atoms move on the device", __FILE__, __LINE__);
@@ -283,7 +283,8 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
     const bool use_graph = st->use_graph && complete_prev && capturable;
     if (use_graph) {
       const bool same = w->exec && (ns_in_graph || w->exec2) && memcmp(key, w->key, sizeof(key)) == 0 &&
-                        w->key_nterm == st->mixed_nterm && w->key_dt == st->dt && w->key_tol == st->norb_tol;
+                        w->key_nterm == st->mixed_nterm && w->key_dt == st->dt && w->key_tol == st->norb_tol &&
+                        w->key_ns_tol == st->ns_tol && w->key_ns_iter == st->ns_max_iter;
       if (!same) {
         if (w->exec) { cudaGraphExecDestroy(w->exec); w->exec = nullptr; }
         if (w->exec2) { cudaGraphExecDestroy(w->exec2); w->exec2 = nullptr; }
@@ -328,6 +329,8 @@ static oa_status run_steps(oa_ctx* c, void* stream, oa_cp_state* st, int nsteps,
         w->key_nterm = st->mixed_nterm;
         w->key_dt = st->dt;
         w->key_tol = st->norb_tol;
+        w->key_ns_tol = st->ns_tol;
+        w->key_ns_iter = st->ns_max_iter;
       }
       OA_CUDA_TRY(cudaGraphLaunch(w->exec, s));
       if (!ns_in_graph) {
@@ -407,10 +410,9 @@ extern "C" oa_status oa_gpu_cp_run_batch(oa_ctx** ctxs, oa_cp_state** states, in
         oa_set_error("a context appears twice in the batch", __FILE__, __LINE__);
         return OA_ERR_BAD_ARG;
       }
-    // the whole step must be capturable: the cluster Newton-Schulz kernel
+    // the whole step must be capturable
     if (!oa_ns_capturable(c)) {
-      oa_set_error("the batched run needs the cluster Newton-Schulz kernel (at most 128 states)", __FILE__,
-                   __LINE__);
+      oa_set_error("the batched run takes up to 48 states, or an even number up to 128", __FILE__, __LINE__);
       return OA_ERR_UNSUPPORTED;
     }
   }
