@@ -463,6 +463,7 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
       if (oa_pair_plane_shape(c, &dbps, &vbps, &split) == cudaSuccess) {
         c->ngroup_pair = pick_pair_groups(d->nz * split, npair, dbps, nsm);
         c->ngroup_vks = pick_pair_groups(d->nz, npair, vbps, nsm);
+        c->pair_split = split;
       } else {
         cudaGetLastError();
         c->pair_on = 0;
@@ -475,9 +476,9 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     }
     if (c->pair_on && precision == OA_MIXED) {
       // charge partials of the z forward pass (state x 16-line block) and of
-      // the pair density pass (group x plane) for the density renormalisation
+      // the pair density pass (group x plane x row split) for the density renormalisation
       c->nq = d->nstate * ((d->nlines + OA_LB - 1) / OA_LB);
-      c->nq2 = c->ngroup_pair * d->nz;
+      c->nq2 = c->ngroup_pair * d->nz * c->pair_split;
       TRY(cudaMalloc(&c->qpart, (size_t)c->nq * sizeof(double)));
       TRY(cudaMalloc(&c->qpart2, (size_t)c->nq2 * sizeof(double)));
       c->nq2_cap = c->nq2;
@@ -1061,7 +1062,8 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
   const int gs = t->group_state ? t->group_state : c->ngroup;
   const int gp = t->group_pair ? t->group_pair : c->ngroup_pair;
   const int need = gs > gp ? gs : gp;
-  if (need > c->rho_groups_cap || (c->qpart && gp * c->nz > c->nq2_cap)) {
+  const int nq2 = gp * c->nz * c->pair_split;
+  if (need > c->rho_groups_cap || (c->qpart && nq2 > c->nq2_cap)) {
     OA_CUDA_TRY(cudaDeviceSynchronize());
     if (need > c->rho_groups_cap) {
       double* r = nullptr;
@@ -1070,17 +1072,17 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
       c->rho_part = r;
       c->rho_groups_cap = need;
     }
-    if (c->qpart && gp * c->nz > c->nq2_cap) {
+    if (c->qpart && nq2 > c->nq2_cap) {
       double* q = nullptr;
-      OA_CUDA_TRY(cudaMalloc(&q, (size_t)gp * c->nz * sizeof(double)));
+      OA_CUDA_TRY(cudaMalloc(&q, (size_t)nq2 * sizeof(double)));
       cudaFree(c->qpart2);
       c->qpart2 = q;
-      c->nq2_cap = gp * c->nz;
+      c->nq2_cap = nq2;
     }
   }
   c->ngroup = gs;
   c->ngroup_pair = gp;
-  if (c->qpart) c->nq2 = gp * c->nz;
+  if (c->qpart) c->nq2 = nq2;
   if (t->dgemm_kblocks) p->nkb = t->dgemm_kblocks;
   if (t->tgemm_kblocks) p->umax_kb = t->tgemm_kblocks;
   if (t->fft_path) c->fft_runtime = t->fft_path == 2 ? 1 : 0;

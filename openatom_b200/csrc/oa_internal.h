@@ -115,6 +115,7 @@ struct oa_ctx {
   int rho_ngroup;         // groups summed in rho_part by the last density pass
   int* pair_cols;         // [nkx_s] {first line, ky of the first line, lines, 0} when the lines form column runs
   int pair_on;            // the state-pair plane kernels take this system
+  int pair_split;         // row splits of the state-pair density kernel (blocks per plane and group)
   int pair_kymax;         // largest |ky| of the state lines
   int z_ext;              // largest kz count of a state line on either side (max of nneg, npos)
   void* psir;             // psi(r), compute precision: [nstate][nz][ny][nx] (two-pass kernels)
