@@ -203,7 +203,9 @@ oa_status oa_gpu_check(oa_ctx *ctx, void *stream);
  * product skips the loads of one pipeline stage in one block, so that
  * block's bounded wait runs out and oa_gpu_check reports it (acts on the
  * current device); kind 2: the next graph capture of this context's native
- * step is reported as failed on the host; kind 0 clears the hooks. */
+ * step is reported as failed on the host; kind 3: the next device allocation
+ * of this thread that psi(r) makes room for (or psi(r)'s own in
+ * oa_gpu_init) is reported as failed on the host; kind 0 clears the hooks. */
 oa_status oa_gpu_fault_inject(oa_ctx *ctx, int kind);
 
 /* Small dense C = alpha A B (N x N), e.g. Gamma = T Lambda (ortho.C:565-570). */

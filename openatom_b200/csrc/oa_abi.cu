@@ -88,6 +88,24 @@ extern "C" const char* oa_gpu_last_error(void) { return g_err; }
     if (!(cond)) { oa_set_error(msg, __FILE__, __LINE__); return OA_ERR_BAD_ARG; } \
   } while (0)
 
+// host hook of the tests (oa_gpu_fault_inject 3)
+static thread_local bool t_fail_alloc = false;
+void oa_fail_next_alloc(bool on) { t_fail_alloc = on; }
+
+cudaError_t oa_ctx_malloc(oa_ctx* c, void** p, size_t bytes) {
+  const bool fail = t_fail_alloc;
+  t_fail_alloc = false;
+  const cudaError_t e = fail ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !c->psir) return e;
+  cudaGetLastError();
+  cudaFree(c->psir);  // waits for the kernels that use it
+  c->psir = nullptr;
+  c->psir_valid = 0;
+  c->pair_on = 0;
+  c->xc_gen += 1;  // captured steps hold its address
+  return cudaMalloc(p, bytes);
+}
+
 // unique id of the device's current CUDA context (0: unknown): it changes
 // when the device has been reset
 static unsigned long long context_id() {
@@ -147,7 +165,7 @@ static void forget_stale_smem_limits() {
 
 // FP64-accurate int8 tensor-core products of the mixed form (oa_ozaki.cu)
 struct oa_oz;
-oa_oz* oa_oz_create(int n, int ng, int nkx0, int nsm);
+oa_oz* oa_oz_create(oa_ctx* ctx, int n, int ng, int nkx0, int nsm);
 void oa_oz_free(oa_oz* z);
 size_t oa_oz_bytes(const oa_oz* z);
 cudaError_t oa_oz_overlap(oa_oz* z, cudaStream_t s, const double* X, long ldx, double alpha, double w_kx0,
@@ -446,17 +464,10 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     c->zbuf_bytes = (size_t)d->nstate * d->nz * c->ldl * csz;
     TRY(cudaMalloc(&c->zbuf, c->zbuf_bytes));
     {
-      // state-pair kernels: lines in column runs, room for psi(r) of all
-      // states (without it the per-state kernels redo the forward transforms)
+      // state-pair kernels: lines in column runs (and room for psi(r), below)
       std::vector<int> runs;
       const bool pairs = d->nx == d->ny && column_runs(d, c->nkx_s, &runs);
       if (pairs) TRY(upload(&c->pair_cols, runs.data(), runs.size()));
-      if (pairs || (d->nx == d->ny && oa_plane2_supported(d->nx))) {
-        if (cudaMalloc(&c->psir, (size_t)(d->nstate + 1) / 2 * 2 * c->npts * rsz) != cudaSuccess) {
-          c->psir = nullptr;
-          cudaGetLastError();
-        }
-      }
       int dbps = 1, vbps = 1, split = 1;
       const int npair = (d->nstate + 1) / 2;
       c->pair_on = c->pair_cols != nullptr;
@@ -467,10 +478,6 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
       } else {
         cudaGetLastError();
         c->pair_on = 0;
-        if (c->psir && !(d->nx == d->ny && oa_plane2_supported(d->nx))) {
-          cudaFree(c->psir);
-          c->psir = nullptr;
-        }
         c->ngroup_pair = pick_pair_groups(d->nz, npair, 1, nsm);
       }
     }
@@ -548,6 +555,15 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     }
     TRY(cudaMallocHost(&p->h_status, 4 * sizeof(int)));
     TRY(cudaMallocHost(&p->h_vals, 16 * sizeof(double)));
+    // psi(r) of all states, after what a context cannot do without: where
+    // there is no memory left for it the per-state kernels redo the forward
+    // transforms
+    if ((c->pair_on || (d->nx == d->ny && oa_plane2_supported(d->nx))) &&
+        oa_ctx_malloc(c, &c->psir, (size_t)(d->nstate + 1) / 2 * 2 * c->npts * rsz) != cudaSuccess) {
+      cudaGetLastError();
+      c->psir = nullptr;
+      c->pair_on = 0;
+    }
     TRY(cudaDeviceSynchronize());
   }
 #undef TRY
@@ -734,7 +750,7 @@ extern "C" oa_status oa_gpu_pc_forward(oa_ctx* c, void* stream, const double* le
 static bool oz_ready(oa_ctx* c) {
   oa_ctx_pc* p = pcx(c);
   if (!p->oz && c->precision == OA_MIXED && c->nstate <= 128)
-    p->oz = oa_oz_create(c->nstate, c->ng, c->nkx0, p->nsm);
+    p->oz = oa_oz_create(c, c->nstate, c->ng, c->nkx0, p->nsm);
   return p->oz != nullptr;
 }
 
@@ -901,9 +917,9 @@ extern "C" oa_status oa_gpu_set_xc(oa_ctx* c, int functional, double gradient_cu
     oa_set_error("gradient_cutoff must be > 0", __FILE__, __LINE__);
     return OA_ERR_BAD_ARG;
   }
-  if (functional == 1 && !c->grad) {
-    OA_CUDA_TRY(cudaMalloc(&c->grad, (size_t)3 * c->npts * sizeof(double)));
-    OA_CUDA_TRY(cudaMalloc(&c->dzg, (size_t)3 * c->nz * c->ldl_d * sizeof(double2)));
+  if (functional == 1) {
+    if (!c->grad) OA_CUDA_TRY(oa_ctx_malloc(c, &c->grad, (size_t)3 * c->npts * sizeof(double)));
+    if (!c->dzg) OA_CUDA_TRY(oa_ctx_malloc(c, &c->dzg, (size_t)3 * c->nz * c->ldl_d * sizeof(double2)));
   }
   c->gga = functional;
   c->gga_cut = gradient_cutoff;
@@ -1067,7 +1083,7 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
     OA_CUDA_TRY(cudaDeviceSynchronize());
     if (need > c->rho_groups_cap) {
       double* r = nullptr;
-      OA_CUDA_TRY(cudaMalloc(&r, (size_t)need * c->npts * sizeof(double)));
+      OA_CUDA_TRY(oa_ctx_malloc(c, &r, (size_t)need * c->npts * sizeof(double)));
       cudaFree(c->rho_part);
       c->rho_part = r;
       c->rho_groups_cap = need;
@@ -1532,24 +1548,31 @@ extern "C" oa_status oa_gpu_ees_init(oa_ctx* c, int na, int nb, int nc, int orde
   e->tw_b = make_twiddles(nb);
   e->tw_c = make_twiddles(nc);
   if (!e->tw_a || !e->tw_b || !e->tw_c) { ees_free(c); oa_set_error("twiddle allocation failed", __FILE__, __LINE__); return OA_ERR_CUDA; }
-  TRYE(cudaMalloc(&e->zbuf, (size_t)c->nstate * nc * c->ldl * csz));
+  TRYE(oa_ctx_malloc(c, &e->zbuf, (size_t)c->nstate * nc * c->ldl * csz));
   TRYE(upload(&e->dyp, (const double2*)dyp_host, (size_t)c->ng));
   TRYE(cudaMalloc(&e->idx, (size_t)c->natm_nl * 3 * order * sizeof(int)));
   TRYE(cudaMalloc(&e->mn, (size_t)c->natm_nl * 3 * order * sizeof(double)));
-  TRYE(cudaMalloc(&e->zpart, (size_t)c->nstate * c->natm_nl * order * order * sizeof(double)));
-  TRYE(cudaMalloc(&e->zmat, (size_t)c->nstate * c->natm_nl * sizeof(double)));
-  TRYE(cudaMalloc(&e->zs, (size_t)c->nstate * c->natm_nl * sizeof(double)));
-  TRYE(cudaMalloc(&e->enl, (size_t)c->nstate * sizeof(double)));
-  TRYE(cudaMalloc(&e->dmn, (size_t)c->natm_nl * 3 * order * sizeof(double)));
-  TRYE(cudaMalloc(&e->fpart, (size_t)c->nstate * c->natm_nl * order * order * 3 * sizeof(double)));
-#undef TRYE
   int pbps = 1;
-  e->ngroup_pair = 0;
   if (oa_ees_pair_shape(c, &pbps) == cudaSuccess)
     e->ngroup_pair = pick_pair_groups(nc, (c->nstate + 1) / 2, pbps, pcx(c)->nsm);
   else
     cudaGetLastError();
+  e->npmax = e->ngroup_pair > 0 ? order * order : order;
+  TRYE(oa_ctx_malloc(c, &e->zpart, (size_t)c->nstate * c->natm_nl * e->npmax * sizeof(double)));
+  TRYE(cudaMalloc(&e->zmat, (size_t)c->nstate * c->natm_nl * sizeof(double)));
+  TRYE(cudaMalloc(&e->zs, (size_t)c->nstate * c->natm_nl * sizeof(double)));
+  TRYE(cudaMalloc(&e->enl, (size_t)c->nstate * sizeof(double)));
+  TRYE(cudaMalloc(&e->dmn, (size_t)c->natm_nl * 3 * order * sizeof(double)));
+  if (c->ions) TRYE(oa_ees_ion_partials(c));
+#undef TRYE
   return OA_OK;
+}
+
+// atom-force partials of the EES method, for contexts with ion dynamics
+cudaError_t oa_ees_ion_partials(oa_ctx* c) {
+  oa_ees* e = c->ees;
+  if (!e || e->fpart) return cudaSuccess;
+  return oa_ctx_malloc(c, &e->fpart, (size_t)3 * c->nstate * c->natm_nl * e->npmax * sizeof(double));
 }
 
 // get_bspline_wght1d (set_cp_ewald.C:1237-1325): for m = 0..ngrid-1
@@ -1616,8 +1639,8 @@ extern "C" oa_status oa_gpu_set_ees_local(oa_ctx* c, int na, int nb, int nc, int
   TRYL(upload(&L->bc, bc.data(), bc.size()));
   TRYL(upload(&L->gzvps, c->gzvps_t, (size_t)c->ntype));
   const size_t gbytes = (size_t)L->ngrid * na * nb * nc * sizeof(double2);
-  TRYL(cudaMalloc(&L->zq, gbytes));
-  TRYL(cudaMalloc(&L->zy, gbytes));
+  TRYL(oa_ctx_malloc(c, &L->zq, gbytes));
+  TRYL(oa_ctx_malloc(c, &L->zy, gbytes));
 #undef TRYL
   return OA_OK;
 }

@@ -38,6 +38,7 @@ static inline cudaError_t oa_smem_limit(K kernel) {
 struct oa_ees {
   int na, nb, nc, order, ngroup;
   int ngroup_pair;     // pair groups of the state-pair kernels (0: they do not take this grid)
+  int npmax;           // Z partials per (state, atom): order, or order^2 with the pair kernels
   OaFftPlan pa, pb, pc;
   double2 *tw_a, *tw_b, *tw_c;
   void* zbuf;          // [nstate][nc][ldl] compute precision
@@ -49,7 +50,7 @@ struct oa_ees {
   double* zs;          // [nstate][natm_nl]
   double* enl;         // [nstate]
   double* dmn;         // [natm_nl][3][order] B-spline derivative weights (ion dynamics)
-  double* fpart;       // [3] atom-force sums beside each zpart entry (ion dynamics)
+  double* fpart;       // [3] atom-force sums beside each zpart entry (null without ion dynamics)
 };
 
 // EES local pseudopotential and reciprocal Ewald path (oa_gpu_set_ees_local,
@@ -225,6 +226,16 @@ cudaError_t oa_launch_phase_tables(oa_ctx* c, cudaStream_t s);
   } while (0)
 
 void oa_set_error(const char* msg, const char* file, int line);
+
+// Device memory of a context.  Where there is none left, psi(r) gives its own
+// back (the per-state kernels then redo the forward transforms) and the
+// allocation is tried again: what fits without psi(r) fits.
+cudaError_t oa_ctx_malloc(oa_ctx* c, void** p, size_t bytes);
+template <typename T> static inline cudaError_t oa_ctx_malloc(oa_ctx* c, T** p, size_t bytes) {
+  return oa_ctx_malloc(c, (void**)p, bytes);
+}
+void oa_fail_next_alloc(bool on);
+cudaError_t oa_ees_ion_partials(oa_ctx* c);
 
 void oa_planes_step_begin(oa_ctx* c);
 void oa_planes_step_end(oa_ctx* c);

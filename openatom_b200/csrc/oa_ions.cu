@@ -282,6 +282,8 @@ cudaError_t oa_launch_ion_step(oa_ctx* c, cudaStream_t s, double* dev_e, double 
 
 int oa_rho_z_nblk(const oa_ctx* c);
 
+void oa_ions_free(oa_ctx* c);
+
 extern "C" oa_status oa_gpu_set_ions(oa_ctx* c, const double* masses, const double* vel) {
   if (!c || !masses) {
     oa_set_error("null argument", __FILE__, __LINE__);
@@ -298,13 +300,21 @@ extern "C" oa_status oa_gpu_set_ions(oa_ctx* c, const double* masses, const doub
     if (!io) { oa_set_error("out of host memory", __FILE__, __LINE__); return OA_ERR_CUDA; }
     c->ions = io;
     io->nfpart = oa_rho_z_nblk(c);
-    OA_ION_TRY(cudaMalloc(&io->m, (size_t)c->natm * sizeof(double)));
-    OA_ION_TRY(cudaMalloc(&io->v, (size_t)3 * c->natm * sizeof(double)));
-    OA_ION_TRY(cudaMalloc(&io->fpart, (size_t)io->nfpart * 3 * c->natm * sizeof(double)));
-    OA_ION_TRY(cudaMalloc(&io->fnl, (size_t)3 * c->natm * sizeof(double)));
-    OA_ION_TRY(cudaMalloc(&io->fr, (size_t)3 * c->natm * sizeof(double)));
-    OA_ION_TRY(cudaMalloc(&io->er, (size_t)c->natm * sizeof(double)));
-    OA_ION_TRY(cudaMalloc(&io->y, ((size_t)2 * c->natm_nl * c->ng + 1) * sizeof(double)));
+    const size_t na = c->natm;
+    cudaError_t e = oa_ctx_malloc(c, &io->m, na * sizeof(double));
+    if (e == cudaSuccess) e = oa_ctx_malloc(c, &io->v, 3 * na * sizeof(double));
+    if (e == cudaSuccess) e = oa_ctx_malloc(c, &io->fpart, (size_t)io->nfpart * 3 * na * sizeof(double));
+    if (e == cudaSuccess) e = oa_ctx_malloc(c, &io->fnl, 3 * na * sizeof(double));
+    if (e == cudaSuccess) e = oa_ctx_malloc(c, &io->fr, 3 * na * sizeof(double));
+    if (e == cudaSuccess) e = oa_ctx_malloc(c, &io->er, na * sizeof(double));
+    if (e == cudaSuccess) e = oa_ctx_malloc(c, &io->y, ((size_t)2 * c->natm_nl * c->ng + 1) * sizeof(double));
+    if (e == cudaSuccess) e = oa_ees_ion_partials(c);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      oa_ions_free(c);  // ion dynamics stays off
+      oa_set_error(cudaGetErrorString(e), __FILE__, __LINE__);
+      return OA_ERR_CUDA;
+    }
     OA_ION_TRY(cudaMemset(io->fpart, 0, (size_t)io->nfpart * 3 * c->natm * sizeof(double)));
     // per-atom charges on the host for the self and background terms
     std::vector<int> at(c->natm);

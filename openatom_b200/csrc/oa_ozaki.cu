@@ -570,7 +570,7 @@ void oa_oz_free(oa_oz* z) {
 
 // Set up the int8 products for n <= 128 states over ng g-points with nkx0
 // on the kx = 0 plane; nullptr when not available (the caller keeps FP64).
-oa_oz* oa_oz_create(int n, int ng, int nkx0, int nsm) {
+oa_oz* oa_oz_create(oa_ctx* ctx, int n, int ng, int nkx0, int nsm) {
   if (n < 1 || n > 128 || !oz_encoder()) return nullptr;
   oa_oz* z = (oa_oz*)calloc(1, sizeof(oa_oz));
   if (!z) return nullptr;
@@ -604,13 +604,13 @@ oa_oz* oa_oz_create(int n, int ng, int nkx0, int nsm) {
   for (int q = 0; q < R; ++q) maxlen = std::max(maxlen, rc[q + 1] - rc[q]);
   z->maxlen = maxlen;
   bool okm = true;
-  okm &= cudaMalloc(&z->rc, (R + 1) * sizeof(int)) == cudaSuccess;
-  okm &= cudaMalloc(&z->cr, z->nch * sizeof(int)) == cudaSuccess;
-  okm &= cudaMalloc(&z->sl, (size_t)OZ_ND * z->nch * OZ_TILE) == cudaSuccess;
-  okm &= cudaMalloc(&z->tsl, (size_t)R * OZ_NDT * OZ_TILE) == cudaSuccess;
-  okm &= cudaMalloc(&z->ex, (size_t)R * 128 * sizeof(int)) == cudaSuccess;
-  okm &= cudaMalloc(&z->fx, (size_t)R * 128 * sizeof(int)) == cudaSuccess;
-  okm &= cudaMalloc(&z->part, (size_t)R * 128 * 128 * sizeof(double)) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->rc, (R + 1) * sizeof(int)) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->cr, z->nch * sizeof(int)) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->sl, (size_t)OZ_ND * z->nch * OZ_TILE) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->tsl, (size_t)R * OZ_NDT * OZ_TILE) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->ex, (size_t)R * 128 * sizeof(int)) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->fx, (size_t)R * 128 * sizeof(int)) == cudaSuccess;
+  okm &= oa_ctx_malloc(ctx, &z->part, (size_t)R * 128 * 128 * sizeof(double)) == cudaSuccess;
   if (!okm) { oa_oz_free(z); cudaGetLastError(); return nullptr; }
   // rows n..127 of the slices stay zero
   okm &= cudaMemset(z->sl, 0, (size_t)OZ_ND * z->nch * OZ_TILE) == cudaSuccess;

@@ -441,7 +441,7 @@ static cudaError_t pencil_plane(oa_ctx* c, cudaStream_t s, int mode, void* psir)
 // the launch shape (resident blocks per SM, row splits).
 static cudaError_t pair_plane(oa_ctx* c, cudaStream_t s, int mode, double* qpart, int* dbps = nullptr,
                               int* vbps = nullptr, int* split = nullptr) {
-  if (c->fft_runtime || !c->pair_on || !c->psir) return cudaErrorNotSupported;
+  if (c->fft_runtime || !c->pair_on || (!c->psir && mode >= 0)) return cudaErrorNotSupported;
   PpArgs A;
   A.mode = mode; A.n = c->nx; A.st = s; A.zbuf = c->zbuf;
   A.nstate = c->nstate; A.nz = c->nz; A.ldl = c->ldl; A.nlines = c->nlines;

@@ -97,9 +97,9 @@ static oa_status ensure_scratch(oa_ctx* c) {
   const size_t cb = (size_t)c->nstate * c->ng * sizeof(double2);
   const size_t mb = (size_t)c->nstate * c->nstate * sizeof(double);
   c->step = s;  // freed by oa_step_free on failure below or at destroy
-  if (cudaMalloc(&s->F, cb) != cudaSuccess || cudaMalloc(&s->F2, cb) != cudaSuccess ||
-      cudaMalloc(&s->Fnl, cb) != cudaSuccess || cudaMalloc(&s->S, mb) != cudaSuccess ||
-      cudaMalloc(&s->lam, mb) != cudaSuccess || cudaMalloc(&s->gam, mb) != cudaSuccess ||
+  if (oa_ctx_malloc(c, &s->F, cb) != cudaSuccess || oa_ctx_malloc(c, &s->F2, cb) != cudaSuccess ||
+      oa_ctx_malloc(c, &s->Fnl, cb) != cudaSuccess || oa_ctx_malloc(c, &s->S, mb) != cudaSuccess ||
+      oa_ctx_malloc(c, &s->lam, mb) != cudaSuccess || oa_ctx_malloc(c, &s->gam, mb) != cudaSuccess ||
       cudaMalloc(&s->flag, 4 * sizeof(int)) != cudaSuccess || cudaMemset(s->flag, 0, 4 * sizeof(int)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess ||

@@ -182,13 +182,14 @@ __global__ void k_split_kc(const double* __restrict__ X, int rows, int rows_pad,
 __device__ int g_oa_inject_skip_load = 0;
 
 extern "C" oa_status oa_gpu_fault_inject(oa_ctx* c, int kind) {
-  if (!c || kind < 0 || kind > 2) {
-    oa_set_error("kind must be 0 (clear), 1 (skip one stage's loads) or 2 (fail a step's capture)", __FILE__,
-                 __LINE__);
+  if (!c || kind < 0 || kind > 3) {
+    oa_set_error("kind must be 0 (clear), 1 (skip one stage's loads), 2 (fail a step's capture) or 3 (fail an "
+                 "allocation)", __FILE__, __LINE__);
     return OA_ERR_BAD_ARG;
   }
-  if (kind != 1) c->fail_capture = kind == 2;
-  if (kind == 2) return OA_OK;
+  if (kind == 0 || kind == 2) c->fail_capture = kind == 2;
+  if (kind == 0 || kind == 3) oa_fail_next_alloc(kind == 3);
+  if (kind >= 2) return OA_OK;
   const int v = kind;
   OA_CUDA_TRY(cudaMemcpyToSymbol(g_oa_inject_skip_load, &v, sizeof(int)));
   return OA_OK;

@@ -389,7 +389,8 @@ class CPContext:
     def fault_inject(self, kind: int):
         """Test hook: kind 1 makes the next split-BF16 forward product skip
         one stage's loads in one block (its bounded wait runs out); kind 2
-        reports the next capture of a native step as failed; 0 clears."""
+        reports the next capture of a native step as failed, kind 3 the next
+        device allocation that psi(r) can make room for; 0 clears."""
         _check(self._lib.oa_gpu_fault_inject(self._h, int(kind)))
 
     def small_gemm(self, A, B, alpha, out):

@@ -9,7 +9,9 @@ CkAbort / EXIT: ortho.C:129-133, cp_lowdin.C:246-252):
   host: the native run returns OA_ERR_NONFINITE / OA_ERR_NOT_CONVERGED and
   names the first failing step;
 * a step capture reported as failed by a host hook: the stage calls that
-  follow sum their energies, and the next native run captures again."""
+  follow sum their energies, and the next native run captures again;
+* a device allocation reported as failed by a host hook: psi(r) gives its
+  memory back and the per-state kernels take the system."""
 import time
 
 import numpy as np
@@ -113,3 +115,51 @@ def test_failed_capture_leaves_the_context_usable(nstate):
     for g, r in zip(d.run_native(st, 2), ref.run_native(sr, 2)):
         for k in ("EKE", "EHART", "EEXT", "EEXC", "ENL", "FICT_KE"):
             assert g[k] == r[k], k
+
+
+KEYS = ("EKE", "EHART", "EEXT", "EEXC", "ENL", "FICT_KE")
+
+
+def agree(got, ref, s, precision):
+    """Two transform paths: FP64 to rounding; mixed, FP32 transforms with and
+    without the renormalised density, as for the tuning choices."""
+    tol = 1e-11 if precision == "fp64" else 2e-6
+    for g, r in zip(got, ref):
+        for k in KEYS:
+            assert abs(g[k] - r[k]) <= tol * max(1.0, abs(r[k])), (k, g[k], r[k])
+        assert abs(sum(g[k] - r[k] for k in KEYS[:5])) / s.natm <= (1e-11 if precision == "fp64" else 1e-6)
+
+
+# lengths whose per-state kernels are the runtime plan (45) and the two-pass kernels (64)
+@pytest.mark.parametrize("n,nstate", [(45, 5), (64, 8)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_no_memory_for_psir(n, nstate, precision):
+    from openatom_b200.gpu import CPContext, CPDriver
+    s = make_system("w2", seed=35, nfft=(n, n, n), nstate=nstate, box=7.0, ecut_ry=60.0, dt=0.5)
+    def driver():
+        return CPDriver(s, precision, tuning="default")
+    ref = driver()
+    assert ref.ctx.sizes()["pair_planes"] == 1
+    want = ref.run_native(ref.native_state(), 3)
+    # at init
+    other = CPContext(make_system("w2", seed=3), "fp64")
+    other.fault_inject(3)
+    d = driver()
+    assert d.ctx.sizes()["pair_planes"] == 0
+    agree(d.run_native(d.native_state(), 3), want, s, precision)
+    # at the first native call, between two passes of the force half
+    d = driver()
+    d.ctx.state_fft_fwd(d.psi)
+    d.ctx.fault_inject(3)
+    agree(d.run_native(d.native_state(), 3), want, s, precision)
+    assert d.ctx.sizes()["pair_planes"] == 0
+    # with a captured step in hand
+    d = driver()
+    st, sr = d.native_state(), ref.native_state()
+    d.run_native(st, 3)
+    assert d.ctx.sizes()["pair_planes"] == 1
+    d.ctx.fault_inject(3)
+    d.ctx.set_xc("blyp")
+    ref.ctx.set_xc("blyp")
+    assert d.ctx.sizes()["pair_planes"] == 0
+    agree(d.run_native(st, 3), ref.run_native(sr, 3), s, precision)

@@ -148,6 +148,37 @@ def test_local_forces_of_uneven_atoms(nz, types):
     assert np.max(np.abs(runs[0] - ions.v)) <= 1e-10 * np.max(np.abs(ions.v))
 
 
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-5)])
+@pytest.mark.parametrize("nstate,order,ions_first", [(5, 4, True), (7, 6, False), (8, 8, False)])
+def test_ees_atom_forces(nstate, order, ions_first, precision, tol):
+    """Atom forces of the EES method in both forms, with a last state alone
+    in its pair, and ion dynamics switched on before or after the method:
+    the first half kick against the oracle (mixed: FP32 transforms)."""
+    from openatom_b200.gpu import CPDriver
+    s, m, _ = _start("w2", nstate, 46)
+    d = CPDriver(s, precision, norb_tol=0.003)
+    if ions_first:
+        d.ctx.set_ions(m)
+    d.ctx.ees_init(1.2, order)
+    if not ions_first:
+        d.ctx.set_ions(m)
+    d.run_native(d.native_state(), 1)
+    so = copy.deepcopy(s)
+    ions = O.IonState(so)
+    ees = O.ees_setup(so, 1.2, order)
+
+    def nl(psi, sysm):
+        f, enl, _ = O.nl_ees_energy_forces(psi, sysm, ees)
+        return f, float(enl.sum())
+
+    O.cp_step(O.CPState(so), so, nl=nl, norb_tol=0.003, ions=ions, ees=ees)
+    v = d.ctx.get_ions()[1]
+    assert np.max(np.abs(v - ions.v)) <= tol * np.max(np.abs(ions.v))
+    # the nonlocal part alone is a visible share of it
+    f_nl = O.nl_ees_energy_forces(s.psi, s, ees, atom_forces=True)[3]
+    assert np.max(np.abs(0.5 * s.dt * f_nl / m[:, None])) > 1e-3 * np.max(np.abs(ions.v))
+
+
 def test_ion_dynamics_refuses_host_positions():
     from openatom_b200.gpu import CPDriver, OaError
     s, m, vel = _start("w2", None, 44)
