@@ -1524,6 +1524,7 @@ extern "C" oa_status oa_gpu_ees_init(oa_ctx* c, int na, int nb, int nc, int orde
   oa_ees* e = (oa_ees*)calloc(1, sizeof(oa_ees));
   if (!e) return OA_ERR_CUDA;
   c->ees = e;
+  c->xc_gen += 1;  // captured steps hold the old buffers (the new record may lie where the old one did)
   e->na = na; e->nb = nb; e->nc = nc; e->order = order;
   if (!make_plan(na, &e->pa) || !make_plan(nb, &e->pb) || !make_plan(nc, &e->pc)) {
     ees_free(c);

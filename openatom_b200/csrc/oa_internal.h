@@ -172,7 +172,7 @@ struct oa_ctx {
   // exchange + Becke 88 + LYP, oa_gpu_set_xc); gga_cut = \gradient_cutoff
   int gga;
   double gga_cut;
-  unsigned xc_gen;        // bumped by every oa_gpu_set_xc (captured step graphs key on it)
+  unsigned xc_gen;        // bumped by every call that captured steps depend on (their graphs key on it)
   double *grad;           // [3][nz][ny][nx] grad rho, then the GGA vector h (BLYP)
   void *dzg;              // [3][nz][ldl_d] C  z-lines of grad rho / h (BLYP)
   oa_ions *ions;          // ion dynamics, after oa_gpu_set_ions

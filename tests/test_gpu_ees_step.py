@@ -51,3 +51,20 @@ def test_native_step_ees_mixed_matches_host_runner():
             assert ec[i][k] == ea[i][k], (i, k, ea[i][k], ec[i][k])
     assert np.array_equal(a.psi.cpu().numpy(), c.psi.cpu().numpy())
     assert ec[0]["ENL"] != 0.0
+
+
+def test_captured_step_follows_a_new_ees_grid():
+    """oa_gpu_ees_init between two native runs: the captured step is made
+    again on the new buffers, the same bits as steps run eagerly."""
+    from openatom_b200.gpu import CPDriver
+    s = make_system("w2", seed=36, dt=0.5)
+    out = []
+    for graph in (True, False):
+        d = CPDriver(s, "fp64", nl_method="ees", ees_order=4)
+        st = d.native_state(use_graph=graph)
+        recs = d.run_native(st, 3)
+        d.ctx.ees_init(1.2, 6)
+        recs += d.run_native(st, 3)
+        out.append((recs, d.psi.cpu().numpy()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1])
