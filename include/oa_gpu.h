@@ -261,7 +261,8 @@ oa_status oa_gpu_time_kernels(oa_ctx *ctx, void *stream, const double *psi, int 
  * allow. */
 typedef struct oa_tuning {
   int group_state;   /* state groups of the per-state plane kernels: nz x groups blocks (1..32) */
-  int group_pair;    /* pair groups of the state-pair density kernel (1..32) */
+  int group_pair;    /* pair groups of the state-pair plane kernels (1..32); at the built-in count of the
+                        density kernel the V_KS kernel has its own built-in one */
   int dgemm_kblocks; /* most split-K blocks of the FP64 tensor-core products (2..160) */
   int tgemm_kblocks; /* most split-K blocks of the split-BF16 tcgen05 products (1..the limit set at init) */
   int fft_path;      /* 1: two-pass register transforms where compiled; 2: runtime-plan shared-memory

@@ -475,6 +475,8 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
         c->ngroup_pair = pick_pair_groups(d->nz * split, npair, dbps, nsm);
         c->ngroup_vks = pick_pair_groups(d->nz, npair, vbps, nsm);
         c->pair_split = split;
+        c->built_pair = c->ngroup_pair;
+        c->built_vks = c->ngroup_vks;
       } else {
         cudaGetLastError();
         c->pair_on = 0;
@@ -1098,6 +1100,9 @@ extern "C" oa_status oa_gpu_set_tuning(oa_ctx* c, const oa_tuning* t) {
   }
   c->ngroup = gs;
   c->ngroup_pair = gp;
+  // a given count holds for the V_KS kernel too; at the built-in count of the
+  // density kernel that kernel has its own built-in one
+  if (t->group_pair && c->ngroup_vks) c->ngroup_vks = gp == c->built_pair ? c->built_vks : gp;
   if (c->qpart) c->nq2 = nq2;
   if (t->dgemm_kblocks) p->nkb = t->dgemm_kblocks;
   if (t->tgemm_kblocks) p->umax_kb = t->tgemm_kblocks;

@@ -113,6 +113,7 @@ struct oa_ctx {
   int ngroup;             // state groups in the plane kernels
   int ngroup_pair;        // pair groups of the state-pair density kernel (oa_tuning group_pair)
   int ngroup_vks;         // pair groups of the state-pair V_KS kernel
+  int built_pair, built_vks;  // the built-in choices of the two
   int rho_ngroup;         // groups summed in rho_part by the last density pass
   int* pair_cols;         // [nkx_s] {first line, ky of the first line, lines, 0} when the lines form column runs
   int pair_on;            // the state-pair plane kernels take this system

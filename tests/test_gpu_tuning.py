@@ -31,7 +31,9 @@ def _run(s, prec, steps, **choice):
 @pytest.mark.parametrize("prec,choice,tol", [
     ("fp64", {"group_state": 3, "dgemm_kblocks": 48}, 1e-12),
     ("fp64", {"fft_path": 2}, 1e-12),
+    ("fp64", {"group_pair": 16}, 1e-12),
     ("mixed", {"group_pair": 7, "dgemm_kblocks": 96}, 1e-6),
+    ("mixed", {"group_pair": 16}, 1e-6),
 ])
 def test_tuning_changes_rounding_only(prec, choice, tol):
     s = make_system("w8", nstate=32, seed=11)
