@@ -19,12 +19,19 @@ __host__ __device__ __forceinline__ size_t oa_plane_at(int r, long c, int rows_p
   return ((size_t)(c >> 6) * rows_pad + r) * 64 + (size_t)(c & 63);
 }
 
+// a + b = s + e exactly, s = fl(a + b) (Knuth's two-sum)
+__host__ __device__ __forceinline__ void oa_two_sum(float a, float b, float& s, float& e) {
+  const float c = a + b, t = c - a;
+  e = (a - (c - t)) + (b - t);
+  s = c;
+}
+
 // the nt bf16 digits of v (nt <= 3): v is split into two FP32 parts first and
 // the digits are taken in FP32 (conversions from and to FP64 run at a quarter
-// of the FP32 rate), where the sum of the remainder and the low part rounds
-// 2^-33 below v, far under the last digit
-__device__ __forceinline__ void oa_bf16_digits(double v, int nt, __nv_bfloat16* h) {
-  float r = (float)v;
+// of the FP32 rate); remainders are exact, so the digits are those of FP64
+// remainders but for the low part's own rounding, 2^-48 below v
+__host__ __device__ __forceinline__ void oa_bf16_digits(double v, int nt, __nv_bfloat16* h) {
+  float r = (float)v, e = 0.f;
   const float lo = (float)(v - (double)r);
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
@@ -32,13 +39,14 @@ __device__ __forceinline__ void oa_bf16_digits(double v, int nt, __nv_bfloat16* 
     const __nv_bfloat16 b = __float2bfloat16_rn(r);
     h[q] = b;
     r -= __bfloat162float(b);
-    if (q == 0) r += lo;
+    if (q == 0) oa_two_sum(r, lo, r, e);
+    else r += e;
   }
 }
 
 // the digits of a pair, one conversion instruction for both
-__device__ __forceinline__ void oa_bf16_digits2(double x, double y, int nt, __nv_bfloat162* h) {
-  float rx = (float)x, ry = (float)y;
+__host__ __device__ __forceinline__ void oa_bf16_digits2(double x, double y, int nt, __nv_bfloat162* h) {
+  float rx = (float)x, ry = (float)y, ex = 0.f, ey = 0.f;
   const float lx = (float)(x - (double)rx), ly = (float)(y - (double)ry);
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
@@ -47,7 +55,13 @@ __device__ __forceinline__ void oa_bf16_digits2(double x, double y, int nt, __nv
     h[q] = b;
     rx -= __low2float(b);
     ry -= __high2float(b);
-    if (q == 0) { rx += lx; ry += ly; }
+    if (q == 0) {
+      oa_two_sum(rx, lx, rx, ex);
+      oa_two_sum(ry, ly, ry, ey);
+    } else {
+      rx += ex;
+      ry += ey;
+    }
   }
 }
 
