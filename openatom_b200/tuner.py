@@ -7,9 +7,10 @@ value is set (oa_gpu_set_tuning) on a fresh context started from the same
 quenched coefficients and timed as whole native CP steps (one
 oa_gpu_cp_run call of ``steps`` steps after a warm-up call, CUDA events on
 the context's stream, best of ``reps``).  A value is
-kept only when it beats the current choice by more than ``margin``.  The
-result is recorded in a JSON table keyed by the system's sizes and
-precision (``tuning/b200.json``), which CPContext applies at creation.
+kept only when it beats the current choice by more than ``margin``.  A
+result that differs from the built-in choice is recorded in a JSON table
+keyed by the system's sizes and precision (``tuning/b200.json``), which
+CPContext applies at creation.
 
 Run on a B200:  python -m openatom_b200.tuner --presets w8 w32 w128 --batch 48
 """
@@ -51,6 +52,15 @@ def lookup(sysm, precision: str, path: str = TABLE):
     """The recorded choice for this system, or None."""
     e = load_table(path).get(system_key(sysm, precision))
     return None if e is None else dict(e["choice"])
+
+
+def record(tab: dict, key: str, entry: dict):
+    """Put a tuned entry in the table, which holds only what differs from
+    the built-in choice."""
+    if entry["choice"] != entry["default"]:
+        tab[key] = entry
+    else:
+        tab.pop(key, None)
 
 
 def candidates(knob: str, sysm, precision: str, current: dict, caps: dict) -> list:
@@ -189,9 +199,10 @@ def main(argv=None):
         with open(a.out) as f:
             tab = json.load(f).get("entries", {})
     t0 = time.time()
+    done = set()
     for sysm, prec in jobs:
         key = system_key(sysm, prec)
-        if key in tab and (tab[key].get("seen_this_run") or a.only_missing):
+        if key in done or (key in tab and a.only_missing):
             continue
         print(f"{key}", flush=True)
         steps = a.steps if sysm.nstate <= 128 else max(2, a.steps // 4)
@@ -200,12 +211,11 @@ def main(argv=None):
         except Exception as exc:  # record and go on with the other systems
             print(f"  failed: {exc}", flush=True)
             continue
-        e["seen_this_run"] = True
-        tab[key] = e
+        done.add(key)
+        record(tab, key, e)
         print(f"  -> {e['choice']}  {e['ms_default']:.4f} -> {e['ms_tuned']:.4f} ms/step", flush=True)
-    for e in tab.values():
-        e.pop("seen_this_run", None)
     meta = {"device": torch.cuda.get_device_name(0), "tuned_s": round(time.time() - t0, 1),
+            "systems_timed": len(done),
             "method": "coordinate descent over oa_tuning, native CP steps timed with CUDA events, "
                       f"best of {a.reps}, {a.steps} steps (fewer above 128 states), 1.5% margin"}
     os.makedirs(os.path.dirname(a.out), exist_ok=True)

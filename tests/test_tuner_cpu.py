@@ -42,3 +42,11 @@ def test_committed_table_is_well_formed():
         assert e["ms_tuned"] <= e["ms_default"] * 1.05
         if prec == "mixed":
             assert e["choice"]["fft_path"] == 1
+
+
+def test_table_holds_only_what_differs():
+    tab = {"a": {"choice": {"group_pair": 2}, "default": {"group_pair": 1}}}
+    tuner.record(tab, "b", {"choice": {"group_pair": 3}, "default": {"group_pair": 1}})
+    tuner.record(tab, "a", {"choice": {"group_pair": 1}, "default": {"group_pair": 1}})
+    assert list(tab) == ["b"]
+    assert all(e["choice"] != e["default"] for e in tuner.load_table().values())
