@@ -44,13 +44,7 @@ cudaError_t oa_launch_step_record(cudaStream_t s, const OaSumJobs& J, const int*
                                   unsigned* ticket);
 cudaError_t oa_launch_sum_partials(cudaStream_t s, const double* part, int n, int stride, int off, double scale,
                                    double* out);
-cudaError_t oa_launch_umma_fwd(cudaStream_t s, int nterm, const double* A, const double* B, int m, int n, long K,
-                               long kx0_cols, double w_kx0, double alpha, float* part, int max_kb, double* C,
-                               int* err_flag, int nsm);
-cudaError_t oa_launch_umma_bwd(cudaStream_t s, int nterm, const double* M1, const double* X1, double a1_kx0,
-                               double a1_rest, const double* M2, const double* X2, double a2, int nj, int nk,
-                               long ncol, long kx0_cols, double* out, int* err_flag);
-int oa_umma_max_kb(int m, int n, int nsm);
+int oa_tg_max_kb(int m, int n, int nsm);
 cudaError_t oa_split_kc(cudaStream_t s, int nt, const double* X, int rows, int rows_pad, long K, long ldx,
                         long kx0_cols, double w_kx0, __nv_bfloat16* P, long ldp, const int* cond = nullptr);
 int oa_tg_rows_pad(int rows, int box);
@@ -532,10 +526,10 @@ extern "C" oa_status oa_gpu_init(const oa_system_desc* d, int precision, oa_ctx*
     }
     TRY(cudaMalloc(&p->vtmp, (size_t)d->nstate * d->ng * sizeof(double2)));
     p->nsm = nsm;
-    p->umax_kb = oa_umma_max_kb(d->nstate, d->nstate, nsm);
+    p->umax_kb = oa_tg_max_kb(d->nstate, d->nstate, nsm);
     {
       const int mx = d->nstate > d->natm_nl ? d->nstate : d->natm_nl;
-      const int kbz = oa_umma_max_kb(d->nstate, d->natm_nl > 0 ? d->natm_nl : 1, nsm);
+      const int kbz = oa_tg_max_kb(d->nstate, d->natm_nl > 0 ? d->natm_nl : 1, nsm);
       const size_t need = (size_t)(p->umax_kb > kbz ? p->umax_kb : kbz) * d->nstate * mx;
       TRY(cudaMalloc(&p->upart, need * sizeof(float)));
       p->umax_kb = p->umax_kb > kbz ? p->umax_kb : kbz;
@@ -1241,10 +1235,9 @@ oa_status oa_planes_psi_refresh(oa_ctx* c, cudaStream_t s, const double* psi, in
   return OA_OK;
 }
 
-// Split-BF16 forward product through bf16 planes (oa_tgemm.cu); the
-// element-wise-staging kernels (oa_umma.cu) for shapes the planes path does
-// not take.  A: [m][K] (kx0 columns weighted by w_kx0), B: [n][K], in
-// plane slots sa and sb.
+// Split-BF16 forward product through bf16 planes (oa_tgemm.cu).
+// A: [m][K] (kx0 columns weighted by w_kx0), B: [n][K], in plane slots sa
+// and sb.
 static cudaError_t mixed_fwd(oa_ctx* c, cudaStream_t s, int nt, const double* A, const double* B, int m, int n,
                              long K, long kx0_cols, double w_kx0, double alpha, double* C, int sa, int sb,
                              const int* cond) {
@@ -1252,28 +1245,22 @@ static cudaError_t mixed_fwd(oa_ctx* c, cudaStream_t s, int nt, const double* A,
   const int mx = c->nstate > c->natm_nl ? c->nstate : c->natm_nl;
   const int nb = oa_tg_nb(n);
   const int ra = oa_tg_rows_pad(m, 128), rb = oa_tg_rows_pad(n, nb);
-  if (m <= mx && n <= mx && K <= p->pl_ld && ra <= p->pl_rows && rb <= p->pl_rows) {
-    const bool same = B == A && (w_kx0 == 1.0 || kx0_cols == 0) && ra % nb == 0;
-    cudaError_t e = ensure_planes(c, s, nt, sa, A, m, ra, K, kx0_cols, w_kx0, cond);
-    if (e != cudaSuccess) return e;
-    const bf16* pb = (const bf16*)p->pl_big[sa];
-    int rows_b = ra;
-    if (!same) {
-      if ((e = ensure_planes(c, s, nt, sb, B, n, rb, K, 0, 1.0, cond)) != cudaSuccess) return e;
-      pb = (const bf16*)p->pl_big[sb];
-      rows_b = rb;
-    }
-    e = oa_tfwd(s, nt, (const bf16*)p->pl_big[sa], ra, pb, rows_b, m, n, K, p->pl_ld, alpha, p->upart, p->umax_kb, C,
-                p->err_flag, p->nsm, cond);
-    if (e != cudaErrorNotSupported) return e;
+  if (m > mx || n > mx || K > p->pl_ld || ra > p->pl_rows || rb > p->pl_rows) return cudaErrorNotSupported;
+  const bool same = B == A && (w_kx0 == 1.0 || kx0_cols == 0) && ra % nb == 0;
+  cudaError_t e = ensure_planes(c, s, nt, sa, A, m, ra, K, kx0_cols, w_kx0, cond);
+  if (e != cudaSuccess) return e;
+  const bf16* pb = (const bf16*)p->pl_big[sa];
+  int rows_b = ra;
+  if (!same) {
+    if ((e = ensure_planes(c, s, nt, sb, B, n, rb, K, 0, 1.0, cond)) != cudaSuccess) return e;
+    pb = (const bf16*)p->pl_big[sb];
+    rows_b = rb;
   }
-  if (cond) return cudaErrorNotSupported;  // the fallback kernels have no device flag
-  return oa_launch_umma_fwd(s, nt, A, B, m, n, K, kx0_cols, w_kx0, alpha, p->upart, p->umax_kb, C, p->err_flag,
-                            p->nsm);
+  return oa_tfwd(s, nt, (const bf16*)p->pl_big[sa], ra, pb, rows_b, m, n, K, p->pl_ld, alpha, p->upart, p->umax_kb, C,
+              p->err_flag, p->nsm, cond);
 }
 
-// Split-BF16 backward product through bf16 planes, with the same fallback;
-// X1, X2 in plane slots s1, s2.
+// Split-BF16 backward product through bf16 planes; X1, X2 in plane slots s1, s2.
 static cudaError_t mixed_bwd(oa_ctx* c, cudaStream_t s, int nt, const double* M1, const double* X1, double a1_kx0,
                              double a1_rest, const double* M2, const double* X2, double a2, int nj, int nk, long ncol,
                              long kx0_cols, double* out, int s1, int s2, const double* yadd,
@@ -1292,20 +1279,17 @@ static cudaError_t mixed_bwd(oa_ctx* c, cudaStream_t s, int nt, const double* M1
   // M planes that the producer of M1 wrote (oa_m_planes) serve this product only
   const bool mready = p->m_ready == M1 && p->m_ready2 == M2 && p->m_nt == nt && p->m_nk == nk && p->m_nj == nj;
   p->m_ready = nullptr;
-  if (nj <= mx && nk <= mx && ncol <= p->pl_ld && ldm <= p->pl_rows && nkp <= p->pl_rows && (!M2 || s1 != s2)) {
-    bf16 *pm1 = (bf16*)p->pl_ma, *pm2 = (bf16*)p->pl_mb;
-    cudaError_t e = ensure_planes(c, s, nt, s1, X1, nk, rx1, ncol, 0, 1.0, cond);
-    if (e == cudaSuccess && !mready) e = oa_split_kc(s, nt, M1, nk, nkp, nj, nj, 0, 1.0, pm1, ldm, cond);
-    if (e == cudaSuccess && M2) e = ensure_planes(c, s, nt, s2, X2, nk, rx2, ncol, 0, 1.0, cond);
-    if (e == cudaSuccess && M2 && !mready) e = oa_split_kc(s, nt, M2, nk, nkp, nj, nj, 0, 1.0, pm2, ldm, cond);
-    if (e != cudaSuccess) return e;
-    e = oa_tbwd(s, nt, pm1, (const bf16*)p->pl_big[s1], rx1, a1_kx0, a1_rest, M2 ? pm2 : nullptr,
-                M2 ? (const bf16*)p->pl_big[s2] : nullptr, rx2, a2, nj, nkp, ncol, p->pl_ld, kx0_cols, out, p->err_flag,
-                yadd, cond);
-    if (e != cudaErrorNotSupported) return e;
-  }
-  if (cond || yadd) return cudaErrorNotSupported;  // the fallback kernels have neither
-  return oa_launch_umma_bwd(s, nt, M1, X1, a1_kx0, a1_rest, M2, X2, a2, nj, nk, ncol, kx0_cols, out, p->err_flag);
+  if (nj > mx || nk > mx || ncol > p->pl_ld || ldm > p->pl_rows || nkp > p->pl_rows || (M2 && s1 == s2))
+    return cudaErrorNotSupported;
+  bf16 *pm1 = (bf16*)p->pl_ma, *pm2 = (bf16*)p->pl_mb;
+  cudaError_t e = ensure_planes(c, s, nt, s1, X1, nk, rx1, ncol, 0, 1.0, cond);
+  if (e == cudaSuccess && !mready) e = oa_split_kc(s, nt, M1, nk, nkp, nj, nj, 0, 1.0, pm1, ldm, cond);
+  if (e == cudaSuccess && M2) e = ensure_planes(c, s, nt, s2, X2, nk, rx2, ncol, 0, 1.0, cond);
+  if (e == cudaSuccess && M2 && !mready) e = oa_split_kc(s, nt, M2, nk, nkp, nj, nj, 0, 1.0, pm2, ldm, cond);
+  if (e != cudaSuccess) return e;
+  return oa_tbwd(s, nt, pm1, (const bf16*)p->pl_big[s1], rx1, a1_kx0, a1_rest, M2 ? pm2 : nullptr,
+              M2 ? (const bf16*)p->pl_big[s2] : nullptr, rx2, a2, nj, nkp, ncol, p->pl_ld, kx0_cols, out, p->err_flag,
+              yadd, cond);
 }
 
 // v = sign psi / dt under the device flag (and everywhere when cond is

@@ -25,6 +25,7 @@
 // warp-specialised (below).  Every wait is bounded: on timeout the block
 // sets the device error flag, waits (bounded) for the copies it issued,
 // frees its TMEM and returns.  No multicast.
+#include <algorithm>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <mutex>
@@ -589,8 +590,6 @@ static bool tg_map(CUtensorMap* map, const bf16* P, int nt, int rows, long ldp, 
          CUDA_SUCCESS;
 }
 
-int oa_tgemm_available() { return tg_encoder() != nullptr; }
-
 cudaError_t oa_split_kc(cudaStream_t s, int nt, const double* X, int rows, int rows_pad, long K, long ldx,
                         long kx0_cols, double w_kx0, bf16* P, long ldp, const int* cond) {
   if (rows_pad < rows || (ldp & 63)) return cudaErrorInvalidValue;
@@ -605,6 +604,13 @@ cudaError_t oa_split_kc(cudaStream_t s, int nt, const double* X, int rows, int r
 int oa_tg_rows_pad(int rows, int box) { return (rows + box - 1) / box * box; }
 // N tile of the products: 64, or tiles of 128
 int oa_tg_nb(int n) { return n <= 64 ? 64 : 128; }
+
+// K blocks of an m x n product that fill the SMs (the split-K partials are
+// sized for them)
+int oa_tg_max_kb(int m, int n, int nsm) {
+  const int np = std::max((n + 15) / 16 * 16, 16), nb = np > 160 ? TG_M : np;
+  return std::max(nsm / (((m + TG_M - 1) / TG_M) * ((n + nb - 1) / nb)), 1);
+}
 
 // forward stages carry TG_KF columns of K, backward stages TG_KS rows of k
 static size_t tg_smem(int nt, int nb, int stages, bool fwd) {
