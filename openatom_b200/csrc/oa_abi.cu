@@ -1112,10 +1112,11 @@ extern "C" oa_status oa_gpu_sizes(const oa_ctx* c, long* out) {
   OA_ARG_CHECK(c && out, "null argument");
   out[0] = c->nstate; out[1] = c->ng; out[2] = c->nlines; out[3] = c->nz; out[4] = c->ldl;
   out[5] = c->ngroup; out[6] = c->npts; out[7] = c->precision == OA_FP64 ? 8 : 4; out[8] = c->nlines_d;
-  // kernels of the FP64 oa_gpu_cp_step (an estimate; oa_cp_state.last_kernels counts the
-  // graphed step): state_fft_fwd 3 + vks_build 5 + nl_sf 7 + vks_apply 4 + lambda 4 +
-  // integrate 3 + S 2 + Newton-Schulz 1 + Psi T 1
-  out[9] = 3 + 5 + 7 + 4 + 4 + 3 + 2 + 1 + 1;
+  // kernels of an FP64 step with the structure-factor method below 120 points
+  // (oa_cp_state.last_kernels counts the captured step): phase tables 1, forward z pass 1, density 1,
+  // rho and XC 1, V_KS build 3, nonlocal 5, V_KS and backward z pass 2, Lambda 2, Gamma 1, F' 1,
+  // integration 1, S 2, Newton-Schulz 1, record 1, Psi T 2
+  out[9] = 1 + 1 + 1 + 1 + 3 + 5 + 2 + 2 + 1 + 1 + 1 + 2 + 1 + 1 + 2;
   out[10] = c->pair_on && !c->fft_runtime ? 1 : 0;  // state-pair plane kernels in use
   out[11] = c->ngroup_pair;
   out[12] = (c->precision == OA_MIXED && c->nstate <= 128) ? 1 : 0;  // int8 overlap / rotation available
@@ -1276,7 +1277,7 @@ static cudaError_t mixed_bwd(oa_ctx* c, cudaStream_t s, int nt, const double* M1
   };
   const int rx1 = held(s1, X1), rx2 = M2 ? held(s2, X2) : 0;
   const int ldm = oa_tg_rows_pad(nj, oa_tg_nb(nj));  // M planes: leading size of whole N tiles, zero beyond nj
-  // M planes that the producer of M1 wrote (oa_m_planes) serve this product only
+  // M planes that the producer of M1 wrote (m_planes) serve this product only
   const bool mready = p->m_ready == M1 && p->m_ready2 == M2 && p->m_nt == nt && p->m_nk == nk && p->m_nj == nj;
   p->m_ready = nullptr;
   if (nj > mx || nk > mx || ncol > p->pl_ld || ldm > p->pl_rows || nkp > p->pl_rows || (M2 && s1 == s2))

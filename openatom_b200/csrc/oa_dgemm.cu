@@ -528,7 +528,7 @@ k_dgemm_bwd(const double* __restrict__ M1, const double* __restrict__ X1, double
         }
       }
     }
-  __syncthreads();
+    __syncthreads();
     const size_t pstride = (size_t)po.rows_pad * po.ldp;
     for (int i = threadIdx.x; i < po.nt * TJ * (DB_TC / 8); i += D::THREADS) {
       const int q = i / (TJ * (DB_TC / 8)), rem = i - q * (TJ * (DB_TC / 8));

@@ -4,7 +4,8 @@
 //   OA_LENGTHS_LE108: lengths whose density planes fit in shared memory
 //     (k_rho2_fwd / k_rho2_bwd hold two half planes)
 //   OA_LENGTHS_ALL:   the z passes and the density z kernels
-// N1 is a multiple of 4 where there is one, for the band-pruned first DFT.
+// N1 is a multiple of 4, for the band-pruned first DFT, where the length has
+// such a pair of factors, but for 24 and 36.
 // Other 2-3-5 lengths run the runtime-plan transforms (oa_fft.cuh).
 #pragma once
 #define OA_LENGTHS_LE108(X)                                                                              \

@@ -53,7 +53,7 @@ def test_grid_lengths(n, nstate, precision, tol):
     assert rel(f2.cpu().numpy(), fr) < tol
 
 
-@pytest.mark.parametrize("n", [15, 60, 90, 120, 150])
+@pytest.mark.parametrize("n", [15, 25, 27, 45, 60, 81, 90, 100, 120, 125, 128, 135, 144, 150, 160])
 def test_density_path_lengths(n):
     """The density transforms and the Hartree / XC path off the preset lengths."""
     import torch
