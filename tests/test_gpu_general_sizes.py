@@ -29,7 +29,9 @@ def grid_system(n, nstate, box=7.0, frac=1.0):
 
 # FP64: rounding; mixed: FP32 transforms, about 3 log2(n) roundings of 6e-8
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("mixed", 1e-5)])
-@pytest.mark.parametrize("n,nstate", [(16, 4), (25, 5), (27, 3), (45, 3), (50, 2), (72, 5), (80, 3), (100, 3),
+@pytest.mark.parametrize("n,nstate", [(12, 3), (15, 2), (18, 3), (20, 5), (30, 3), (32, 2), (36, 3), (40, 3), (48, 5),
+                                      (54, 3), (60, 2), (75, 3), (81, 2), (90, 3), (96, 3), (108, 5), (150, 3),
+                                      (16, 4), (25, 5), (27, 3), (45, 3), (50, 2), (72, 5), (80, 3), (100, 3),
                                       (120, 3), (125, 2), (128, 3), (135, 2), (144, 3), (160, 2)])
 def test_grid_lengths(n, nstate, precision, tol):
     import torch

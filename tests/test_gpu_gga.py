@@ -29,7 +29,9 @@ def _rel(a, b):
 
 
 @pytest.mark.parametrize("preset,nfft,nstate", [("w2", None, None), ("w4", None, None), ("w8", None, 16),
-                                                 ("w2", (30, 30, 30), None)])
+                                                 ("w2", (30, 30, 30), None), ("w2", (27, 27, 27), 3),
+                                                 ("w2", (120, 120, 120), 3), ("w2", (125, 125, 125), 2),
+                                                 ("w2", (160, 160, 160), 3)])
 def test_vks_build_blyp(preset, nfft, nstate):
     import torch
     from openatom_b200.gpu import CPContext
