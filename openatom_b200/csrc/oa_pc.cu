@@ -184,6 +184,9 @@ k_pc_bwd_f64(const double* __restrict__ M1, const double* __restrict__ X1, doubl
 // 256 threads (one output each, k in ascending order), K in slabs of 16
 // through shared memory
 // ---------------------------------------------------------------------------
+// PLANES: with the plane outputs (their conversions cost a plain product 0.5 to
+// 1 us of its 3 to 8)
+template <bool PLANES>
 __global__ void __launch_bounds__(256)
 k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int n, double alpha,
              double* __restrict__ C, OaPlaneOut pc, OaPlaneOut pa) {
@@ -203,6 +206,7 @@ k_small_gemm(const double* __restrict__ A, const double* __restrict__ B, int n, 
   }
   const int i = i0 + ty, j = j0 + tx;
   if (i < n && j < n) C[(size_t)i * n + j] = alpha * acc;
+  if constexpr (!PLANES) return;
   // bf16 planes of C and of A, zero in the padding rows and columns (the
   // backward product reads them next; their split kernels were 3-4 us each)
   if (pc.P && i < pc.rows_pad && j < pc.ldp) oa_plane_put(pc, i, j, i < n && j < n ? alpha * acc : 0.0);
@@ -669,7 +673,8 @@ cudaError_t oa_launch_small_gemm(cudaStream_t s, const double* A, const double* 
       cols = q->ldp > cols ? (int)q->ldp : cols;
     }
   dim3 grid((cols + 15) / 16, (rows + 15) / 16);
-  k_small_gemm<<<grid, 256, 0, s>>>(A, B, n, alpha, C, c, a);
+  if (c.P || a.P) k_small_gemm<true><<<grid, 256, 0, s>>>(A, B, n, alpha, C, c, a);
+  else k_small_gemm<false><<<grid, 256, 0, s>>>(A, B, n, alpha, C, c, a);
   return cudaGetLastError();
 }
 
