@@ -469,8 +469,21 @@ cudaError_t oa_launch_state_plane_density(oa_ctx* c, cudaStream_t s) {
   if (e != cudaErrorNotSupported) return e;
   return c->precision == OA_FP64 ? launch_plane<double, 0>(c, s) : launch_plane<float, 0>(c, s);
 }
+// Without psi(r) of the last density pass: the fused forward and backward pass
+// of the per-state two-pass kernels, or the density kernel for psi(r) and the
+// V_KS kernel.  The fused pass keeps psi(r) in shared memory but makes twice
+// the transforms; with few states, and in large planes, where psi(r) leaves
+// the L2, it is the faster one.  Whole call, fused / pairs in us: 24^3, 8 and
+// 16 states, FP64 25 / 27 and 29 / 27; 64^3, FP64, 1 and 16 states 27 / 30 and
+// 54 / 50; 96^3, FP64, 32 and 64 states 222 / 231 and 429 / 418; 108^3, mixed,
+// 16 and 64 states 119 / 135 and 407 / 392; 160^3, mixed, 16, 64 and 128
+// states 285 / 339, 1049 / 1032 (smaller sphere: 780 / 855) and 2062 / 1900.
+static bool recompute_fused(const oa_ctx* c) {
+  return c->nx == c->ny && oa_plane2_supported(c->nx) && c->nstate < (c->nx < 96 ? 16 : c->nx < 120 ? 64 : 128);
+}
+
 cudaError_t oa_launch_state_plane_vks(oa_ctx* c, cudaStream_t s) {
-  if (c->psir_valid == 0) {
+  if (c->psir_valid == 0 && !recompute_fused(c)) {
     // psi(r) of the z-line buffer by the density kernel (its density sums go
     // to the partials of the last density pass, which rho has taken up)
     const cudaError_t e = pair_plane(c, s, 0, nullptr);

@@ -31,6 +31,7 @@ def grid_system(n, nstate, box=7.0, frac=1.0):
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("mixed", 1e-5)])
 @pytest.mark.parametrize("n,nstate", [(12, 3), (15, 2), (18, 3), (20, 5), (30, 3), (32, 2), (36, 3), (40, 3), (48, 5),
                                       (54, 3), (60, 2), (75, 3), (81, 2), (90, 3), (96, 3), (108, 5), (150, 3),
+                                      (24, 16), (64, 15), (64, 17), (96, 64),
                                       (16, 4), (25, 5), (27, 3), (45, 3), (50, 2), (72, 5), (80, 3), (100, 3),
                                       (120, 3), (125, 2), (128, 3), (135, 2), (144, 3), (160, 2)])
 def test_grid_lengths(n, nstate, precision, tol):
@@ -73,7 +74,9 @@ def test_density_path_lengths(n):
 
 
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-9), ("mixed", 1e-5)])
-@pytest.mark.parametrize("n,nstate,order,scale", [(40, 5, 4, 1.2), (45, 3, 6, 1.3), (64, 4, 8, 1.0), (96, 3, 4, 1.2)])
+@pytest.mark.parametrize("n,nstate,order,scale", [(40, 5, 4, 1.2), (45, 3, 6, 1.3), (64, 4, 8, 1.0), (96, 3, 4, 1.2),
+                                                (24, 15, 4, 1.2), (24, 33, 6, 1.2), (40, 16, 4, 1.2), (64, 9, 8, 1.0),
+                                                (96, 8, 4, 1.2)])
 def test_ees_pairs(n, nstate, order, scale, precision, tol):
     import torch
     from openatom_b200.gpu import CPContext
