@@ -1543,8 +1543,18 @@ extern "C" oa_status oa_gpu_ees_init(oa_ctx* c, int na, int nb, int nc, int orde
   TRYE(upload(&e->dyp, (const double2*)dyp_host, (size_t)c->ng));
   TRYE(cudaMalloc(&e->idx, (size_t)c->natm_nl * 3 * order * sizeof(int)));
   TRYE(cudaMalloc(&e->mn, (size_t)c->natm_nl * 3 * order * sizeof(double)));
+  // With few states on a small grid the per-state two-pass kernels are the
+  // faster ones: the pair kernels build the row lists of a plane first, and
+  // there are few pairs for them.  Whole call, per state / pairs in us: 12^3,
+  // mixed, 16 and 32 states 33 / 36 and 38 / 36; 24^3, FP64, 8 and 16 states
+  // 45 / 47 and 53 / 47; 40^3, 4 and 8 states, FP64 47 / 46 and 57 / 53, mixed
+  // 41 / 45 and 47 / 45; 64^3, FP64, 2 and 4 states 56 / 59 and 68 / 64.
+  const int min_pair = !(na == nb && oa_plane2_supported(na)) ? 1
+                       : na >= 40 ? 8 : c->precision == OA_FP64 ? 16 : 32;
   int pbps = 1;
-  if (oa_ees_pair_shape(c, &pbps) == cudaSuccess)
+  if (c->nstate < min_pair)
+    e->ngroup_pair = 0;
+  else if (oa_ees_pair_shape(c, &pbps) == cudaSuccess)
     e->ngroup_pair = pick_pair_groups(nc, (c->nstate + 1) / 2, pbps, pcx(c)->nsm);
   else
     cudaGetLastError();

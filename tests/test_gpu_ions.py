@@ -149,7 +149,8 @@ def test_local_forces_of_uneven_atoms(nz, types):
 
 
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-5)])
-@pytest.mark.parametrize("nstate,order,ions_first", [(5, 4, True), (7, 6, False), (8, 8, False)])
+@pytest.mark.parametrize("nstate,order,ions_first", [(5, 4, True), (7, 6, False), (8, 8, False), (33, 4, False),
+                                                     (47, 6, True)])
 def test_ees_atom_forces(nstate, order, ions_first, precision, tol):
     """Atom forces of the EES method in both forms, with a last state alone
     in its pair, and ion dynamics switched on before or after the method:
