@@ -2,6 +2,7 @@
 with and without the band-pruned first DFT, the row-split FP64 density pass),
 odd state counts, state counts at the edges of the product tiles and of
 several tiles, and the three Newton-Schulz forms, against the oracle."""
+import dataclasses
 import math
 
 import numpy as np
@@ -54,6 +55,62 @@ def test_grid_lengths(n, nstate, precision, tol):
     assert rel(rho.cpu().numpy(), O.density(psir, s)) < tol
     assert rel(f.cpu().numpy(), fr) < tol
     assert rel(f2.cpu().numpy(), fr) < tol
+
+
+def with_lines(s, order):
+    """The same system with its z-lines (and their coefficients) in another
+    order; returns it and the map new -> old of the coefficients."""
+    ln = s.line_nneg + s.line_npos
+    src = np.concatenate([np.arange(s.line_off[l], s.line_off[l] + ln[l]) for l in order])
+    lines = {k: getattr(s, k)[order] for k in ("line_kx", "line_ky", "line_nneg", "line_npos")}
+    off = np.concatenate([[0], np.cumsum(ln[order])[:-1]]).astype(np.int32)
+    pts = {k: getattr(s, k)[src] for k in ("kx", "ky", "kz", "cmass")}
+    return dataclasses.replace(s, psi=np.ascontiguousarray(s.psi[:, src]), line_off=off, **lines, **pts), src
+
+
+# planes with per-state two-pass kernels, with the runtime plan only, and (FP64) without pair kernels
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("mixed", 1e-5)])
+@pytest.mark.parametrize("n", [40, 45, 125])
+@pytest.mark.parametrize("order", ["columns", "shuffled", "rows"])
+def test_line_orders(n, order, precision, tol):
+    """Whole kx columns in another order (the state-pair kernels take them),
+    lines shuffled or sorted by ky (they do not): the same density, forces
+    and nonlocal forces as the oracle's."""
+    import torch
+    from openatom_b200.gpu import CPContext
+    s0 = grid_system(n, 3)
+    first = int((s0.line_kx == 0).sum())      # kx = 0 stays first, in the reference's order
+    rest = np.arange(first, s0.nlines)
+    if order == "columns":
+        rest = np.concatenate([rest[s0.line_kx[rest] == k] for k in sorted(set(s0.line_kx[rest]), reverse=True)])
+    elif order == "shuffled":
+        rest = np.random.default_rng(5).permutation(rest)
+    else:
+        rest = rest[np.argsort(s0.line_ky[rest], kind="stable")]
+    s, src = with_lines(s0, np.concatenate([np.arange(first), rest]))
+    ctx = CPContext(s, precision)
+    pairs = order == "columns" and not (n == 125 and precision == "fp64")
+    assert ctx.sizes()["pair_planes"] == int(pairs)
+    psi = torch.from_numpy(s.psi).cuda()
+    rho = torch.zeros(n, n, n, dtype=torch.float64, device="cuda")
+    f, f2, fnl, fees = (torch.zeros_like(psi) for _ in range(4))
+    v = np.random.default_rng(4).standard_normal((n, n, n)) * 0.3
+    ctx.state_fft_fwd(psi, rho)
+    ctx.set_vks(torch.from_numpy(v).cuda())
+    ctx.vks_apply_fft_bwd(psi, f)
+    ctx.vks_apply_fft_bwd(psi, f2, recompute_fwd=True)
+    ctx.nl_sf(psi, fnl)
+    ctx.ees_init(1.2, 4)
+    ctx.nl_ees(psi, fees)
+    torch.cuda.synchronize()
+    psir = O.state_g_to_r(s0.psi, s0)
+    fr, _ = O.eke(s0.psi, O.add_forces(O.vks_forces(psir, v, s0), None, s0), s0)
+    assert rel(rho.cpu().numpy(), O.density(psir, s0)) < tol
+    assert rel(f.cpu().numpy(), fr[:, src]) < tol
+    assert rel(f2.cpu().numpy(), fr[:, src]) < tol
+    assert rel(fnl.cpu().numpy(), O.nl_energy_forces(s0.psi, s0)[0][:, src]) < 1e-9
+    fe = O.nl_ees_energy_forces(s0.psi, s0, O.ees_setup(s0, 1.2, 4))[0]
+    assert rel(fees.cpu().numpy(), fe[:, src]) < (1e-9 if precision == "fp64" else 1e-5)
 
 
 @pytest.mark.parametrize("n", [15, 25, 27, 45, 60, 81, 90, 100, 120, 125, 128, 135, 144, 150, 160])
