@@ -19,10 +19,12 @@ __host__ __device__ __forceinline__ size_t oa_plane_at(int r, long c, int rows_p
   return ((size_t)(c >> 6) * rows_pad + r) * 64 + (size_t)(c & 63);
 }
 
-// a + b = s + e exactly, s = fl(a + b) (Knuth's two-sum)
+// a + b = s + e exactly, s = fl(a + b), for a = 0 or |a| >= |b| (Dekker's
+// fast two-sum).  Here a is a remainder of the FP32 part, a multiple of its
+// last place, and b the low part, at most half of that place.
 __host__ __device__ __forceinline__ void oa_two_sum(float a, float b, float& s, float& e) {
-  const float c = a + b, t = c - a;
-  e = (a - (c - t)) + (b - t);
+  const float c = a + b;
+  e = b - (c - a);
   s = c;
 }
 
